@@ -150,3 +150,69 @@ def tolerance(case):
     and 2.8e-7): a sum in another order flips a bf16 (or e4m3) rounding here and there."""
     return {"gateup": {"rel": 3e-4, "max": 6e-2}, "mlp": {"rel": 1.6e-3, "max": 9e-2},
             "mamba": {"rel": 1.2e-3, "max": 1.5e-1}, "rmsnorm": {"rel": 2.5e-7, "max": 1.1e-6}}[case["op"]]
+
+
+def _dequantized(q, scale, rows_per_scale):
+    s = scale.double().repeat_interleave(BLOCK, 1)
+    return q.float().double() * (s if rows_per_scale == 1 else s.repeat_interleave(rows_per_scale, 0))
+
+
+def _block_matmul(q, scale, weight, scale_weight):
+    return _dequantized(q, scale, 1) @ _dequantized(weight, scale_weight, BLOCK).t()
+
+
+def _bf16(t):
+    return t.float().to(torch.bfloat16).double()
+
+
+def _swiglu(gate, up):
+    gate, up = _bf16(gate), _bf16(up)
+    return _bf16(gate * torch.sigmoid(gate)) * up
+
+
+def _quantized(t):
+    t = t.float().reshape(t.shape[0], -1, BLOCK)
+    amax = t.abs().amax(-1, keepdim=True).clamp_min(1e-12)
+    scale = amax / torch.full_like(amax, 448.0)  # a tensor: by a plain number the GPU would multiply by its reciprocal
+    q = (t / scale).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
+    return q.reshape(t.shape[0], -1), scale[:, :, 0]
+
+
+@torch.no_grad()
+def exact(case, seed):
+    """The formulas in float64; the roundings between the steps (e4m3 activations, bf16 gate, up, SiLU, convolution and
+    sigmoid) are part of the operations and are kept, the last one of a result is not."""
+    state = prepare(case, seed)
+    op = state["op"]
+    if op == "gateup":
+        x, scale_x, gate_w, scale_gate, up_w, scale_up = state["args"]
+        gate = _block_matmul(x, scale_x, gate_w, scale_gate)
+        return _swiglu(gate, _block_matmul(x, scale_x, up_w, scale_up))
+    if op == "mlp":
+        gate_w, scale_gate, up_w, scale_up, down_w, scale_down = state["weights"]
+        x, scale_x = _quantized(state["x"])
+        gate = _block_matmul(x, scale_x, gate_w, scale_gate)
+        middle, scale_middle = _quantized(_bf16(_swiglu(gate, _block_matmul(x, scale_x, up_w, scale_up))))
+        return _block_matmul(middle, scale_middle, down_w, scale_down)
+    if op == "mamba":
+        hidden, mask, weight, bias, conv_w, conv_b = state["args"]
+        batch, seq = mask.shape
+        flat = hidden.reshape(batch * seq, HIDDEN).double()
+        projected = torch.empty(batch * seq, 2 * CHANNELS, dtype=torch.float64, device="cuda")
+        for c in range(0, 2 * CHANNELS, 4096):
+            projected[:, c:c + 4096] = flat @ weight[c:c + 4096].double().t() + bias[c:c + 4096].double()
+        projected = projected.view(batch, seq, 2 * CHANNELS)
+        x = _bf16(_bf16(projected[:, :, :CHANNELS]) * mask.double()[:, :, None])
+        taps = conv_w.double().reshape(CHANNELS, 4)
+        x = torch.nn.functional.pad(x, (0, 0, 3, 0))
+        conv = conv_b.double() + sum(x[:, t:t + seq] * taps[:, t] for t in range(4))
+        conv = _bf16(conv)
+        out = torch.where((mask >= 0.5)[:, :, None], conv * _bf16(torch.sigmoid(conv)), 0.0)
+        return out.transpose(1, 2).contiguous(), projected[:, :, CHANNELS:].transpose(1, 2)
+    query, key, weight_q, weight_k, eps = state["args"][:5]
+
+    def norm(t, w):
+        t = t.double()
+        return t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + eps) * w.double()
+
+    return norm(query, weight_q), norm(key, weight_k)
