@@ -31,6 +31,7 @@ EXPORTS = (
     "gu_version", "gu_error_string", "gu_select_plan", "gu_select_tile_kernel", "gu_workspace_bytes", "gu_workspace_init",
     "gu_run", "gu_run_concat", "gu_last_status", "gu_launch_count", "gu_run_decode_static", "gu_run_gather", "gu_quantize_activation", "gu_blockwise_gemm", "gu_run_fp8out",
     "gu_blockwise_gemm_scatter", "gu_reduce_gather", "gu_set_wait_limit_ns", "gu_trace_read", "gu_wait_probe", "gu_peer_barrier", "gu_is_range_checked_build",
+    "gu_mlp_block",
 )
 
 
@@ -45,6 +46,13 @@ class GuProblem(Structure):
         ("workspace", c_void_p), ("workspace_bytes", c_size_t),
         ("plan", c_int32), ("reserved", c_int32),
     ]
+
+
+class GuMlp(Structure):
+    _fields_ = [(name, c_void_p) for name in ("x", "gate_w", "scale_gate", "up_w", "scale_up", "down_w", "scale_down",
+                                              "x_q", "x_scale", "mid_q", "mid_scale", "output")]
+    _fields_ += [(name, c_int64) for name in ("m", "k", "n", "h_out", "ld_x", "ld_output")]
+    _fields_ += [("x_is_f32", c_int32), ("reserved", c_int32)]
 
 
 class GateUpError(RuntimeError):
@@ -91,6 +99,8 @@ def _load() -> ctypes.CDLL:
     lib.gu_reduce_gather.argtypes = [c_void_p, POINTER(c_void_p), c_int, c_int, c_int64, c_int64, c_void_p]
     lib.gu_run_fp8out.restype = c_int
     lib.gu_run_fp8out.argtypes = [POINTER(GuProblem), c_void_p, c_void_p, c_void_p]
+    lib.gu_mlp_block.restype = c_int
+    lib.gu_mlp_block.argtypes = [POINTER(GuMlp), c_void_p]
     lib.gu_last_status.restype = c_int
     lib.gu_last_status.argtypes = [POINTER(c_int), c_int]
     lib.gu_launch_count.restype = c_int64

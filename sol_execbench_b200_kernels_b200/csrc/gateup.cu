@@ -14,6 +14,7 @@
 #include "gateup_stream.cuh"
 #include "gateup_pair.cuh"
 #include "gateup_tile.cuh"
+#include "gateup_split.cuh"
 #include "quantize_act.cuh"
 #include "reduce_gather.cuh"
 
@@ -97,6 +98,7 @@ struct DeviceInfo {
   int cc_major = 0;
   int max_smem_optin = 0;
   int pair_clusters = 0;  // CTA pairs of the pair kernel that are resident at once (0: pairs cannot be launched)
+  int split_clusters[kSplitMaxCtas + 1] = {};  // [s]: clusters of s CTAs of the K-split kernel resident at once
   bool attrs_set = false;
 };
 DeviceInfo g_dev[64];
@@ -144,6 +146,12 @@ int device_info(DeviceInfo** out) {
         cudaFuncSetAttribute(gateup_pair_fp8out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
             cudaSuccess ||
         cudaFuncSetAttribute(blockwise_gemm_pair_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(gateup_split_kernel<kSplitGateUp>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(gateup_split_kernel<kSplitFp8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(gateup_split_kernel<kSplitGemm>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
             cudaSuccess) {
       cudaGetLastError();
       return GU_ECUDA;
@@ -168,6 +176,18 @@ int device_info(DeviceInfo** out) {
         clusters = 0;
       }
       d.pair_clusters = clusters;
+      // likewise for the K-split kernel, whose cluster size is chosen per launch
+      cfg.blockDim = dim3(kTileThreads, 1, 1);
+      cfg.dynamicSmemBytes = kSplitSmemBytes;
+      for (unsigned c = 2; c <= kSplitMaxCtas; ++c) {
+        cfg.gridDim = dim3(c * static_cast<unsigned>(d.sm_count), 1, 1);
+        attr.val.clusterDim.x = c;
+        if (cudaOccupancyMaxActiveClusters(&clusters, gateup_split_kernel<kSplitGemm>, &cfg) != cudaSuccess) {
+          cudaGetLastError();
+          clusters = 0;
+        }
+        d.split_clusters[c] = clusters;
+      }
     }
     d.attrs_set = true;
   }
@@ -203,6 +223,37 @@ unsigned int next_epoch() {
   return e;
 }
 std::atomic<long long> g_launches{0};
+
+// One launch.  Every kernel of the path waits (pdl_wait) before it touches what an earlier kernel may have written or
+// still reads, so it is launched with the programmatic-serialisation attribute: its blocks move in and set themselves
+// up while the kernel in front drains.  `cluster` > 1 sets a cluster size that the kernel does not fix itself.
+template <typename... Params, typename... Args>
+int launch(void (*kernel)(Params...), int grid, int threads, uint32_t smem, cudaStream_t stream, int cluster,
+           const Args&... args) {
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  std::memset(attrs, 0, sizeof(attrs));
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attrs[1].val.clusterDim.y = 1;
+  attrs[1].val.clusterDim.z = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return GU_ECUDA;
+  }
+  return GU_OK;
+}
 
 constexpr int kSmemBudget = 227 * 1024;
 
@@ -303,6 +354,7 @@ int launch_tile(const gu_problem* pr, const DeviceInfo& dev, cudaStream_t stream
   p.scale_out = nullptr;
   p.blocks_per_owner = 1;
   p.slot_rows = 0;
+  p.weights_ready = 0;
   p.out_rows = static_cast<int>(m);
   p.out_cols = static_cast<int>(n);
   const int total_tiles = p.num_tiles;
@@ -319,9 +371,9 @@ int launch_tile(const gu_problem* pr, const DeviceInfo& dev, cudaStream_t stream
   if (dp_tiles > 0) {
     p.num_tiles = dp_tiles;
     const int grid = dp_tiles < sms ? dp_tiles : sms;
-    gateup_tile_kernel<false><<<grid, kTileThreads, kTileSmemBytes, stream>>>(tm_x, tm_g, tm_u, tm_o, p);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    if (cudaGetLastError() != cudaSuccess) return GU_ECUDA;
+    if ((rc = launch(gateup_tile_kernel<false>, grid, kTileThreads, kTileSmemBytes, stream, 1, tm_x, tm_g, tm_u, tm_o, p)) !=
+        GU_OK)
+      return rc;
   }
   if (dp_tiles < total_tiles) {
     p.tile_begin = dp_tiles;
@@ -334,9 +386,8 @@ int launch_tile(const gu_problem* pr, const DeviceInfo& dev, cudaStream_t stream
     p.flags = static_cast<unsigned int*>(pr->workspace) + 256;
     p.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(pr->workspace) + kTileFlagBytes);
     p.epoch = next_epoch();
-    gateup_tile_kernel<true><<<static_cast<int>(grid), kTileThreads, kTileSmemBytes, stream>>>(tm_x, tm_g, tm_u, tm_o, p);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    if (cudaGetLastError() != cudaSuccess) return GU_ECUDA;
+    return launch(gateup_tile_kernel<true>, static_cast<int>(grid), kTileThreads, kTileSmemBytes, stream, 1, tm_x, tm_g,
+                  tm_u, tm_o, p);
   }
   return GU_OK;
 }
@@ -412,12 +463,9 @@ int launch_pair(const gu_problem* pr, const DeviceInfo& dev, cudaStream_t stream
     p.tile_begin = (rounds - 1) * clusters;
     p.flags = static_cast<unsigned int*>(pr->workspace);
     p.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(pr->workspace) + kTileFlagBytes);
-    gateup_pair_sk_kernel<<<2 * clusters, kPairThreads, kPairSmemBytes, stream>>>(tm_x, tm_g, tm_u, tm_o, p);
-  } else {
-    gateup_pair_kernel<<<2 * clusters, kPairThreads, kPairSmemBytes, stream>>>(tm_x, tm_g, tm_u, tm_o, p);
+    return launch(gateup_pair_sk_kernel, 2 * clusters, kPairThreads, kPairSmemBytes, stream, 1, tm_x, tm_g, tm_u, tm_o, p);
   }
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
+  return launch(gateup_pair_kernel, 2 * clusters, kPairThreads, kPairSmemBytes, stream, 1, tm_x, tm_g, tm_u, tm_o, p);
 }
 
 // The tile plan's kernel for a shape: CTA pairs once there is more than one 128-token block (a lone block would
@@ -505,9 +553,7 @@ int launch_stream_t(const gu_problem* pr, const DeviceInfo& dev, cudaStream_t st
   int64_t grid = dev.sm_count < kStreamMaxGrid ? dev.sm_count : kStreamMaxGrid;
   if (units < grid) grid = units;
   const uint32_t smem = StreamCfg<MPAD>::smem_bytes(stages, p.kb);
-  gateup_stream_kernel<MPAD><<<static_cast<int>(grid), kStreamThreads, smem, stream>>>(tm_x, tm_g, tm_u, p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
+  return launch(gateup_stream_kernel<MPAD>, static_cast<int>(grid), kStreamThreads, smem, stream, 1, tm_x, tm_g, tm_u, p);
 }
 
 
@@ -563,6 +609,247 @@ int encode_map_uncached(CUtensorMap* out, const void* ptr, uint64_t cols, uint64
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? GU_OK : GU_ECUDA;
+}
+
+// CTAs per tile of the K-split kernel, or 1 where the other kernels are the better choice.  Worth it when a launch has
+// so few 128-token tiles that most SMs would have none: as many CTAs per tile as can be resident together, each with
+// at least kSplitMinBlocks K blocks.
+constexpr int64_t kSplitMinBlocks = 4;
+int split_ctas(const DeviceInfo& dev, int64_t tiles, int64_t kb) {
+  for (int c = kSplitMaxCtas; c >= 2; --c)
+    if (tiles <= dev.split_clusters[c] && kb >= kSplitMinBlocks * c) return c;
+  return 1;
+}
+
+// `p` comes with its pointers; the map of x has 128-row boxes.
+template <int kOp>
+int launch_split(SplitParams& p, int64_t m, int64_t k, int64_t n, int64_t col_tiles, int splits, const CUtensorMap& tm_x,
+                 const CUtensorMap& tm_gate, const CUtensorMap& tm_up, cudaStream_t stream) {
+  p.m = static_cast<int>(m);
+  p.kb = static_cast<int>(k / 128);
+  p.num_m_blocks = static_cast<int>((m + kTileM - 1) / kTileM);
+  p.n_blocks128 = static_cast<int>(n / 128);
+  const int64_t ctas = p.num_m_blocks * col_tiles * splits;
+  return launch(gateup_split_kernel<kOp>, static_cast<int>(ctas), kTileThreads, kSplitSmemBytes, stream, splits, tm_x, tm_gate,
+                tm_up, p);
+}
+
+int launch_split_run(const gu_problem* pr, int splits, cudaStream_t stream) {
+  const int64_t m = pr->m, k = pr->k, n = pr->n;
+  CUtensorMap tm_x, tm_g, tm_u;
+  int rc;
+  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->gate_w, k, n, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
+  SplitParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.scale_x = pr->scale_x;
+  p.scale_gate = pr->scale_gate;
+  p.scale_up = pr->scale_up;
+  p.out = pr->output;
+  p.ld_out = pr->ld_output;
+  return launch_split<kSplitGateUp>(p, m, k, n, n / kTileN, splits, tm_x, tm_g, tm_u, stream);
+}
+
+int quantize_launch(const void* x, int x_is_f32, int64_t ld_x, void* q, float* scale, int64_t m, int64_t k,
+                    void* stream_v) {
+  if (!x || !q || !scale) return GU_EINVAL_NULL;
+  if (m < 1 || k < 128 || (k % 128) != 0 || ld_x < k) return GU_EINVAL_SHAPE;
+  const int64_t elem = x_is_f32 ? 4 : 2;
+  if (!aligned16(x) || !aligned16(q) || (reinterpret_cast<uintptr_t>(scale) & 3u) || (ld_x * elem) % 16 != 0)
+    return GU_EINVAL_ALIGN;
+  DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != GU_OK) return rc;
+  const long long blocks = static_cast<long long>(m) * (k / 128);
+  if (blocks >= (1ll << 31)) return GU_EINVAL_SHAPE;  // the kernel counts 1x128 blocks in 32 bits
+  const long long per_cta = (kQuantThreads / 16) * (x_is_f32 ? quant_unroll<float>() : quant_unroll<__nv_bfloat16>());
+  long long grid = (blocks + per_cta - 1) / per_cta;
+  // one wave: as many CTAs as are resident at once (the kernel's registers allow 4 of 256 threads per SM; a grid
+  // of 8 per SM ran as two waves and paid two ramps)
+  static const int resident[2][2] = {
+      {resident_ctas(quantize_act_kernel<__nv_bfloat16, false>, kQuantThreads),
+       resident_ctas(quantize_act_kernel<__nv_bfloat16, true>, kQuantThreads)},
+      {resident_ctas(quantize_act_kernel<float, false>, kQuantThreads),
+       resident_ctas(quantize_act_kernel<float, true>, kQuantThreads)}};
+  const long long cap = static_cast<long long>(dev->sm_count) * resident[x_is_f32 ? 1 : 0][ld_x != k ? 1 : 0];
+  if (grid > cap) grid = cap;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  const int g = static_cast<int>(grid);
+  const uint32_t nblk = static_cast<uint32_t>(blocks), kb = static_cast<uint32_t>(k / 128);
+  uint8_t* qb = static_cast<uint8_t*>(q);
+  const bool pitched = ld_x != k;
+  const int t = kQuantThreads;
+  if (x_is_f32) {
+    const float* xf = static_cast<const float*>(x);
+    return pitched ? launch(quantize_act_kernel<float, true>, g, t, 0, stream, 1, xf, qb, scale, nblk, ld_x, kb)
+                   : launch(quantize_act_kernel<float, false>, g, t, 0, stream, 1, xf, qb, scale, nblk, ld_x, kb);
+  }
+  const __nv_bfloat16* xh = static_cast<const __nv_bfloat16*>(x);
+  return pitched ? launch(quantize_act_kernel<__nv_bfloat16, true>, g, t, 0, stream, 1, xh, qb, scale, nblk, ld_x, kb)
+                 : launch(quantize_act_kernel<__nv_bfloat16, false>, g, t, 0, stream, 1, xh, qb, scale, nblk, ld_x, kb);
+}
+
+// `chained`: a step of gu_mlp_block — the kernel in front is the block's own quantiser, so the weights were complete
+// before it began, and tiles may be cut along K.
+int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chained, void* stream_v) {
+  if (!pr || !out_q || !out_scale) return GU_EINVAL_NULL;
+  if (!pr->x || !pr->scale_x || !pr->gate_w || !pr->scale_gate || !pr->up_w || !pr->scale_up) return GU_EINVAL_NULL;
+  if (!shape_ok(pr->m, pr->k, pr->n)) return GU_EINVAL_SHAPE;
+  if (!aligned16(pr->x) || !aligned16(pr->gate_w) || !aligned16(pr->up_w) || !aligned16(out_q) ||
+      (reinterpret_cast<uintptr_t>(pr->scale_x) & 3u) || (reinterpret_cast<uintptr_t>(pr->scale_gate) & 3u) ||
+      (reinterpret_cast<uintptr_t>(pr->scale_up) & 3u) || (reinterpret_cast<uintptr_t>(out_scale) & 3u))
+    return GU_EINVAL_ALIGN;
+  DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != GU_OK) return rc;
+  const int64_t m = pr->m, k = pr->k, n = pr->n;
+  CUtensorMap tm_x, tm_g, tm_u, tm_q;
+  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->gate_w, k, n, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
+
+  if (chained) {
+    const int splits = split_ctas(*dev, (m + kTileM - 1) / kTileM * (n / kTileN), k / 128);
+    if (splits > 1) {
+      SplitParams sp;
+      std::memset(&sp, 0, sizeof(sp));
+      sp.scale_x = pr->scale_x;
+      sp.scale_gate = pr->scale_gate;
+      sp.scale_up = pr->scale_up;
+      sp.out = out_q;
+      sp.scale_out = out_scale;
+      sp.ld_out = n;
+      sp.weights_ready = 1;
+      return launch_split<kSplitFp8>(sp, m, k, n, n / kTileN, splits, tm_x, tm_g, tm_u, static_cast<cudaStream_t>(stream_v));
+    }
+  }
+  TileParams p;
+  p.scale_x = pr->scale_x;
+  p.scale_gate = pr->scale_gate;
+  p.scale_up = pr->scale_up;
+  p.m = static_cast<int>(m);
+  p.kb = static_cast<int>(k / 128);
+  p.num_m_blocks = static_cast<int>((m + kTileM - 1) / kTileM);
+  p.num_n_blocks = static_cast<int>(n / kTileN);
+  const int64_t tiles = int64_t(p.num_m_blocks) * p.num_n_blocks;
+  if (tiles * (k / 128) >= (1ll << 31)) return GU_EINVAL_SHAPE;
+  p.num_tiles = static_cast<int>(tiles);
+  int64_t gm = (24ll << 20) / (128 * k);
+  if (gm < 1) gm = 1;
+  if (gm > p.num_m_blocks) gm = p.num_m_blocks;
+  p.group_m = static_cast<int>(gm);
+  p.tile_begin = 0;
+  p.flags = nullptr;
+  p.partials = nullptr;
+  p.epoch = 0;
+  p.out_count = 1;
+  p.out_rank = 0;
+  p.out_col0 = 0;
+  p.n_blocks128 = static_cast<int>(n / 128);
+  p.scale_out = out_scale;
+  p.blocks_per_owner = 1;
+  p.slot_rows = 0;
+  p.weights_ready = chained ? 1 : 0;
+
+  if (!tile_prefers_lone(kOpGateUpFp8, m, k / 128, n / kTileN, dev->sm_count, dev->pair_clusters, false)) {
+    const int clusters = pair_geometry(p, *dev, m, k, static_cast<int>(n / kTileN));
+    if (clusters < 1) return GU_EINVAL_SHAPE;
+    return launch(gateup_pair_fp8out_kernel, 2 * clusters, kPairThreads, kPairSmemBytes, static_cast<cudaStream_t>(stream_v),
+                  1, tm_x, tm_g, tm_u, tm_q, p);
+  }
+  const int grid = p.num_tiles < dev->sm_count ? p.num_tiles : dev->sm_count;
+  return launch(gateup_tile_fp8out_kernel, grid, kTileThreads, kTileSmemBytes, static_cast<cudaStream_t>(stream_v), 1, tm_x,
+                tm_g, tm_u, tm_q, p);
+}
+
+int gemm_launch(const void* a, const float* scale_a, const void* b, const float* scale_b, void* c, int64_t m,
+                int64_t k, int64_t n, int64_t ld_c, bool chained, void* stream_v) {
+  if (!a || !scale_a || !b || !scale_b || !c) return GU_EINVAL_NULL;
+  if (!shape_ok(m, k, n) || ld_c < n) return GU_EINVAL_SHAPE;
+  if (!aligned16(a) || !aligned16(b) || !aligned16(c) || (reinterpret_cast<uintptr_t>(scale_a) & 3u) ||
+      (reinterpret_cast<uintptr_t>(scale_b) & 3u) || (ld_c % 8) != 0)
+    return GU_EINVAL_ALIGN;
+  DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != GU_OK) return rc;
+
+  CUtensorMap tm_a, tm_b, tm_c;
+  if ((rc = get_map(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b, k, n, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, n, m, ld_c * 2, 64, 128)) != GU_OK) return rc;
+
+  if (chained) {
+    const int64_t col_tiles = (n / 128 + 1) / 2;
+    const int splits = split_ctas(*dev, (m + kTileM - 1) / kTileM * col_tiles, k / 128);
+    if (splits > 1) {
+      SplitParams sp;
+      std::memset(&sp, 0, sizeof(sp));
+      sp.scale_x = scale_a;
+      sp.scale_gate = scale_b;
+      sp.scale_up = scale_b;
+      sp.out = c;
+      sp.ld_out = ld_c;
+      sp.weights_ready = 1;
+      return launch_split<kSplitGemm>(sp, m, k, n, col_tiles, splits, tm_a, tm_b, tm_b, static_cast<cudaStream_t>(stream_v));
+    }
+  }
+  TileParams p;
+  p.scale_x = scale_a;
+  p.scale_gate = scale_b;
+  p.scale_up = scale_b;
+  p.m = static_cast<int>(m);
+  p.kb = static_cast<int>(k / 128);
+  p.n_blocks128 = static_cast<int>(n / 128);
+  p.scale_out = nullptr;
+  p.blocks_per_owner = 1;
+  p.slot_rows = 0;
+  p.weights_ready = chained ? 1 : 0;
+  p.out_rows = static_cast<int>(m);
+  p.out_cols = static_cast<int>(n);
+  if (!tile_prefers_lone(kOpGemm, m, k / 128, (n / 128 + 1) / 2, dev->sm_count, dev->pair_clusters, false)) {
+    // CTA pairs: 256-token x 256-column tiles, one per two-CTA cluster
+    p.num_m_blocks = static_cast<int>((m + 2 * kTileM - 1) / (2 * kTileM));
+    p.num_n_blocks = (p.n_blocks128 + 1) / 2;
+    const int64_t pair_tiles = int64_t(p.num_m_blocks) * p.num_n_blocks;
+    if (pair_tiles * (k / 128) >= (1ll << 31)) return GU_EINVAL_SHAPE;
+    p.num_tiles = static_cast<int>(pair_tiles);
+    int64_t pgm = (24ll << 20) / (256 * k);
+    if (pgm < 1) pgm = 1;
+    if (pgm > p.num_m_blocks) pgm = p.num_m_blocks;
+    p.group_m = static_cast<int>(pgm);
+    p.tile_begin = 0;
+    p.flags = nullptr;
+    p.partials = nullptr;
+    p.epoch = 0;
+    p.out_count = 1;
+    p.out_rank = 0;
+    p.out_col0 = 0;
+    const int clusters = p.num_tiles < dev->pair_clusters ? p.num_tiles : dev->pair_clusters;
+    return launch(blockwise_gemm_pair_kernel, 2 * clusters, kPairThreads, kPairSmemBytes, static_cast<cudaStream_t>(stream_v), 1,
+                  tm_a, tm_b, tm_c, p);
+  }
+  p.num_m_blocks = static_cast<int>((m + kTileM - 1) / kTileM);
+  p.num_n_blocks = (p.n_blocks128 + 1) / 2;  // a CTA tile spans two 128-column blocks of B
+  const int64_t tiles = int64_t(p.num_m_blocks) * p.num_n_blocks;
+  if (tiles * (k / 128) >= (1ll << 31)) return GU_EINVAL_SHAPE;
+  p.num_tiles = static_cast<int>(tiles);
+  int64_t gm = (24ll << 20) / (128 * k);
+  if (gm < 1) gm = 1;
+  if (gm > p.num_m_blocks) gm = p.num_m_blocks;
+  p.group_m = static_cast<int>(gm);
+  p.tile_begin = 0;
+  p.flags = nullptr;
+  p.partials = nullptr;
+  p.epoch = 0;
+  p.out_count = 1;
+  p.out_rank = 0;
+  p.out_col0 = 0;
+
+  const int grid = p.num_tiles < dev->sm_count ? p.num_tiles : dev->sm_count;
+  return launch(blockwise_gemm_kernel, grid, kTileThreads, kTileSmemBytes, static_cast<cudaStream_t>(stream_v), 1, tm_a, tm_b,
+                tm_c, p);
 }
 
 }  // namespace
@@ -629,6 +916,9 @@ size_t gu_workspace_bytes(int64_t m, int64_t k, int64_t n, int plan) {
     // what the tile plan would launch on a B200 (one cluster per two SMs): scratch only where stream-K is chosen
     const int clusters = gu::sm_count_or_default() / 2;
     const int64_t tiles = ((m + 255) / 256) * (n / 128);
+    gu::DeviceInfo like_b200;
+    for (int c = 2; c <= gu::kSplitMaxCtas; ++c) like_b200.split_clusters[c] = gu::sm_count_or_default() / c;
+    if (gu::split_ctas(like_b200, (m + gu::kTileM - 1) / gu::kTileM * (n / gu::kTileN), k / 128) > 1) return gu::kStreamFlagBytes;
     if (m > gu::kTileM && tiles < (1ll << 31) && gu::pair_prefers_stream_k(static_cast<int>(tiles), clusters) &&
         !gu::tile_prefers_lone(gu::kOpGateUp, m, k / 128, n / gu::kTileN, gu::sm_count_or_default(), clusters, true))
       return gu::tile_stream_k_bytes();
@@ -657,6 +947,11 @@ int gu_run(const gu_problem* pr, void* stream_v) {
   if (plan == GU_PLAN_TILE_PAIR) return gu::launch_pair(pr, *dev, stream, 0);
   if (plan == GU_PLAN_TILE_PAIR_SK) return gu::launch_pair(pr, *dev, stream, 1);
   const bool have_ws = pr->workspace && pr->workspace_bytes >= gu::tile_stream_k_bytes() && gu::aligned16(pr->workspace);
+  // (scratch stands for leave to cut tiles along K; this kernel needs none of it)
+  if (plan == GU_PLAN_TILE && pr->workspace && pr->workspace_bytes >= gu::kStreamFlagBytes) {
+    const int splits = gu::split_ctas(*dev, (pr->m + gu::kTileM - 1) / gu::kTileM * (pr->n / gu::kTileN), pr->k / 128);
+    if (splits > 1) return gu::launch_split_run(pr, splits, stream);
+  }
   if (plan == GU_PLAN_TILE && pr->m > gu::kTileM) {
     if (!gu::tile_prefers_lone(gu::kOpGateUp, pr->m, pr->k / 128, pr->n / gu::kTileN, dev->sm_count, dev->pair_clusters,
                                have_ws))
@@ -750,10 +1045,8 @@ int gu_run_decode_static(const gu_problem* pr, void* stream_v) {
   int64_t grid = dev->sm_count < gu::kStreamMaxGrid ? dev->sm_count : gu::kStreamMaxGrid;
   if (units < grid) grid = units;
   const uint32_t smem = gu::StreamCfg<16>::smem_bytes(stages, p.kb);
-  gu::gateup_stream_kernel<16><<<static_cast<int>(grid), gu::kStreamThreads, smem,
-                                 static_cast<cudaStream_t>(stream_v)>>>(tm_x, tm_g, tm_u, p);
-  gu::g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
+  return gu::launch(gu::gateup_stream_kernel<16>, static_cast<int>(grid), gu::kStreamThreads, smem,
+                    static_cast<cudaStream_t>(stream_v), 1, tm_x, tm_g, tm_u, p);
 }
 
 int gu_run_gather(const gu_problem* pr, void* const* rank_outputs, int world, int rank, int64_t ld_full,
@@ -808,6 +1101,7 @@ int gu_run_gather(const gu_problem* pr, void* const* rank_outputs, int world, in
   p.scale_out = nullptr;
   p.blocks_per_owner = 1;
   p.slot_rows = 0;
+  p.weights_ready = 0;
   p.out_count = world;
   p.out_rank = rank;
   p.out_col0 = static_cast<int>(int64_t(rank) * n);
@@ -882,6 +1176,7 @@ int gu_blockwise_gemm_scatter(const void* a, const float* scale_a, const void* b
   p.out_col0 = 0;
   p.blocks_per_owner = p.num_m_blocks / world;  // in 128-token blocks, whichever kernel runs
   p.slot_rows = static_cast<int>(slot_rows);
+  p.weights_ready = 0;
 
   if (gu::tile_prefers_pairs(m, *dev)) {
     const int clusters = gu::pair_geometry(p, *dev, m, k, (p.n_blocks128 + 1) / 2);
@@ -947,180 +1242,51 @@ int gu_peer_barrier(void* const* rank_flags, int world, int rank, uint64_t limit
 }
 
 int gu_quantize_activation(const void* x, int x_is_f32, int64_t ld_x, void* q, float* scale, int64_t m, int64_t k,
-                           void* stream_v) {
-  if (!x || !q || !scale) return GU_EINVAL_NULL;
-  if (m < 1 || k < 128 || (k % 128) != 0 || ld_x < k) return GU_EINVAL_SHAPE;
-  const int64_t elem = x_is_f32 ? 4 : 2;
-  if (!gu::aligned16(x) || !gu::aligned16(q) || (reinterpret_cast<uintptr_t>(scale) & 3u) || (ld_x * elem) % 16 != 0)
-    return GU_EINVAL_ALIGN;
-  gu::DeviceInfo* dev = nullptr;
-  int rc = gu::device_info(&dev);
-  if (rc != GU_OK) return rc;
-  const long long blocks = static_cast<long long>(m) * (k / 128);
-  if (blocks >= (1ll << 31)) return GU_EINVAL_SHAPE;  // the kernel counts 1x128 blocks in 32 bits
-  const long long per_cta = (gu::kQuantThreads / 16) * (x_is_f32 ? gu::quant_unroll<float>() : gu::quant_unroll<__nv_bfloat16>());
-  long long grid = (blocks + per_cta - 1) / per_cta;
-  // one wave: as many CTAs as are resident at once (the kernel's registers allow 4 of 256 threads per SM; a grid
-  // of 8 per SM ran as two waves and paid two ramps)
-  static const int resident[2][2] = {
-      {gu::resident_ctas(gu::quantize_act_kernel<__nv_bfloat16, false>, gu::kQuantThreads),
-       gu::resident_ctas(gu::quantize_act_kernel<__nv_bfloat16, true>, gu::kQuantThreads)},
-      {gu::resident_ctas(gu::quantize_act_kernel<float, false>, gu::kQuantThreads),
-       gu::resident_ctas(gu::quantize_act_kernel<float, true>, gu::kQuantThreads)}};
-  const long long cap = static_cast<long long>(dev->sm_count) * resident[x_is_f32 ? 1 : 0][ld_x != k ? 1 : 0];
-  if (grid > cap) grid = cap;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  const int g = static_cast<int>(grid);
-  const uint32_t nblk = static_cast<uint32_t>(blocks), kb = static_cast<uint32_t>(k / 128);
-  uint8_t* qb = static_cast<uint8_t*>(q);
-  const bool pitched = ld_x != k;
-  if (x_is_f32) {
-    const float* xf = static_cast<const float*>(x);
-    if (pitched) gu::quantize_act_kernel<float, true><<<g, gu::kQuantThreads, 0, stream>>>(xf, qb, scale, nblk, ld_x, kb);
-    else gu::quantize_act_kernel<float, false><<<g, gu::kQuantThreads, 0, stream>>>(xf, qb, scale, nblk, ld_x, kb);
-  } else {
-    const __nv_bfloat16* xh = static_cast<const __nv_bfloat16*>(x);
-    if (pitched) gu::quantize_act_kernel<__nv_bfloat16, true><<<g, gu::kQuantThreads, 0, stream>>>(xh, qb, scale, nblk, ld_x, kb);
-    else gu::quantize_act_kernel<__nv_bfloat16, false><<<g, gu::kQuantThreads, 0, stream>>>(xh, qb, scale, nblk, ld_x, kb);
-  }
-  gu::g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
+                           void* stream) {
+  return gu::quantize_launch(x, x_is_f32, ld_x, q, scale, m, k, stream);
 }
 
-int gu_run_fp8out(const gu_problem* pr, void* out_q, float* out_scale, void* stream_v) {
-  if (!pr || !out_q || !out_scale) return GU_EINVAL_NULL;
-  if (!pr->x || !pr->scale_x || !pr->gate_w || !pr->scale_gate || !pr->up_w || !pr->scale_up) return GU_EINVAL_NULL;
-  if (!gu::shape_ok(pr->m, pr->k, pr->n)) return GU_EINVAL_SHAPE;
-  if (!gu::aligned16(pr->x) || !gu::aligned16(pr->gate_w) || !gu::aligned16(pr->up_w) || !gu::aligned16(out_q) ||
-      (reinterpret_cast<uintptr_t>(pr->scale_x) & 3u) || (reinterpret_cast<uintptr_t>(pr->scale_gate) & 3u) ||
-      (reinterpret_cast<uintptr_t>(pr->scale_up) & 3u) || (reinterpret_cast<uintptr_t>(out_scale) & 3u))
-    return GU_EINVAL_ALIGN;
-  gu::DeviceInfo* dev = nullptr;
-  int rc = gu::device_info(&dev);
-  if (rc != GU_OK) return rc;
-  const int64_t m = pr->m, k = pr->k, n = pr->n;
-  CUtensorMap tm_x, tm_g, tm_u, tm_q;
-  if ((rc = gu::get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, 128)) != GU_OK) return rc;
-  if ((rc = gu::get_map(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->gate_w, k, n, k, 128, 128)) != GU_OK) return rc;
-  if ((rc = gu::get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
-  if ((rc = gu::get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
-
-  gu::TileParams p;
-  p.scale_x = pr->scale_x;
-  p.scale_gate = pr->scale_gate;
-  p.scale_up = pr->scale_up;
-  p.m = static_cast<int>(m);
-  p.kb = static_cast<int>(k / 128);
-  p.num_m_blocks = static_cast<int>((m + gu::kTileM - 1) / gu::kTileM);
-  p.num_n_blocks = static_cast<int>(n / gu::kTileN);
-  const int64_t tiles = int64_t(p.num_m_blocks) * p.num_n_blocks;
-  if (tiles * (k / 128) >= (1ll << 31)) return GU_EINVAL_SHAPE;
-  p.num_tiles = static_cast<int>(tiles);
-  int64_t gm = (24ll << 20) / (128 * k);
-  if (gm < 1) gm = 1;
-  if (gm > p.num_m_blocks) gm = p.num_m_blocks;
-  p.group_m = static_cast<int>(gm);
-  p.tile_begin = 0;
-  p.flags = nullptr;
-  p.partials = nullptr;
-  p.epoch = 0;
-  p.out_count = 1;
-  p.out_rank = 0;
-  p.out_col0 = 0;
-  p.n_blocks128 = static_cast<int>(n / 128);
-  p.scale_out = out_scale;
-  p.blocks_per_owner = 1;
-  p.slot_rows = 0;
-
-  if (!gu::tile_prefers_lone(gu::kOpGateUpFp8, m, k / 128, n / gu::kTileN, dev->sm_count, dev->pair_clusters, false)) {
-    const int clusters = gu::pair_geometry(p, *dev, m, k, static_cast<int>(n / gu::kTileN));
-    if (clusters < 1) return GU_EINVAL_SHAPE;
-    gu::gateup_pair_fp8out_kernel<<<2 * clusters, gu::kPairThreads, gu::kPairSmemBytes,
-                                    static_cast<cudaStream_t>(stream_v)>>>(tm_x, tm_g, tm_u, tm_q, p);
-    gu::g_launches.fetch_add(1, std::memory_order_relaxed);
-    return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
-  }
-  const int grid = p.num_tiles < dev->sm_count ? p.num_tiles : dev->sm_count;
-  gu::gateup_tile_fp8out_kernel<<<grid, gu::kTileThreads, gu::kTileSmemBytes, static_cast<cudaStream_t>(stream_v)>>>(
-      tm_x, tm_g, tm_u, tm_q, p);
-  gu::g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
+int gu_run_fp8out(const gu_problem* pr, void* out_q, float* out_scale, void* stream) {
+  return gu::fp8out_launch(pr, out_q, out_scale, false, stream);
 }
 
 int gu_blockwise_gemm(const void* a, const float* scale_a, const void* b, const float* scale_b, void* c, int64_t m,
-                      int64_t k, int64_t n, int64_t ld_c, void* stream_v) {
-  if (!a || !scale_a || !b || !scale_b || !c) return GU_EINVAL_NULL;
-  if (!gu::shape_ok(m, k, n) || ld_c < n) return GU_EINVAL_SHAPE;
-  if (!gu::aligned16(a) || !gu::aligned16(b) || !gu::aligned16(c) || (reinterpret_cast<uintptr_t>(scale_a) & 3u) ||
-      (reinterpret_cast<uintptr_t>(scale_b) & 3u) || (ld_c % 8) != 0)
-    return GU_EINVAL_ALIGN;
-  gu::DeviceInfo* dev = nullptr;
-  int rc = gu::device_info(&dev);
+                      int64_t k, int64_t n, int64_t ld_c, void* stream) {
+  return gu::gemm_launch(a, scale_a, b, scale_b, c, m, k, n, ld_c, false, stream);
+}
+
+int gu_mlp_block(const gu_mlp* b, void* stream) {
+  if (!b) return GU_EINVAL_NULL;
+  // everything is checked before the first launch
+  if (!b->x || !b->gate_w || !b->scale_gate || !b->up_w || !b->scale_up || !b->down_w || !b->scale_down || !b->x_q ||
+      !b->x_scale || !b->mid_q || !b->mid_scale || !b->output)
+    return GU_EINVAL_NULL;
+  if (!gu::shape_ok(b->m, b->k, b->n) || !gu::shape_ok(b->m, b->n, b->h_out) || b->ld_x < b->k || b->ld_output < b->h_out)
+    return GU_EINVAL_SHAPE;
+  const void* wide[] = {b->x, b->gate_w, b->up_w, b->down_w, b->x_q, b->mid_q, b->output};
+  const void* words[] = {b->scale_gate, b->scale_up, b->scale_down, b->x_scale, b->mid_scale};
+  for (const void* p : wide)
+    if (!gu::aligned16(p)) return GU_EINVAL_ALIGN;
+  for (const void* p : words)
+    if (reinterpret_cast<uintptr_t>(p) & 3u) return GU_EINVAL_ALIGN;
+  if ((b->ld_x * (b->x_is_f32 ? 4 : 2)) % 16 != 0 || b->ld_output % 8 != 0) return GU_EINVAL_ALIGN;
+
+  int rc = gu::quantize_launch(b->x, b->x_is_f32, b->ld_x, b->x_q, b->x_scale, b->m, b->k, stream);
   if (rc != GU_OK) return rc;
-
-  CUtensorMap tm_a, tm_b, tm_c;
-  if ((rc = gu::get_map(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k, 128, 128)) != GU_OK) return rc;
-  if ((rc = gu::get_map(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b, k, n, k, 128, 128)) != GU_OK) return rc;
-  if ((rc = gu::get_map(&tm_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, n, m, ld_c * 2, 64, 128)) != GU_OK) return rc;
-
-  gu::TileParams p;
-  p.scale_x = scale_a;
-  p.scale_gate = scale_b;
-  p.scale_up = scale_b;
-  p.m = static_cast<int>(m);
-  p.kb = static_cast<int>(k / 128);
-  p.n_blocks128 = static_cast<int>(n / 128);
-  p.scale_out = nullptr;
-  p.blocks_per_owner = 1;
-  p.slot_rows = 0;
-  p.out_rows = static_cast<int>(m);
-  p.out_cols = static_cast<int>(n);
-  if (!gu::tile_prefers_lone(gu::kOpGemm, m, k / 128, (n / 128 + 1) / 2, dev->sm_count, dev->pair_clusters, false)) {
-    // CTA pairs: 256-token x 256-column tiles, one per two-CTA cluster
-    p.num_m_blocks = static_cast<int>((m + 2 * gu::kTileM - 1) / (2 * gu::kTileM));
-    p.num_n_blocks = (p.n_blocks128 + 1) / 2;
-    const int64_t pair_tiles = int64_t(p.num_m_blocks) * p.num_n_blocks;
-    if (pair_tiles * (k / 128) >= (1ll << 31)) return GU_EINVAL_SHAPE;
-    p.num_tiles = static_cast<int>(pair_tiles);
-    int64_t pgm = (24ll << 20) / (256 * k);
-    if (pgm < 1) pgm = 1;
-    if (pgm > p.num_m_blocks) pgm = p.num_m_blocks;
-    p.group_m = static_cast<int>(pgm);
-    p.tile_begin = 0;
-    p.flags = nullptr;
-    p.partials = nullptr;
-    p.epoch = 0;
-    p.out_count = 1;
-    p.out_rank = 0;
-    p.out_col0 = 0;
-    const int clusters = p.num_tiles < dev->pair_clusters ? p.num_tiles : dev->pair_clusters;
-    gu::blockwise_gemm_pair_kernel<<<2 * clusters, gu::kPairThreads, gu::kPairSmemBytes,
-                                     static_cast<cudaStream_t>(stream_v)>>>(tm_a, tm_b, tm_c, p);
-    gu::g_launches.fetch_add(1, std::memory_order_relaxed);
-    return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
-  }
-  p.num_m_blocks = static_cast<int>((m + gu::kTileM - 1) / gu::kTileM);
-  p.num_n_blocks = (p.n_blocks128 + 1) / 2;  // a CTA tile spans two 128-column blocks of B
-  const int64_t tiles = int64_t(p.num_m_blocks) * p.num_n_blocks;
-  if (tiles * (k / 128) >= (1ll << 31)) return GU_EINVAL_SHAPE;
-  p.num_tiles = static_cast<int>(tiles);
-  int64_t gm = (24ll << 20) / (128 * k);
-  if (gm < 1) gm = 1;
-  if (gm > p.num_m_blocks) gm = p.num_m_blocks;
-  p.group_m = static_cast<int>(gm);
-  p.tile_begin = 0;
-  p.flags = nullptr;
-  p.partials = nullptr;
-  p.epoch = 0;
-  p.out_count = 1;
-  p.out_rank = 0;
-  p.out_col0 = 0;
-
-  const int grid = p.num_tiles < dev->sm_count ? p.num_tiles : dev->sm_count;
-  gu::blockwise_gemm_kernel<<<grid, gu::kTileThreads, gu::kTileSmemBytes, static_cast<cudaStream_t>(stream_v)>>>(
-      tm_a, tm_b, tm_c, p);
-  gu::g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? GU_OK : GU_ECUDA;
+  gu_problem pr;
+  std::memset(&pr, 0, sizeof(pr));
+  pr.x = b->x_q;
+  pr.scale_x = b->x_scale;
+  pr.gate_w = b->gate_w;
+  pr.scale_gate = b->scale_gate;
+  pr.up_w = b->up_w;
+  pr.scale_up = b->scale_up;
+  pr.m = b->m;
+  pr.k = b->k;
+  pr.n = b->n;
+  if ((rc = gu::fp8out_launch(&pr, b->mid_q, b->mid_scale, true, stream)) != GU_OK) return rc;
+  return gu::gemm_launch(b->mid_q, b->mid_scale, b->down_w, b->scale_down, b->output, b->m, b->n, b->h_out, b->ld_output, true,
+                         stream);
 }
 
 int gu_last_status(int* detail, int clear) {

@@ -346,6 +346,7 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tm_x, const 
 #endif
 
   if (threadIdx.x == 0) {
+    pdl_trigger();
     for (int s = 0; s < kPairStages; ++s) {
       mbar_init(bar_full + 8 * s, 2);
       mbar_init(bar_done + 8 * s, 1);
@@ -374,6 +375,7 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tm_x, const 
   cluster_sync_all();  // barriers and the abort flag of both CTAs exist before anything reaches across
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
+  pdl_wait();
 
   WaitCtx ctx{abort_slot, false, true};
   const bool is_consumer = warp >= 4 && warp < 12;
@@ -739,8 +741,8 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tm_x, const 
       if (!GU_IN_RANGE(m_global >= 0 && m_global < p.m && wblock >= 0 &&
                            wblock < (kSingle ? p.n_blocks128 : p.num_n_blocks), kSitePairScale))
         return;
-      sx0 = __ldg(p.scale_x + sx_off + j0);
-      sw0 = __ldg(scale_w + sw_off + j0);
+      sx0 = ld_dep(p.scale_x + sx_off + j0);
+      sw0 = ld_dep(scale_w + sw_off + j0);
     };
     if (have) start_tile(tile, jb);
 #ifdef GU_TRACE
@@ -771,8 +773,8 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tm_x, const 
         // the next K block's scales are fetched one block ahead of their use
         float sx1 = 0.f, sw1 = 0.f;
         if (j + 1 < je) {
-          sx1 = __ldg(p.scale_x + sx_off + j + 1);
-          sw1 = __ldg(scale_w + sw_off + j + 1);
+          sx1 = ld_dep(p.scale_x + sx_off + j + 1);
+          sw1 = ld_dep(scale_w + sw_off + j + 1);
         }
         const float sc = sx0 * sw0;
         const float2 scv = make_float2(sc, sc);

@@ -104,6 +104,7 @@ gateup_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
   const long long u_end = stream_range_start(units, ranges, my_range + 1);
 
   if (threadIdx.x == 0) {
+    pdl_trigger();
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
@@ -127,6 +128,7 @@ gateup_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
+  pdl_wait();
 
   WaitCtx ctx{abort_slot, false, false};
 
@@ -200,7 +202,7 @@ gateup_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     // scale_x, transposed to [kb][MPAD] so one K block's token scales are contiguous
     for (int i = ctid; i < p.kb * MPAD; i += 128) {
       const int jj = i / MPAD, t = i - jj * MPAD;
-      sx_smem[i] = (t < p.m) ? __ldg(p.scale_x + static_cast<size_t>(t) * p.kb + jj) : 0.f;
+      sx_smem[i] = (t < p.m) ? ld_dep(p.scale_x + static_cast<size_t>(t) * p.kb + jj) : 0.f;
     }
     named_bar_sync(1, 128);
 
@@ -215,15 +217,15 @@ gateup_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     int seg_first_j = j;
     float sg_next = 0.f, su_next = 0.f;
     if (GU_IN_RANGE(u_begin >= 0 && u_begin < units && u_end <= units, kSiteStreamScale)) {
-      sg_next = __ldg(p.scale_gate + u_begin);  // scale grids are [nb][kb]: unit index == flat index
-      su_next = __ldg(p.scale_up + u_begin);
+      sg_next = ld_dep(p.scale_gate + u_begin);  // scale grids are [nb][kb]: unit index == flat index
+      su_next = ld_dep(p.scale_up + u_begin);
     }
 
     for (long long u = u_begin; u < u_end; ++u) {
       const float sgw = sg_next, suw = su_next;
       if (u + 1 < u_end) {
-        sg_next = __ldg(p.scale_gate + u + 1);
-        su_next = __ldg(p.scale_up + u + 1);
+        sg_next = ld_dep(p.scale_gate + u + 1);
+        su_next = ld_dep(p.scale_up + u + 1);
       }
       const bool ok = mbar_wait(ctx, bar_acc_full + 8 * acc, acc_phase, kWaitStreamAccFull);
       tc_fence_after();

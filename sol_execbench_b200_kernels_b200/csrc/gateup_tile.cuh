@@ -94,6 +94,7 @@ struct TileParams {
   // sending rank (slot s starts at row s * slot_rows of that buffer)
   int blocks_per_owner;
   int slot_rows;
+  int weights_ready;        // the weights were complete before the kernel in front of this one began (see pdl_wait)
   // stream-K schedule only
   unsigned int* flags;      // [gridDim.x] epoch of the last call that filled slot i
   float* partials;          // [gridDim.x][32][256] float4: values 4i..4i+3 of consumer thread t at [i * 256 + t]
@@ -196,6 +197,7 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    pdl_trigger();
     for (int s = 0; s < kTileStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
@@ -233,28 +235,50 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
       // ------------------------------ TMA producer ------------------------------
       int stage = 0;
       uint32_t phase = 0;
+      auto in_range = [&](int st, int j, int mb, int nb) {
+        (void)st; (void)j; (void)mb; (void)nb;  // (only the range-checked build looks at them)
+        return GU_IN_RANGE(st >= 0 && st < kTileStages, kSiteTileStage) &&
+               GU_IN_RANGE(load_coords_ok(p.kb, j, mb * kTileM, p.num_m_blocks * kTileM) &&
+                               load_coords_ok(p.kb, j, nb * kTileN, p.num_n_blocks * kTileN), kSiteTileLoad);
+      };
+      auto load_weights = [&](int st, int j, int nb) {
+        const uint32_t full = bar_full + 8 * st;
+        const uint32_t dst = ring + st * kTileStageBytes;
+        mbar_arrive_expect_tx(full, kTileStageBytes);
+        if constexpr (kSingle) {  // two adjacent 128-row blocks of the one B matrix (rows past N read as zero)
+          tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, 2 * nb * kTileN);
+          tma_load_2d(dst + 2 * kOperandTileBytes, &tm_gate, full, j * kBlockK, (2 * nb + 1) * kTileN);
+        } else {
+          tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, nb * kTileN);
+          tma_load_2d(dst + 2 * kOperandTileBytes, &tm_up, full, j * kBlockK, nb * kTileN);
+        }
+      };
+      auto load_x = [&](int st, int j, int mb) {
+        tma_load_2d(ring + st * kTileStageBytes, &tm_x, bar_full + 8 * st, j * kBlockK, mb * kTileM);
+      };
       TileWalk<kStreamK> walk(p, blockIdx.x, gridDim.x);
       int tile, jb, je;
+      // K blocks of the first tile whose weights are loaded while the kernel in front still runs
+      int early = 0;
+      if constexpr (!kStreamK) {
+        if (p.weights_ready && static_cast<int>(blockIdx.x) < p.num_tiles) {
+          early = min(kTileStages, p.kb);
+          int mb, nb;
+          tile_coords(p, blockIdx.x, mb, nb);
+          for (int j = 0; j < early; ++j)
+            if (in_range(j, j, mb, nb)) load_weights(j, j, nb);
+        }
+      }
+      pdl_wait();
       while (walk.next(p, tile, jb, je)) {
         int mb, nb;
         tile_coords(p, kStreamK ? tile + p.tile_begin : tile, mb, nb);
         for (int j = jb; j < je; ++j) {
-          bool ok = mbar_wait(ctx, bar_empty + 8 * stage, phase ^ 1u, kWaitTileEmpty);
-          ok = ok && GU_IN_RANGE(stage >= 0 && stage < kTileStages, kSiteTileStage) &&
-               GU_IN_RANGE(load_coords_ok(p.kb, j, mb * kTileM, p.num_m_blocks * kTileM) &&
-                               load_coords_ok(p.kb, j, nb * kTileN, p.num_n_blocks * kTileN), kSiteTileLoad);
-          if (ok) {
-            const uint32_t full = bar_full + 8 * stage;
-            const uint32_t dst = ring + stage * kTileStageBytes;
-            mbar_arrive_expect_tx(full, kTileStageBytes);
-            tma_load_2d(dst, &tm_x, full, j * kBlockK, mb * kTileM);
-            if constexpr (kSingle) {  // two adjacent 128-row blocks of the one B matrix (rows past N read as zero)
-              tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, 2 * nb * kTileN);
-              tma_load_2d(dst + 2 * kOperandTileBytes, &tm_gate, full, j * kBlockK, (2 * nb + 1) * kTileN);
-            } else {
-              tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, nb * kTileN);
-              tma_load_2d(dst + 2 * kOperandTileBytes, &tm_up, full, j * kBlockK, nb * kTileN);
-            }
+          const bool weights_here = early > 0;
+          if (weights_here) --early;
+          if (mbar_wait(ctx, bar_empty + 8 * stage, phase ^ 1u, kWaitTileEmpty) && in_range(stage, j, mb, nb)) {
+            if (!weights_here) load_weights(stage, j, nb);
+            load_x(stage, j, mb);
           }
           if (++stage == kTileStages) { stage = 0; phase ^= 1u; }
         }
@@ -293,6 +317,7 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
   } else {
     reg_alloc<216>();
     // ------------------------------- consumers --------------------------------
+    pdl_wait();  // the scales of x come from the kernel in front; the stores may overwrite what it reads
     const int quarter = warp & 3;          // TMEM lane quarter this warp may read
     const int half = (warp - 4) >> 2;      // which 64 output columns
     const int row = quarter * 32 + lane;   // token row inside the tile
@@ -326,8 +351,8 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
         if (!GU_IN_RANGE(m_global >= 0 && m_global < p.m && (sg_row - p.scale_gate) / p.kb < w_blocks &&
                              (su_row - (kSingle ? p.scale_gate : p.scale_up)) / p.kb < w_blocks, kSiteTileScale))
           return;
-        sx0 = __ldg(sx_row); sg0 = __ldg(sg_row); su0 = __ldg(su_row);
-        if (p.kb > 1) { sx1 = __ldg(sx_row + 1); sg1 = __ldg(sg_row + 1); su1 = __ldg(su_row + 1); }
+        sx0 = ld_dep(sx_row); sg0 = ld_dep(sg_row); su0 = ld_dep(su_row);
+        if (p.kb > 1) { sx1 = ld_dep(sx_row + 1); sg1 = ld_dep(sg_row + 1); su1 = ld_dep(su_row + 1); }
       };
       if (tile < p.num_tiles) start_tile(tile);
 
@@ -342,7 +367,7 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
         for (int j = 0; j < p.kb; ++j) {
           // scales are fetched two K blocks ahead of their use
           float sx2 = 0.f, sg2 = 0.f, su2 = 0.f;
-          if (j + 2 < p.kb) { sx2 = __ldg(sx_row + j + 2); sg2 = __ldg(sg_row + j + 2); su2 = __ldg(su_row + j + 2); }
+          if (j + 2 < p.kb) { sx2 = ld_dep(sx_row + j + 2); sg2 = ld_dep(sg_row + j + 2); su2 = ld_dep(su_row + j + 2); }
           const float sgx = sx0 * sg0;
           const float sux = sx0 * su0;
           const float2 sg2v = make_float2(sgx, sgx);
@@ -525,11 +550,11 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
           g[i] = make_float2(0.f, 0.f);
           u[i] = make_float2(0.f, 0.f);
         }
-        float sx_n = __ldg(sx_row + jb), sg_n = __ldg(sg_row + jb), su_n = __ldg(su_row + jb);
+        float sx_n = ld_dep(sx_row + jb), sg_n = ld_dep(sg_row + jb), su_n = ld_dep(su_row + jb);
         for (int j = jb; j < je; ++j) {
           const float sgx = sx_n * sg_n;
           const float sux = sx_n * su_n;
-          if (j + 1 < je) { sx_n = __ldg(sx_row + j + 1); sg_n = __ldg(sg_row + j + 1); su_n = __ldg(su_row + j + 1); }
+          if (j + 1 < je) { sx_n = ld_dep(sx_row + j + 1); sg_n = ld_dep(sg_row + j + 1); su_n = ld_dep(su_row + j + 1); }
           const float2 sg2v = make_float2(sgx, sgx);
           const float2 su2v = make_float2(sux, sux);
           const bool ok = mbar_wait(ctx, my_acc_full + 8 * acc, acc_phase, kWaitTileAccFull);

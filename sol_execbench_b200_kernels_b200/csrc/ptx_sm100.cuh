@@ -296,6 +296,11 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t smem_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
 // hardware barrier over all threads of the cluster (cannot time out: only placed where every thread arrives)
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -348,6 +353,31 @@ __device__ __forceinline__ void umma_f8_pair(uint32_t tmem_d, uint64_t adesc, ui
 __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
                : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch.  A kernel launched with that attribute may start while the kernel in front of it in
+// the stream is still running: its blocks move in as the other's leave, and set up barriers, TMEM and descriptors.
+// pdl_wait() returns once every kernel in front has completed and its writes are visible; no thread touches memory
+// that another kernel may write (or still read) before it.  The one exception is weights that were complete before
+// the kernel in front began.  pdl_trigger() lets the next kernel start: from then on its blocks may take this grid's
+// place as its blocks leave.  A kernel that lets a successor prefetch weights triggers only after its own pdl_wait().
+// Both do nothing for a kernel launched without the attribute.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Load of a value that an earlier kernel wrote: volatile, so that it stays below pdl_wait(), and not through the
+// read-only path, which assumes that nothing writes the location while this kernel runs.
+__device__ __forceinline__ float ld_dep(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+// The same, 16 bytes that are read once.
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 
 // ---------------------------------------------------------------------------

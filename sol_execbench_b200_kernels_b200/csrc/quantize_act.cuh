@@ -19,6 +19,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx_sm100.cuh"
+
 namespace gu {
 
 constexpr int kQuantThreads = 256;
@@ -29,7 +31,7 @@ struct Raw8;
 template <>
 struct Raw8<__nv_bfloat16> {
   uint4 w;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { w = __ldcs(reinterpret_cast<const uint4*>(p)); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { w = ld_stream_v4(p); }
   __device__ __forceinline__ void zero() { w = make_uint4(0, 0, 0, 0); }
   // fp32 values and the largest magnitude (the maximum of bf16 values is exact in bf16: two elements per instruction)
   __device__ __forceinline__ float unpack(float (&v)[8]) const {
@@ -55,8 +57,9 @@ template <>
 struct Raw8<float> {
   float4 a, b;
   __device__ __forceinline__ void load(const float* p) {
-    a = __ldcs(reinterpret_cast<const float4*>(p));
-    b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+    const uint4 lo = ld_stream_v4(p), hi = ld_stream_v4(p + 4);
+    a = make_float4(__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(lo.w));
+    b = make_float4(__uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z), __uint_as_float(hi.w));
   }
   __device__ __forceinline__ void zero() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
   __device__ __forceinline__ float unpack(float (&v)[8]) const {
@@ -104,12 +107,14 @@ __host__ __device__ constexpr int quant_min_ctas() { return sizeof(T) == 2 ? 6 :
 // kPitched = false: rows are contiguous (ld_x == K), block b starts at element 128 * b and no division is needed.
 template <typename T, bool kPitched>
 __global__ void __launch_bounds__(kQuantThreads, quant_min_ctas<T>())
-quantize_act_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, uint32_t blocks,
+quantize_act_kernel(const T* x, uint8_t* __restrict__ q, float* __restrict__ scale, uint32_t blocks,
                     long long ld_x, uint32_t kb) {
   const int lane = threadIdx.x & 31;
   const int sub = lane & 15;                 // position inside the half-warp: elements 8*sub .. 8*sub+7 of the block
   constexpr int kQuantUnroll = quant_unroll<T>();
   const uint32_t half_warps = gridDim.x * (kQuantThreads / 16);
+  pdl_wait();
+  pdl_trigger();  // only now: a successor may prefetch weights that a kernel in front of this one has written
   // the host keeps blocks + kQuantUnroll * half_warps below 2^32
   for (uint32_t b = blockIdx.x * (kQuantThreads / 16) + (threadIdx.x >> 4); b < blocks; b += half_warps * kQuantUnroll) {
     Raw8<T> raw[kQuantUnroll];

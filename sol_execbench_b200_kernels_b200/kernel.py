@@ -236,19 +236,51 @@ def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch
               output: Optional[torch.Tensor] = None) -> torch.Tensor:
     """bf16 / fp32 activations [M, H] -> bf16 [M, H_out]: quantise, gate/up + SwiGLU (e4m3 out), down projection.
 
-    Three launches: `quantize_activation`, `run_fp8_output`, `blockwise_gemm`.  `down_proj_weight` is e4m3
-    [H_out, N] with scales [H_out/128, N/128].  The intermediate [M, N] exists only as e4m3 + scales.
+    One call into the library, three launches (the steps of `quantize_activation`, `run_fp8_output` and
+    `blockwise_gemm`).  `down_proj_weight` is e4m3 [H_out, N] with scales [H_out/128, N/128].  The intermediate [M, N]
+    exists only as e4m3 + scales.  With few tokens the library cuts tiles along K (see gu_mlp_block in gateup.h).
     """
-    m = x.shape[0]
-    n = gate_proj_weight.shape[0]
-    h_out = down_proj_weight.shape[0]
-    xq, sx = quantize_activation(x)
-    mid_q = torch.empty(m, n, dtype=torch.float8_e4m3fn, device=x.device)
-    mid_s = torch.empty(m, n // BLOCK, dtype=torch.float32, device=x.device)
-    run_fp8_output(xq, sx, gate_proj_weight, scale_gate, up_proj_weight, scale_up, mid_q, mid_s)
+    m, k = _activation_shape(x)
+    if gate_proj_weight.dim() != 2 or up_proj_weight.dim() != 2:
+        raise ValueError("x, gate_proj_weight and up_proj_weight must be 2-D")
+    if down_proj_weight.dim() != 2 or (output is not None and output.dim() != 2):
+        raise ValueError("a, b and output must be 2-D")
+    n, h_out = gate_proj_weight.shape[0], down_proj_weight.shape[0]
+    for rows, cols in ((n, k), (h_out, n)):
+        if cols % BLOCK or rows % BLOCK or cols < BLOCK or rows < BLOCK:
+            raise ValueError(f"Unsupported contract shape M={m}, K={cols}, N={rows}: need M >= 1 and K, N multiples of {BLOCK}")
+    kb, nb, hb = k // BLOCK, n // BLOCK, h_out // BLOCK
+    expected = {
+        "gate_proj_weight": (gate_proj_weight, (n, k), torch.float8_e4m3fn),
+        "scale_gate": (scale_gate, (nb, kb), torch.float32),
+        "up_proj_weight": (up_proj_weight, (n, k), torch.float8_e4m3fn),
+        "scale_up": (scale_up, (nb, kb), torch.float32),
+        "b": (down_proj_weight, (h_out, n), torch.float8_e4m3fn),
+        "scale_b": (scale_down, (hb, nb), torch.float32),
+    }
+    if output is not None:
+        expected["output"] = (output, (m, h_out), torch.bfloat16)
+    _check(expected, x.device)
     if output is None:
         output = torch.empty(m, h_out, dtype=torch.bfloat16, device=x.device)
-    blockwise_gemm(mid_q, mid_s, down_proj_weight, scale_down, output)
+    elif output.stride(1) != 1 or output.stride(0) < h_out:
+        raise ValueError("output must be row-major with unit column stride")
+    # one allocation for the quantised activations and the quantised intermediate with their scales
+    offsets, nbytes = [], 0
+    for size in (m * k, 4 * m * kb, m * n, 4 * m * nb):
+        offsets.append(nbytes)
+        nbytes += (size + 255) // 256 * 256
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    base = scratch.data_ptr()
+    block = _cabi.GuMlp(
+        x.data_ptr(), gate_proj_weight.data_ptr(), scale_gate.data_ptr(), up_proj_weight.data_ptr(), scale_up.data_ptr(),
+        down_proj_weight.data_ptr(), scale_down.data_ptr(), base + offsets[0], base + offsets[1], base + offsets[2],
+        base + offsets[3], output.data_ptr(), m, k, n, h_out, x.stride(0), output.stride(0),
+        1 if x.dtype == torch.float32 else 0, 0)
+    with torch.cuda.device(x.device):
+        stream_ptr = torch.cuda.current_stream(x.device).cuda_stream
+        code = _cabi.lib.gu_mlp_block(ctypes.byref(block), stream_ptr)
+    _raise_for(code)
     return output
 
 
@@ -338,14 +370,8 @@ def peer_barrier(rank_flag_ptrs, rank: int, device, limit_ns: int = 0) -> None:
     _raise_for(code)
 
 
-@torch.no_grad()
-def quantize_activation(x: torch.Tensor, q: Optional[torch.Tensor] = None,
-                        scale: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
-    """bf16 / fp32 activations [M, K] -> (e4m3 [M, K], fp32 scales [M, K/128]), scale = block amax / 448.
-
-    The producer of `run`'s first two arguments (the reference receives them ready-made:
-    kernel.py:356-357).  One streaming kernel on the current stream; rows of `x` may be pitched.
-    """
+def _activation_shape(x: torch.Tensor) -> Tuple[int, int]:
+    """(M, K) of activations the quantiser takes; raises ValueError otherwise."""
     if x.dim() != 2 or x.dtype not in (torch.bfloat16, torch.float32):
         raise ValueError("x must be a 2-D bf16 or fp32 tensor")
     if not x.is_cuda:
@@ -355,6 +381,18 @@ def quantize_activation(x: torch.Tensor, q: Optional[torch.Tensor] = None,
         raise ValueError(f"Unsupported shape M={m}, K={k}: need M >= 1 and K a multiple of {BLOCK}")
     if x.stride(1) != 1 or x.stride(0) < k:
         raise ValueError("x must be row-major with unit column stride")
+    return m, k
+
+
+@torch.no_grad()
+def quantize_activation(x: torch.Tensor, q: Optional[torch.Tensor] = None,
+                        scale: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
+    """bf16 / fp32 activations [M, K] -> (e4m3 [M, K], fp32 scales [M, K/128]), scale = block amax / 448.
+
+    The producer of `run`'s first two arguments (the reference receives them ready-made:
+    kernel.py:356-357).  One streaming kernel on the current stream; rows of `x` may be pitched.
+    """
+    m, k = _activation_shape(x)
     if q is None:
         q = torch.empty(m, k, dtype=torch.float8_e4m3fn, device=x.device)
     if scale is None:

@@ -1,0 +1,103 @@
+"""The K-split kernel (a cluster of CTAs per tile): `run` and `mlp_block` on shapes with few tiles, against the same
+operations with whole tiles, which the other tests hold against the oracle."""
+import pytest
+import torch
+
+from sol_execbench_b200_kernels_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(out, ref, rel_limit, what):
+    rel = float(torch.linalg.vector_norm(out.float() - ref.float()) / torch.linalg.vector_norm(ref.float()))
+    assert bool(torch.isfinite(out.float()).all()) and rel <= rel_limit, (what, rel)
+
+
+# tokens at the edges of a warp's 32 rows and of the 128-row tile; K blocks that no cluster size divides; one column
+# block (8 CTAs) up to as many tiles as still leave two CTAs each
+@pytest.mark.parametrize("m,kb,nb", [(1, 33, 1), (31, 56, 18), (33, 32, 18), (128, 35, 13), (129, 40, 9), (200, 17, 30),
+                                     (257, 32, 24), (7, 8, 74), (64, 12, 48), (5, 64, 25)])
+def test_gateup_cut_along_k(m, kb, nb):
+    import sol_execbench_b200_kernels_b200 as pkg
+
+    k, n = 128 * kb, 128 * nb
+    inp = W.make_inputs(m, k, n, seed=m, device="cuda:0")
+    whole = torch.empty(m, n, dtype=torch.bfloat16, device="cuda:0")
+    pkg.run_with_plan(*inp.args(), whole, "tile_dp")
+    wide = torch.full((m + 1, n + 128), 7.0, dtype=torch.bfloat16, device="cuda:0")
+    pkg.run_with_plan(*inp.args(), wide[:m, :n], "tile")
+    again = torch.empty_like(whole)
+    pkg.run_with_plan(*inp.args(), again, "tile")
+    kept = torch.empty_like(whole)
+    pkg.run_with_plan(*inp.args(), kept, "tile", whole_tiles=True)
+    torch.cuda.synchronize()
+    assert pkg.last_status()[0] == 0
+    # up to eight fp32 partial sums joined: a bf16 rounding flips where a sum is within 2^-24 * 8 of a tie
+    _close(wide[:m, :n], whole, 1e-4, (m, k, n))
+    assert float((wide[:m, :n] != whole).float().mean()) <= 5e-3
+    assert torch.equal(wide[:m, :n], again)  # the order of the sums is fixed
+    assert torch.equal(kept, whole)
+    assert bool((wide[m] == 7.0).all()) and bool((wide[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("m,kb,nb,hb", [(1, 4, 40, 1), (8, 32, 112, 32), (8, 9, 33, 3), (31, 7, 18, 5), (128, 16, 35, 16),
+                                        (129, 24, 18, 8), (300, 32, 24, 12), (515, 8, 112, 8), (1, 1, 1, 1)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_mlp_block_cut_along_k(m, kb, nb, hb, dtype):
+    import sol_execbench_b200_kernels_b200 as pkg
+
+    k, n, h = 128 * kb, 128 * nb, 128 * hb
+    g = torch.Generator(device="cuda:0").manual_seed(m)
+    x = torch.randn(m, k + 8, generator=g, device="cuda:0").to(dtype)[:, :k]  # pitched rows
+    weights = []
+    for rows, cols in ((n, k), (n, k), (h, n)):
+        weights += W.quantize_weight_128x128(torch.randn(rows, cols, generator=g, device="cuda:0") * 0.02)
+    xq, sx = pkg.quantize_activation(x)
+    mid_q = torch.empty(m, n, dtype=torch.float8_e4m3fn, device="cuda:0")
+    mid_s = torch.empty(m, nb, device="cuda:0")
+    pkg.run_fp8_output(xq, sx, *weights[:4], mid_q, mid_s)
+    ref = torch.empty(m, h, dtype=torch.bfloat16, device="cuda:0")
+    pkg.blockwise_gemm(mid_q, mid_s, *weights[4:], ref)
+    wide = torch.full((m + 1, h + 128), 7.0, dtype=torch.bfloat16, device="cuda:0")
+    pkg.mlp_block(x, *weights, wide[:m, :h])
+    own = pkg.mlp_block(x, *weights)
+    torch.cuda.synchronize()
+    assert pkg.last_status()[0] == 0
+    # a flipped bf16 rounding may move an e4m3 value of the intermediate by a step (2^-3 relative, on fewer than one in
+    # a thousand values)
+    _close(own, ref, 2e-3, (m, k, n, h))
+    assert torch.equal(wide[:m, :h], own)
+    assert bool((wide[m] == 7.0).all()) and bool((wide[:, h:] == 7.0).all())
+
+
+def test_mlp_block_in_a_graph_and_after_a_weight_update():
+    """The block's kernels start before the ones in front of them have ended: weights written just before the call have
+    to be the ones that count, in eager calls and in replays."""
+    import sol_execbench_b200_kernels_b200 as pkg
+
+    m, k, n = 8, 2048, 5632
+    g = torch.Generator(device="cuda:0").manual_seed(3)
+    x = torch.randn(m, k, generator=g, device="cuda:0").bfloat16()
+    sets = []
+    for _ in range(2):
+        s = []
+        for rows, cols in ((n, k), (n, k), (k, n)):
+            s += W.quantize_weight_128x128(torch.randn(rows, cols, generator=g, device="cuda:0") * 0.02)
+        sets.append(s)
+    want = [pkg.mlp_block(x, *s).clone() for s in sets]
+    live = [t.clone() for t in sets[0]]
+    out = torch.empty_like(want[0])
+    pkg.mlp_block(x, *live, out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        pkg.mlp_block(x, *live, out)
+    for trial in range(20):
+        for dst, src in zip(live, sets[trial % 2]):
+            dst.view(torch.uint8).copy_(src.view(torch.uint8))
+        if trial % 4 < 2:
+            pkg.mlp_block(x, *live, out)
+        else:
+            graph.replay()
+        assert torch.equal(out, want[trial % 2]), trial
+    assert pkg.last_status()[0] == 0
