@@ -12,8 +12,12 @@
 //                  `hidden` and HALF of the 256 weight rows of a K block (32 KiB per CTA and 64-wide K block), the
 //                  even CTA issues cta_group::2 MMAs (M = 256, N = 256, K = 16) for both; each CTA finds its
 //                  128 x 256 fp32 accumulator in its own TMEM.  Used for M > 128.
-//   kPair = false  one CTA owns a 128-row x 256-column tile and stages all 256 weight rows (48 KiB per K block).
-//                  Used for M <= 128, where the second CTA of a pair would have no rows.
+//   kPair = false  one CTA owns a 128-row x tile_n-column tile (tile_n <= 256) and stages all its weight rows.  Used
+//                  for M <= 128, where the second CTA of a pair would have no rows.  That launch is bound by how fast
+//                  the SMs pull the weights from HBM, so the host picks the narrowest tile (a multiple of 32 columns)
+//                  with which one round of tiles still covers N, and the ring takes the whole shared memory: the
+//                  staging tiles then lie in the ring, idle once a CTA's only tile has been accumulated.  At M = 128,
+//                  K = 8192, N = 32768: 147 CTAs with 224 columns and 5 stages instead of 128 with 256 and 4.
 //
 // Warp roles (192 threads): warp 0 TMA producer, warp 1 TMEM allocation and (in the even CTA) MMA issue, warps 2-5
 // epilogue: a warp reads TMEM lanes 32 (w % 4) .. +31 in chunks of 64 columns, adds the bias in fp32, rounds to bf16
@@ -39,13 +43,18 @@ constexpr uint32_t kPjOutChunkBytes = kPjTileM * 128;   // 128 rows x 64 bf16
 constexpr uint32_t kPjOutBytes = 2 * kPjOutChunkBytes;
 constexpr uint32_t kPjTmemCols = 512;         // two 256-column fp32 accumulators
 
+constexpr int kPjMaxStages = 8;
+constexpr uint32_t kPjFixedBytes = 256 /*barriers*/ + 1024 /*alignment*/;
+
 template <bool kPair>
 struct PjCfg {
-  static constexpr int b_rows = kPair ? 128 : 256;  // weight rows this CTA stages per K block
-  static constexpr uint32_t stage_bytes = kPjATileBytes + b_rows * 128;
-  static constexpr int stages = kPair ? 6 : 4;
-  static constexpr uint32_t smem_bytes = stages * stage_bytes + kPjOutBytes + 256 /*barriers*/ + 1024 /*alignment*/;
+  static constexpr int pair_b_rows = 128;  // weight rows each CTA of a pair stages per K block
+  static constexpr int pair_stages = 6;
   static constexpr int rows_per_tile = kPair ? 2 * kPjTileM : kPjTileM;
+  __host__ __device__ static constexpr uint32_t stage_bytes(int b_rows) {
+    return kPjATileBytes + static_cast<uint32_t>(b_rows) * 128;
+  }
+  static constexpr uint32_t pair_smem_bytes = pair_stages * (kPjATileBytes + pair_b_rows * 128) + kPjOutBytes + kPjFixedBytes;
 };
 
 enum : unsigned { kWaitPjSlot = 40, kWaitPjFull = 41, kWaitPjAccFree = 42, kWaitPjAccFull = 43 };
@@ -54,9 +63,12 @@ enum : unsigned { kSitePjLoad = 49, kSitePjStage = 50, kSitePjStore = 51, kSiteP
 
 struct ProjParams {
   const __nv_bfloat16* bias;  // [N]
+  __nv_bfloat16* out;         // [M, N] (lone CTAs: a last chunk of 32 columns is stored without TMA)
   int m, n, kb;               // kb = ceil(K / 64)
   int m_tiles, n_tiles, num_tiles;
   int group_m;                // raster: tiles walk `group_m` row tiles at a time, row tile fastest
+  int tile_n, stages;         // lone CTAs: columns per tile (a multiple of 32, at most 256) and ring depth
+  int staging_in_ring;        // lone CTAs: no CTA has a second tile, so the staging tiles may lie in the idle ring
 };
 
 // Instruction descriptor, kind::f16: D fp32 (bits 4-5 = 1), A and B bf16 (format 1 at bits 7-9 and 10-12), both
@@ -113,12 +125,17 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
 
+  const uint32_t stages = kPair ? Cfg::pair_stages : p.stages;
+  const int tile_n = kPair ? kPjTileN : p.tile_n;
+  const int b_rows = kPair ? Cfg::pair_b_rows : p.tile_n;  // weight rows this CTA stages per K block
+  const uint32_t stage_bytes = Cfg::stage_bytes(b_rows);
   const uint32_t ring = smem_base;
-  const uint32_t stag = ring + Cfg::stages * Cfg::stage_bytes;
-  const uint32_t bars = stag + kPjOutBytes;
+  const bool in_ring = !kPair && p.staging_in_ring;
+  const uint32_t stag = in_ring ? ring : ring + stages * stage_bytes;
+  const uint32_t bars = ring + stages * stage_bytes + (in_ring ? 0u : kPjOutBytes);
   const uint32_t bar_full = bars;                             // [stages] pair: the even CTA's, 2 arrivals + both CTAs' bytes
-  const uint32_t bar_empty = bar_full + 8 * Cfg::stages;      // [stages] one commit: the slot's MMAs have read it
-  const uint32_t bar_acc_full = bar_empty + 8 * Cfg::stages;  // [2] one commit: the tile's accumulator is complete
+  const uint32_t bar_empty = bar_full + 8 * kPjMaxStages;      // [stages] one commit: the slot's MMAs have read it
+  const uint32_t bar_acc_full = bar_empty + 8 * kPjMaxStages;  // [2] one commit: the tile's accumulator is complete
   const uint32_t bar_acc_free = bar_acc_full + 16;            // [2] pair: the even CTA's; 4 epilogue warps per CTA
   const uint32_t tmem_slot = bar_acc_free + 16;
   const uint32_t abort_slot = tmem_slot + 4;
@@ -132,7 +149,8 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
   const int units = kPair ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < Cfg::stages; ++s) {
+    pdl_trigger();
+    for (uint32_t s = 0; s < stages; ++s) {
       mbar_init(bar_full + 8 * s, kPair ? 2 : 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
@@ -161,6 +179,7 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
+  pdl_wait();
 
   WaitCtx ctx{abort_slot, false, kPair};
 
@@ -173,26 +192,26 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
       int tm, tn;
       pj_tile_coords(p, tile, tm, tn);
       const int row0 = tm * Cfg::rows_per_tile + static_cast<int>(rank) * kPjTileM;
-      const int wrow0 = tn * kPjTileN + static_cast<int>(rank) * Cfg::b_rows;  // (rank is 0 without pairs)
+      const int wrow0 = tn * tile_n + static_cast<int>(rank) * b_rows;  // (rank is 0 without pairs)
       for (int j = 0; j < p.kb; ++j, ++slots) {
-        const uint32_t stage = slots % Cfg::stages, phase = (slots / Cfg::stages) & 1u;
+        const uint32_t stage = slots % stages, phase = (slots / stages) & 1u;
         const bool ok = pj_wait_elected(ctx, elected, bar_empty + 8 * stage, phase ^ 1u, kWaitPjSlot);
         const uint32_t full = full_base + 8 * stage;
-        const uint32_t dst = ring + stage * Cfg::stage_bytes;
+        const uint32_t dst = ring + stage * stage_bytes;
         // (loads may start past the last row of a ragged tile, where they read zeros, but never before row 0, past the
         // padded row range, or at a K offset that is not 16-byte aligned)
-        if (ok && elected && GU_IN_RANGE(stage < static_cast<uint32_t>(Cfg::stages), kSitePjStage) &&
+        if (ok && elected && GU_IN_RANGE(stage < stages && stages <= kPjMaxStages, kSitePjStage) &&
             GU_IN_RANGE(tm >= 0 && tm < p.m_tiles && tn >= 0 && tn < p.n_tiles, kSitePjTile) &&
             GU_IN_RANGE(j >= 0 && j < p.kb && ((j * kPjBlockK * 2) & 15) == 0 && row0 >= 0 &&
-                            row0 < p.m_tiles * Cfg::rows_per_tile && wrow0 >= 0 && wrow0 < p.n_tiles * kPjTileN,
+                            row0 < p.m_tiles * Cfg::rows_per_tile && wrow0 >= 0 && wrow0 < p.n_tiles * tile_n,
                         kSitePjLoad)) {
           // rows past M / N and columns past K read as zero
           if constexpr (kPair) {
-            mbar_arrive_expect_tx_cluster(full, Cfg::stage_bytes);
+            mbar_arrive_expect_tx_cluster(full, stage_bytes);
             tma_load_2d_pair(dst, &tm_a, full, j * kPjBlockK, row0);
             tma_load_2d_pair(dst + kPjATileBytes, &tm_w, full, j * kPjBlockK, wrow0);
           } else {
-            mbar_arrive_expect_tx(full, Cfg::stage_bytes);
+            mbar_arrive_expect_tx(full, stage_bytes);
             tma_load_2d(dst, &tm_a, full, j * kPjBlockK, row0);
             tma_load_2d(dst + kPjATileBytes, &tm_w, full, j * kPjBlockK, wrow0);
           }
@@ -201,13 +220,13 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
       }
     }
     // the last commits into this CTA's ring barriers must have landed before the CTA may go away
-    for (int s = 0; s < Cfg::stages; ++s, ++slots)
-      pj_wait_elected(ctx, elected, bar_empty + 8 * (slots % Cfg::stages), ((slots / Cfg::stages) & 1u) ^ 1u, kWaitPjSlot);
+    for (uint32_t s = 0; s < stages; ++s, ++slots)
+      pj_wait_elected(ctx, elected, bar_empty + 8 * (slots % stages), ((slots / stages) & 1u) ^ 1u, kWaitPjSlot);
   } else if (warp == 1) {
     if (rank == 0) {
       // ---------------- MMA issuer: the whole warp walks the loop, one elected lane waits and issues ----------------
       const bool elected = elect_one() != 0u;
-      constexpr uint32_t idesc = umma_idesc_bf16_f32(Cfg::rows_per_tile, kPjTileN);
+      const uint32_t idesc = umma_idesc_bf16_f32(Cfg::rows_per_tile, tile_n);
       const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
       const uint32_t empty_odd = kPair ? mapa_shared(bar_empty, 1) : 0u;
       const uint32_t acc_full_odd = kPair ? mapa_shared(bar_acc_full, 1) : 0u;
@@ -219,9 +238,9 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
         const uint32_t d = tmem_u + acc * kPjTileN;
         bool ok = pj_wait_elected(ctx, elected, bar_acc_free + 8 * acc, acc_phase ^ 1u, kWaitPjAccFree);
         for (int j = 0; j < p.kb; ++j, ++blocks) {
-          const uint32_t stage = blocks % Cfg::stages, phase = (blocks / Cfg::stages) & 1u;
-          const uint64_t adesc = adesc0 + stage * (Cfg::stage_bytes >> 4);
-          const uint64_t bdesc = bdesc0 + stage * (Cfg::stage_bytes >> 4);
+          const uint32_t stage = blocks % stages, phase = (blocks / stages) & 1u;
+          const uint64_t adesc = adesc0 + stage * (stage_bytes >> 4);
+          const uint64_t bdesc = bdesc0 + stage * (stage_bytes >> 4);
           ok = pj_wait_elected(ctx, elected, bar_full + 8 * stage, phase, kWaitPjFull) && ok;
           if (ok && elected) {
             tc_fence_after();
@@ -260,24 +279,26 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
       int tm, tn;
       pj_tile_coords(p, tile, tm, tn);
       const int row0 = tm * Cfg::rows_per_tile + static_cast<int>(rank) * kPjTileM;
-      const int col0 = tn * kPjTileN;
+      const int col0 = tn * tile_n;
+      const int chunks = (tile_n + 63) / 64;
       const uint32_t acc = tiles_done & 1u, acc_phase = (tiles_done >> 1) & 1u;
       const bool ok = pj_wait_elected(ctx, lane == 0, bar_acc_full + 8 * acc, acc_phase, kWaitPjAccFull);
       tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < kPjTileN / 64; ++c) {
+      for (int c = 0; c < chunks; ++c) {
         const int colc = col0 + 64 * c;
+        const bool narrow = !kPair && 64 * c + 64 > tile_n;  // the last 32 columns of a tile
         float v[64];
         tmem_ld32(lane_addr + acc * kPjTileN + 64 * c, v);
-        tmem_ld32(lane_addr + acc * kPjTileN + 64 * c + 32, v + 32);
+        tmem_ld32(lane_addr + acc * kPjTileN + 64 * c + 32, v + 32);  // (narrow: columns of no tile, not used)
         uint4 bq[8];  // this chunk's 64 bias values (the same for every row: broadcast loads)
 #pragma unroll
         for (int q = 0; q < 8; ++q)
           bq[q] = (colc + 8 * q < p.n && GU_IN_RANGE(colc + 8 * q >= 0 && colc + 8 * q + 8 <= p.n, kSitePjBias))
-                      ? __ldg(reinterpret_cast<const uint4*>(p.bias + colc + 8 * q))
+                      ? ld_dep(reinterpret_cast<const uint4*>(p.bias + colc + 8 * q))
                       : make_uint4(0, 0, 0, 0);
         tmem_ld_wait_pin<64>(v);
-        if (c + 1 == kPjTileN / 64) {
+        if (c + 1 == chunks) {
           // the whole accumulator is in registers or stored: hand it back to the issuer
           tc_fence_before();
           __syncwarp();
@@ -299,13 +320,20 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
             const float b_lo = __uint_as_float(bw[i] << 16), b_hi = __uint_as_float(bw[i] & 0xffff0000u);
             o[i] = pack_bf16x2(v[8 * q + 2 * i] + b_lo, v[8 * q + 2 * i + 1] + b_hi);
           }
-          *reinterpret_cast<uint4*>(dst_row + ((q ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+          if (!narrow) {
+            *reinterpret_cast<uint4*>(dst_row + ((q ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+          } else if (q < 4 && row0 + row < p.m && colc + 8 * q < p.n && ok && !ctx.aborted &&
+                     GU_IN_RANGE(row0 + row >= 0 && colc + 8 * q + 8 <= p.n, kSitePjStore)) {
+            // a 64-column TMA store would write into the next tile; N is a multiple of 8
+            *reinterpret_cast<uint4*>(p.out + static_cast<size_t>(row0 + row) * p.n + colc + 8 * q) =
+                make_uint4(o[0], o[1], o[2], o[3]);
+          }
         }
         fence_proxy_async_smem();
         named_bar_sync(2, 128);
         // (a store may reach past the last row or column, where it is clipped, but starts inside the tensor)
         if (et == 0) {
-          if (ok && !ctx.aborted && row0 < p.m && colc < p.n &&
+          if (!narrow && ok && !ctx.aborted && row0 < p.m && colc < p.n &&
               GU_IN_RANGE(row0 >= 0 && colc >= 0 && ((colc * 2) & 15) == 0, kSitePjStore))
             tma_store_2d(&tm_out, stag + (c & 1) * kPjOutChunkBytes, colc, row0);  // rows past M, columns past N are clipped
           // one group per chunk, also when the chunk lies outside the tensor and nothing is stored (an empty group):

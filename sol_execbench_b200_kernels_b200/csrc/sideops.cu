@@ -180,10 +180,9 @@ __device__ __forceinline__ void sigmoid_2x2(uint32_t ca, uint32_t cb, uint32_t& 
   sb = float2_to_bf16x2(__fmul2_rn(rab, ya));   // 1/yb
 }
 
-__global__ void __launch_bounds__(kConvThreads)  // 48 registers: 5 CTAs per SM; forcing 6 (40 registers) measured 7 % slower
-mamba_conv1d_tail_kernel(const __nv_bfloat16* __restrict__ projected, const __nv_bfloat16* __restrict__ mask,
-                         const __nv_bfloat16* __restrict__ conv_weight, const __nv_bfloat16* __restrict__ conv_bias,
-                         __nv_bfloat16* __restrict__ output, int sequence, int channels, long long width) {
+__global__ void __launch_bounds__(kConvThreads, 5)  // 48 registers: 5 CTAs per SM; forcing 6 (40 registers) measured 7 % slower
+mamba_conv1d_tail_kernel(const __nv_bfloat16* projected, const __nv_bfloat16* mask, const __nv_bfloat16* conv_weight,
+                         const __nv_bfloat16* conv_bias, __nv_bfloat16* output, int sequence, int channels, long long width) {
   __shared__ __align__(16) uint32_t s_in[kConvRows * (kConvChannels / 2)];  // [row][channel pair]
   __shared__ __align__(8) uint32_t s_out[kConvChannels * kConvOutPitch];                 // [channel][position pair]
   __shared__ uint32_t s_keep[kConvPositions / 2];  // per position pair: 0xffff in the half of a kept position
@@ -199,6 +198,8 @@ mamba_conv1d_tail_kernel(const __nv_bfloat16* __restrict__ projected, const __nv
   // addresses advance by a constant; all of its global loads are issued before the first use ----
   constexpr int kLoadsPerThread = (kConvRows + 31) / 32;  // 5; the last round has 3 rows
   const int l_first = l0 + (tid >> 3) - (kConvTaps - 1);
+  if (tid == 0) gu::pdl_trigger();
+  gu::pdl_wait();  // every load below is a volatile one, so none moves above this
   uint4 raw[kLoadsPerThread];
   uint32_t m2[kLoadsPerThread];
   {
@@ -211,8 +212,8 @@ mamba_conv1d_tail_kernel(const __nv_bfloat16* __restrict__ projected, const __nv
       raw[i] = make_uint4(0u, 0u, 0u, 0u);
       m2[i] = 0u;
       if ((i < kLoadsPerThread - 1 || tid < 8 * (kConvRows - 32 * (kLoadsPerThread - 1))) && l >= 0 && l < sequence) {
-        raw[i] = __ldcs(src + off);
-        const uint32_t mb = __ldg(mask_bits + l);
+        raw[i] = gu::ld_stream_v4(src + off);
+        const uint32_t mb = gu::ld_dep(mask_bits + l);
         m2[i] = mb | (mb << 16);
       }
       off += 32 * row_pitch;
@@ -222,8 +223,8 @@ mamba_conv1d_tail_kernel(const __nv_bfloat16* __restrict__ projected, const __nv
     // the reference keeps an output only where the mask is at least one half (bf16 bits 0x3f00 .. 0x7f80)
     uint32_t keep = 0u;
     const int l = l0 + 2 * tid;
-    if (l < sequence && __ldg(mask_bits + l) - 0x3f00u <= 0x4080u) keep |= 0x0000ffffu;
-    if (l + 1 < sequence && __ldg(mask_bits + l + 1) - 0x3f00u <= 0x4080u) keep |= 0xffff0000u;
+    if (l < sequence && gu::ld_dep(mask_bits + l) - 0x3f00u <= 0x4080u) keep |= 0x0000ffffu;
+    if (l + 1 < sequence && gu::ld_dep(mask_bits + l + 1) - 0x3f00u <= 0x4080u) keep |= 0xffff0000u;
     s_keep[tid] = keep;
   }
 #pragma unroll
@@ -246,14 +247,14 @@ mamba_conv1d_tail_kernel(const __nv_bfloat16* __restrict__ projected, const __nv
   float2 w[4], bias;
   {
     const int c = c0 + 2 * lane;
-    const uint4 wq = __ldg(reinterpret_cast<const uint4*>(conv_weight + static_cast<long long>(c) * kConvTaps));
+    const uint4 wq = gu::ld_dep(reinterpret_cast<const uint4*>(conv_weight + static_cast<long long>(c) * kConvTaps));
     const float2 wa01 = bf16x2_to_float2(wq.x), wa23 = bf16x2_to_float2(wq.y);  // channel c, taps 0..3
     const float2 wb01 = bf16x2_to_float2(wq.z), wb23 = bf16x2_to_float2(wq.w);  // channel c + 1
     w[0] = make_float2(wa01.x, wb01.x);
     w[1] = make_float2(wa01.y, wb01.y);
     w[2] = make_float2(wa23.x, wb23.x);
     w[3] = make_float2(wa23.y, wb23.y);
-    bias = bf16x2_to_float2(__ldg(reinterpret_cast<const uint32_t*>(conv_bias + c)));
+    bias = bf16x2_to_float2(gu::ld_dep(reinterpret_cast<const uint32_t*>(conv_bias + c)));
   }
   __syncthreads();
 
@@ -367,6 +368,33 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+constexpr uint32_t kPjSmemBudget = 227 * 1024;
+
+// One launch with the programmatic-serialisation attribute (see pdl_wait): the kernel's blocks move in while the kernel
+// in front drains.
+template <typename... Params, typename... Args>
+int launch(void (*kernel)(Params...), dim3 grid, int threads, uint32_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  std::memset(&attr, 0, sizeof(attr));
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return SO_ECUDA;
+  }
+  return SO_OK;
+}
+
 // resolved through the runtime, so the library has no link-time dependency on the driver library
 EncodeTiledFn encode_tiled_fn() {
   static EncodeTiledFn fn = [] {
@@ -414,9 +442,9 @@ int proj_device(ProjDevice** out) {
       return SO_ECUDA;
     if (major != 10) return SO_EDEVICE;
     if (cudaFuncSetAttribute(proj_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             PjCfg<true>::smem_bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(proj_gemm_lone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             PjCfg<false>::smem_bytes) != cudaSuccess) {
+                             PjCfg<true>::pair_smem_bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(proj_gemm_lone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPjSmemBudget) !=
+            cudaSuccess) {
       cudaGetLastError();
       return SO_ECUDA;
     }
@@ -424,7 +452,7 @@ int proj_device(ProjDevice** out) {
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(2 * static_cast<unsigned>(d.sm_count), 1, 1);
     cfg.blockDim = dim3(kPjThreads, 1, 1);
-    cfg.dynamicSmemBytes = PjCfg<true>::smem_bytes;
+    cfg.dynamicSmemBytes = PjCfg<true>::pair_smem_bytes;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2;
@@ -452,16 +480,22 @@ int launch_projection(const void* hidden, const void* weight, const void* bias, 
   const bool pair = m > kPjTileM && dev->pair_clusters >= 1;
   CUtensorMap tm_a, tm_w, tm_o;
   if ((rc = bf16_map(&tm_a, hidden, k, m, kPjTileM)) != SO_OK) return rc;
-  if ((rc = bf16_map(&tm_w, weight, k, n, pair ? PjCfg<true>::b_rows : PjCfg<false>::b_rows)) != SO_OK) return rc;
+  // lone CTAs: the narrowest tile with which one round of tiles covers N (see proj_gemm.cuh); 256 columns otherwise
+  int tile_n = kPjTileN;
+  if (!pair)
+    for (int w = kPjTileN; w >= 64 && (n + w - 1) / w <= dev->sm_count; w -= 32) tile_n = w;
+  if ((rc = bf16_map(&tm_w, weight, k, n, pair ? PjCfg<true>::pair_b_rows : tile_n)) != SO_OK) return rc;
   if ((rc = bf16_map(&tm_o, projected, n, m, kPjTileM)) != SO_OK) return rc;
   ProjParams p;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.out = static_cast<__nv_bfloat16*>(projected);
+  p.tile_n = tile_n;
   p.m = static_cast<int>(m);
   p.n = static_cast<int>(n);
   p.kb = static_cast<int>((k + kPjBlockK - 1) / kPjBlockK);
   const int rows_per_tile = pair ? PjCfg<true>::rows_per_tile : PjCfg<false>::rows_per_tile;
   p.m_tiles = static_cast<int>((m + rows_per_tile - 1) / rows_per_tile);
-  p.n_tiles = static_cast<int>((n + kPjTileN - 1) / kPjTileN);
+  p.n_tiles = static_cast<int>((n + tile_n - 1) / tile_n);
   const int64_t tiles = int64_t(p.m_tiles) * p.n_tiles;
   if (tiles * p.kb >= (1ll << 31)) return SO_EINVAL_SHAPE;
   p.num_tiles = static_cast<int>(tiles);
@@ -470,13 +504,19 @@ int launch_projection(const void* hidden, const void* weight, const void* bias, 
   p.group_m = p.m_tiles < 8 ? p.m_tiles : 8;
   if (pair) {
     const int clusters = p.num_tiles < dev->pair_clusters ? p.num_tiles : dev->pair_clusters;
-    proj_gemm_pair_kernel<<<2 * clusters, kPjThreads, PjCfg<true>::smem_bytes, stream>>>(tm_a, tm_w, tm_o, p);
-  } else {
-    const int ctas = p.num_tiles < dev->sm_count ? p.num_tiles : dev->sm_count;
-    proj_gemm_lone_kernel<<<ctas, kPjThreads, PjCfg<false>::smem_bytes, stream>>>(tm_a, tm_w, tm_o, p);
+    p.stages = PjCfg<true>::pair_stages;
+    p.staging_in_ring = 0;
+    return launch(proj_gemm_pair_kernel, dim3(2 * clusters), kPjThreads, PjCfg<true>::pair_smem_bytes, stream, tm_a, tm_w, tm_o,
+                  p);
   }
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? SO_OK : SO_ECUDA;
+  const int ctas = p.num_tiles < dev->sm_count ? p.num_tiles : dev->sm_count;
+  const uint32_t stage_bytes = PjCfg<false>::stage_bytes(tile_n);
+  p.staging_in_ring = p.num_tiles <= dev->sm_count;
+  const uint32_t staging = p.staging_in_ring ? 0u : kPjOutBytes;
+  const uint32_t fit = (kPjSmemBudget - kPjFixedBytes - staging) / stage_bytes;  // 4 .. 9
+  p.stages = static_cast<int>(fit < kPjMaxStages ? fit : kPjMaxStages);
+  return launch(proj_gemm_lone_kernel, dim3(ctas), kPjThreads, p.stages * stage_bytes + staging + kPjFixedBytes, stream, tm_a,
+                tm_w, tm_o, p);
 }
 
 }  // namespace so
@@ -537,12 +577,11 @@ int so_mamba_conv1d_tail(const void* projected, const void* attention_mask, cons
   if (seq_tiles > 65535) return SO_EINVAL_SHAPE;
   const dim3 grid(static_cast<unsigned>(channels / so::kConvChannels), static_cast<unsigned>(seq_tiles),
                   static_cast<unsigned>(batch));
-  so::mamba_conv1d_tail_kernel<<<grid, so::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(projected), static_cast<const __nv_bfloat16*>(attention_mask),
-      static_cast<const __nv_bfloat16*>(conv_weight), static_cast<const __nv_bfloat16*>(conv_bias),
-      static_cast<__nv_bfloat16*>(output), static_cast<int>(sequence), static_cast<int>(channels), projected_width);
-  so::g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? SO_OK : SO_ECUDA;
+  return so::launch(so::mamba_conv1d_tail_kernel, grid, so::kConvThreads, 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const __nv_bfloat16*>(projected), static_cast<const __nv_bfloat16*>(attention_mask),
+                    static_cast<const __nv_bfloat16*>(conv_weight), static_cast<const __nv_bfloat16*>(conv_bias),
+                    static_cast<__nv_bfloat16*>(output), static_cast<int>(sequence), static_cast<int>(channels),
+                    projected_width);
 }
 
 int so_mamba_in_proj(const void* hidden, const void* weight, const void* bias, void* projected, int64_t m, int64_t k,
