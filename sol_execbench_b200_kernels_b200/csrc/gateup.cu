@@ -292,6 +292,11 @@ bool shape_ok(int64_t m, int64_t k, int64_t n) {
          k < (1ll << 31) && n < (1ll << 31);
 }
 
+// Token rows of an X box of the lone-CTA kernels.  A launch with one token block loads only the rows there are (to the
+// next 16): the other rows of the operand tile keep whatever shared memory held, and so do their accumulator rows, which
+// nothing stores.
+constexpr int x_box_rows(int64_t m) { return m > 112 ? 128 : static_cast<int>((m + 15) / 16 * 16); }
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // CTAs of `threads` threads of `kernel` that one SM holds at once (at least 1), by the runtime's occupancy query
@@ -319,7 +324,7 @@ int launch_tile(const gu_problem* pr, const DeviceInfo& dev, cudaStream_t stream
   const int64_t m = pr->m, k = pr->k, n = pr->n;
   CUtensorMap tm_x, tm_g, tm_u, tm_o;
   int rc;
-  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
   if ((rc = get_map(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->gate_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_o, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, pr->output, n, m, pr->ld_output * 2, 64, 128)) !=
@@ -355,6 +360,7 @@ int launch_tile(const gu_problem* pr, const DeviceInfo& dev, cudaStream_t stream
   p.blocks_per_owner = 1;
   p.slot_rows = 0;
   p.weights_ready = 0;
+  p.x_bytes = x_box_rows(m) * 128;
   p.out_rows = static_cast<int>(m);
   p.out_cols = static_cast<int>(n);
   const int total_tiles = p.num_tiles;
@@ -613,15 +619,16 @@ int encode_map_uncached(CUtensorMap* out, const void* ptr, uint64_t cols, uint64
 
 // CTAs per tile of the K-split kernel, or 1 where the other kernels are the better choice.  Worth it when a launch has
 // so few 128-token tiles that most SMs would have none: as many CTAs per tile as can be resident together, each with
-// at least kSplitMinBlocks K blocks.
-constexpr int64_t kSplitMinBlocks = 4;
+// at least kSplitMinBlocks K blocks, and not below kSplitMinTotal, where a tile is over before a cut has paid.
+constexpr int64_t kSplitMinBlocks = 4, kSplitMinTotal = 12;
 int split_ctas(const DeviceInfo& dev, int64_t tiles, int64_t kb) {
+  if (kb < kSplitMinTotal) return 1;
   for (int c = kSplitMaxCtas; c >= 2; --c)
     if (tiles <= dev.split_clusters[c] && kb >= kSplitMinBlocks * c) return c;
   return 1;
 }
 
-// `p` comes with its pointers; the map of x has 128-row boxes.
+// `p` comes with its pointers; the map of x has boxes of x_box_rows(m) rows.
 template <int kOp>
 int launch_split(SplitParams& p, int64_t m, int64_t k, int64_t n, int64_t col_tiles, int splits, const CUtensorMap& tm_x,
                  const CUtensorMap& tm_gate, const CUtensorMap& tm_up, cudaStream_t stream) {
@@ -629,6 +636,7 @@ int launch_split(SplitParams& p, int64_t m, int64_t k, int64_t n, int64_t col_ti
   p.kb = static_cast<int>(k / 128);
   p.num_m_blocks = static_cast<int>((m + kTileM - 1) / kTileM);
   p.n_blocks128 = static_cast<int>(n / 128);
+  p.x_bytes = x_box_rows(m) * 128;
   const int64_t ctas = p.num_m_blocks * col_tiles * splits;
   return launch(gateup_split_kernel<kOp>, static_cast<int>(ctas), kTileThreads, kSplitSmemBytes, stream, splits, tm_x, tm_gate,
                 tm_up, p);
@@ -638,7 +646,7 @@ int launch_split_run(const gu_problem* pr, int splits, cudaStream_t stream) {
   const int64_t m = pr->m, k = pr->k, n = pr->n;
   CUtensorMap tm_x, tm_g, tm_u;
   int rc;
-  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
   if ((rc = get_map(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->gate_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
   SplitParams p;
@@ -705,7 +713,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
   if (rc != GU_OK) return rc;
   const int64_t m = pr->m, k = pr->k, n = pr->n;
   CUtensorMap tm_x, tm_g, tm_u, tm_q;
-  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
   if ((rc = get_map(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->gate_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
@@ -752,6 +760,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
   p.blocks_per_owner = 1;
   p.slot_rows = 0;
   p.weights_ready = chained ? 1 : 0;
+  p.x_bytes = x_box_rows(m) * 128;
 
   if (!tile_prefers_lone(kOpGateUpFp8, m, k / 128, n / kTileN, dev->sm_count, dev->pair_clusters, false)) {
     const int clusters = pair_geometry(p, *dev, m, k, static_cast<int>(n / kTileN));
@@ -776,7 +785,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
   if (rc != GU_OK) return rc;
 
   CUtensorMap tm_a, tm_b, tm_c;
-  if ((rc = get_map(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k, 128, 128)) != GU_OK) return rc;
+  if ((rc = get_map(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
   if ((rc = get_map(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, n, m, ld_c * 2, 64, 128)) != GU_OK) return rc;
 
@@ -806,6 +815,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
   p.blocks_per_owner = 1;
   p.slot_rows = 0;
   p.weights_ready = chained ? 1 : 0;
+  p.x_bytes = x_box_rows(m) * 128;
   p.out_rows = static_cast<int>(m);
   p.out_cols = static_cast<int>(n);
   if (!tile_prefers_lone(kOpGemm, m, k / 128, (n / 128 + 1) / 2, dev->sm_count, dev->pair_clusters, false)) {
@@ -1102,6 +1112,7 @@ int gu_run_gather(const gu_problem* pr, void* const* rank_outputs, int world, in
   p.blocks_per_owner = 1;
   p.slot_rows = 0;
   p.weights_ready = 0;
+  p.x_bytes = gu::kOperandTileBytes;
   p.out_count = world;
   p.out_rank = rank;
   p.out_col0 = static_cast<int>(int64_t(rank) * n);
@@ -1177,6 +1188,7 @@ int gu_blockwise_gemm_scatter(const void* a, const float* scale_a, const void* b
   p.blocks_per_owner = p.num_m_blocks / world;  // in 128-token blocks, whichever kernel runs
   p.slot_rows = static_cast<int>(slot_rows);
   p.weights_ready = 0;
+  p.x_bytes = gu::kOperandTileBytes;
 
   if (gu::tile_prefers_pairs(m, *dev)) {
     const int clusters = gu::pair_geometry(p, *dev, m, k, (p.n_blocks128 + 1) / 2);

@@ -375,6 +375,21 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tm_x, const 
   cluster_sync_all();  // barriers and the abort flag of both CTAs exist before anything reaches across
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
+  if (warp == 0 && lane == 0) {
+    // the first tile's first weights on their way into L2 while the kernel in front drains
+    PairWalk<kStreamK> walk(p, cluster_id, clusters);
+    int tile, jb, je;
+    if (walk.next(p, tile, jb, je)) {
+      int pm, nb;
+      tile_coords(p, tile, pm, nb);
+      const int block = kSingle ? 2 * nb + static_cast<int>(rank) : nb;
+      const CUtensorMap* tm_w = (kSingle || rank == 0) ? &tm_gate : &tm_up;
+      for (int j = jb; j < min(jb + kPairStages, je); ++j)
+        if ((!kSingle || block < p.n_blocks128) &&
+            GU_IN_RANGE(load_coords_ok(p.kb, j, block * kTileN, (kSingle ? 2 : 1) * p.num_n_blocks * kTileN), kSitePairLoad))
+          tma_prefetch_2d(tm_w, j * kBlockK, block * kTileN);
+    }
+  }
   pdl_wait();
 
   WaitCtx ctx{abort_slot, false, true};

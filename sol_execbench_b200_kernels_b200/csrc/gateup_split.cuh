@@ -10,10 +10,12 @@
 //
 // Per CTA: TMA producer (warp 0), MMA issuer (warp 1), eight consumer warps as in gateup_tile.cuh; those whose 32
 // token rows do not exist take no part.  At the end a CTA writes its fp32 sums into its own (by then idle) operand
-// ring, [column][token] at a pitch of 129 words so that both the writes (lanes = tokens) and the reads (lanes =
-// columns) hit 32 different banks; after the cluster barrier CTA r finishes the r-th share of the tile's token rows:
-// a warp takes a row, adds the S partial sums in ascending K order and applies the epilogue of its mode (SwiGLU to
-// bf16, SwiGLU to e4m3 + scale, plain bf16).  A whole row in one warp makes the row maximum of the e4m3 mode a shuffle.
+// ring, [token][column] at a pitch of 260 words: eight lanes' 16-byte stores (lanes = tokens) hit 32 different banks,
+// and a warp reads a token's 128 columns of a projection from another CTA as 512 contiguous bytes.  (The reads decide:
+// with 4-byte reads 129 words apart, every lane its own 32-byte packet, joining two 128-token halves took 30 us.)
+// After the cluster barrier CTA r finishes the r-th share of the tile's token rows: a warp takes a row, adds the S
+// partial sums in ascending K order and applies the epilogue of its mode (SwiGLU to bf16, SwiGLU to e4m3 + scale, plain
+// bf16).  A whole row in one warp makes the row maximum of the e4m3 mode a shuffle.
 #pragma once
 
 #include "gateup_pair.cuh"
@@ -25,9 +27,9 @@ enum : unsigned { kWaitSplitEmpty = 18, kWaitSplitFull = 19, kWaitSplitAccEmpty 
 enum : unsigned { kSiteSplitLoad = 65, kSiteSplitScale = 66, kSiteSplitStage = 67, kSiteSplitStore = 68, kSiteSplitPart = 69 };
 
 constexpr int kSplitMaxCtas = 8;                // portable cluster size
-constexpr uint32_t kSplitPitch = kTileM + 1;    // words per column of the partial tile
+constexpr uint32_t kSplitPitch = 2 * kTileN + 4;  // words per token row of the partial tile
 constexpr uint32_t kSplitSmemBytes = kTileStages * kTileStageBytes + 256 /*barriers*/ + 1024 /*alignment slack*/;
-static_assert(2 * kTileN * kSplitPitch * 4 <= kTileStages * kTileStageBytes, "the partial tile fits the operand ring");
+static_assert(kTileM * kSplitPitch * 4 <= kTileStages * kTileStageBytes, "the partial tile fits the operand ring");
 
 struct SplitParams {
   const float* scale_x;     // [M, kb]
@@ -38,12 +40,16 @@ struct SplitParams {
   long long ld_out;
   int m, kb;
   int num_m_blocks, n_blocks128;
+  uint32_t x_bytes;         // bytes of an X box (see x_box_rows)
   int weights_ready;        // the weights were complete before the kernel in front of this one began (see pdl_wait)
 };
 
-__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+__device__ __forceinline__ float4 ld_shared_cluster_f32x4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(cluster_addr)
+               : "memory");
   return v;
 }
 
@@ -110,6 +116,7 @@ gateup_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       // ------------------------------ TMA producer ------------------------------
       const int w0 = kSingle ? 2 * nb * kTileN : nb * kTileN;
       const int w1 = kSingle ? w0 + kTileN : w0;
+      const uint64_t read_once = l2_policy_evict_first();
       auto in_range = [&](int stage, int j) {
         (void)stage; (void)j;
         return GU_IN_RANGE(stage >= 0 && stage < kTileStages, kSiteSplitStage) &&
@@ -119,9 +126,14 @@ gateup_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       };
       auto load_weights = [&](int stage, int j) {
         const uint32_t full = bar_full + 8 * stage, dst = ring + stage * kTileStageBytes;
-        mbar_arrive_expect_tx(full, kTileStageBytes);
-        tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, w0);
-        tma_load_2d(dst + 2 * kOperandTileBytes, kSingle ? &tm_gate : &tm_up, full, j * kBlockK, w1);  // rows past N read as zero
+        mbar_arrive_expect_tx(full, 2 * kOperandTileBytes + p.x_bytes);
+        if (p.num_m_blocks == 1) {  // the weights pass through L2 once
+          tma_load_2d_hint(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, w0, read_once);
+          tma_load_2d_hint(dst + 2 * kOperandTileBytes, kSingle ? &tm_gate : &tm_up, full, j * kBlockK, w1, read_once);
+        } else {
+          tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, w0);
+          tma_load_2d(dst + 2 * kOperandTileBytes, kSingle ? &tm_gate : &tm_up, full, j * kBlockK, w1);  // rows past N read as zero
+        }
       };
       auto load_x = [&](int stage, int j) {
         tma_load_2d(ring + stage * kTileStageBytes, &tm_x, bar_full + 8 * stage, j * kBlockK, mb * kTileM);
@@ -130,6 +142,13 @@ gateup_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       const int early = p.weights_ready ? min(kTileStages, je - jb) : 0;
       for (int i = 0; i < early; ++i)
         if (in_range(i, jb + i)) load_weights(i, jb + i);
+      // and where that is not known, into L2 (doing both took bandwidth from the kernel in front: 53.6 against 50.9 us
+      // for the MLP block at 8 x 4096 x 14336)
+      for (int j = jb; early == 0 && j < min(jb + kTileStages, je); ++j) {
+        if (!in_range(0, j)) continue;
+        tma_prefetch_2d(&tm_gate, j * kBlockK, w0);
+        if (!kSingle || 2 * nb + 1 < p.n_blocks128) tma_prefetch_2d(kSingle ? &tm_gate : &tm_up, j * kBlockK, w1);
+      }
       pdl_wait();
       for (int i = 0; i < early; ++i)
         if (in_range(i, jb + i)) load_x(i, jb + i);
@@ -232,13 +251,11 @@ gateup_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       // The last partial has been read, so every load into the ring has landed and every MMA has read it: the ring is
       // free for the partial tile.
       if (row < rows && GU_IN_RANGE(row >= 0 && row < kTileM && half >= 0 && half < 2, kSiteSplitPart)) {
-        float* part = reinterpret_cast<float*>(smem_gen) + static_cast<uint32_t>(half * 64) * kSplitPitch + row;
+        float4* part = reinterpret_cast<float4*>(smem_gen + 4 * (static_cast<uint32_t>(row) * kSplitPitch + half * 64));
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          part[(2 * i) * kSplitPitch] = g[i].x;
-          part[(2 * i + 1) * kSplitPitch] = g[i].y;
-          part[(kTileN + 2 * i) * kSplitPitch] = u[i].x;
-          part[(kTileN + 2 * i + 1) * kSplitPitch] = u[i].y;
+        for (int i = 0; i < 16; ++i) {
+          part[i] = make_float4(g[2 * i].x, g[2 * i].y, g[2 * i + 1].x, g[2 * i + 1].y);
+          part[kTileN / 4 + i] = make_float4(u[2 * i].x, u[2 * i].y, u[2 * i + 1].x, u[2 * i + 1].y);
         }
       }
     }
@@ -247,51 +264,41 @@ gateup_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   cluster_sync_all();  // every CTA's partial tile is in its shared memory
 
   if (warp >= 4) {
-    // ---- finish this CTA's share of the token rows; a warp takes whole rows, a lane columns lane + 32 i ----
+    // ---- finish this CTA's share of the token rows; a warp takes whole rows, a lane columns 4 lane .. 4 lane + 3 ----
     const int r_end = rows * (rank + 1) / splits;
     for (int r = rows * rank / splits + (warp - 4); r < r_end; r += 8) {
-      float a[8];  // columns lane + 32 i of the first (i < 4) and second 128 accumulator columns
-#pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = 0.f;
+      float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;  // of the first and the second 128 accumulator columns
       if (GU_IN_RANGE(r >= 0 && r < rows && rows <= kTileM, kSiteSplitPart)) {
-        const uint32_t word = static_cast<uint32_t>(lane) * kSplitPitch + static_cast<uint32_t>(r);
-#pragma unroll 2
+        const uint32_t local = ring + 4 * (static_cast<uint32_t>(r) * kSplitPitch + 4 * lane);
+#pragma unroll 4
         for (int s = 0; s < splits; ++s) {  // ascending K
-          const uint32_t src = mapa_shared(ring + 4 * word, static_cast<uint32_t>(s));
-#pragma unroll
-          for (int i = 0; i < 8; ++i) a[i] += ld_shared_cluster_f32(src + i * (32 * kSplitPitch * 4));
+          const uint32_t src = mapa_shared(local, static_cast<uint32_t>(s));
+          const float4 a = ld_shared_cluster_f32x4(src), b = ld_shared_cluster_f32x4(src + 4 * kTileN);
+          g.x += a.x; g.y += a.y; g.z += a.z; g.w += a.w;
+          u.x += b.x; u.y += b.y; u.z += b.z; u.w += b.w;
         }
       }
       const size_t m_global = static_cast<size_t>(mb) * kTileM + r;
       if (!GU_IN_RANGE(static_cast<long long>(m_global) < p.m && (kSingle ? 2 * nb : nb) < p.n_blocks128, kSiteSplitStore)) continue;
       if constexpr (kOp == kSplitGemm) {
-        __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.out) + m_global * p.ld_out + 2 * nb * kTileN + lane;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) dst[32 * i] = __float2bfloat16_rn(a[i]);
-        if (2 * nb + 1 < p.n_blocks128) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) dst[kTileN + 32 * i] = __float2bfloat16_rn(a[4 + i]);
-        }
+        uint16_t* dst = static_cast<uint16_t*>(p.out) + m_global * p.ld_out + 2 * nb * kTileN + 4 * lane;
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(g.x, g.y), pack_bf16x2(g.z, g.w));
+        if (2 * nb + 1 < p.n_blocks128)
+          *reinterpret_cast<uint2*>(dst + kTileN) = make_uint2(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w));
       } else {
-        const uint32_t o01 = swiglu_bf16x2(make_float2(a[0], a[1]), make_float2(a[4], a[5]));
-        const uint32_t o23 = swiglu_bf16x2(make_float2(a[2], a[3]), make_float2(a[6], a[7]));
+        const uint32_t o01 = swiglu_bf16x2(make_float2(g.x, g.y), make_float2(u.x, u.y));
+        const uint32_t o23 = swiglu_bf16x2(make_float2(g.z, g.w), make_float2(u.z, u.w));
         if constexpr (kOp == kSplitGateUp) {
-          uint16_t* dst = static_cast<uint16_t*>(p.out) + m_global * p.ld_out + nb * kTileN + lane;
-          dst[0] = static_cast<uint16_t>(o01);
-          dst[32] = static_cast<uint16_t>(o01 >> 16);
-          dst[64] = static_cast<uint16_t>(o23);
-          dst[96] = static_cast<uint16_t>(o23 >> 16);
+          uint16_t* dst = static_cast<uint16_t*>(p.out) + m_global * p.ld_out + nb * kTileN + 4 * lane;
+          *reinterpret_cast<uint2*>(dst) = make_uint2(o01, o23);
         } else {
           float amax = amax_bf16x2(amax_bf16x2(0.f, o01), o23);
 #pragma unroll
           for (int d = 16; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
           const float sc = fmaxf(amax, 1e-12f) / 448.0f;
           const uint32_t q = e4m3x4_from_bf16x4(o01, o23, sc, __frcp_rn(sc));
-          uint8_t* dst = static_cast<uint8_t*>(p.out) + m_global * p.ld_out + nb * kTileN + lane;
-          dst[0] = static_cast<uint8_t>(q);
-          dst[32] = static_cast<uint8_t>(q >> 8);
-          dst[64] = static_cast<uint8_t>(q >> 16);
-          dst[96] = static_cast<uint8_t>(q >> 24);
+          uint8_t* dst = static_cast<uint8_t*>(p.out) + m_global * p.ld_out + nb * kTileN + 4 * lane;
+          *reinterpret_cast<uint32_t*>(dst) = q;
           if (lane == 0) p.scale_out[m_global * p.n_blocks128 + nb] = sc;
         }
       }

@@ -128,6 +128,19 @@ gateup_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
+  if (warp == 0 && lane == 0) {
+    // a ring's worth of weights on its way into L2 while the kernel in front drains (25.0 -> 22.2 us back to back at
+    // 1 x 4096 x 14336)
+    int nbk = static_cast<int>(u_begin / p.kb);
+    int j = static_cast<int>(u_begin - static_cast<long long>(nbk) * p.kb);
+    for (long long u = u_begin; u < min(u_end, u_begin + p.stages); ++u) {
+      if (GU_IN_RANGE(load_coords_ok(p.kb, j, nbk * 128, p.nb * 128), kSiteStreamLoad)) {
+        tma_prefetch_2d(&tm_gate, j * kBlockK, nbk * 128);
+        tma_prefetch_2d(&tm_up, j * kBlockK, nbk * 128);
+      }
+      if (++j == p.kb) { j = 0; ++nbk; }
+    }
+  }
   pdl_wait();
 
   WaitCtx ctx{abort_slot, false, false};

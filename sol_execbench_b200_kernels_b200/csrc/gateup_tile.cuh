@@ -94,6 +94,7 @@ struct TileParams {
   // sending rank (slot s starts at row s * slot_rows of that buffer)
   int blocks_per_owner;
   int slot_rows;
+  uint32_t x_bytes;         // lone-CTA kernels: bytes of an X box (see x_box_rows)
   int weights_ready;        // the weights were complete before the kernel in front of this one began (see pdl_wait)
   // stream-K schedule only
   unsigned int* flags;      // [gridDim.x] epoch of the last call that filled slot i
@@ -235,6 +236,8 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
       // ------------------------------ TMA producer ------------------------------
       int stage = 0;
       uint32_t phase = 0;
+      const uint64_t read_once = l2_policy_evict_first();
+      (void)read_once;
       auto in_range = [&](int st, int j, int mb, int nb) {
         (void)st; (void)j; (void)mb; (void)nb;  // (only the range-checked build looks at them)
         return GU_IN_RANGE(st >= 0 && st < kTileStages, kSiteTileStage) &&
@@ -244,13 +247,18 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
       auto load_weights = [&](int st, int j, int nb) {
         const uint32_t full = bar_full + 8 * st;
         const uint32_t dst = ring + st * kTileStageBytes;
-        mbar_arrive_expect_tx(full, kTileStageBytes);
+        mbar_arrive_expect_tx(full, 2 * kOperandTileBytes + p.x_bytes);
         if constexpr (kSingle) {  // two adjacent 128-row blocks of the one B matrix (rows past N read as zero)
           tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, 2 * nb * kTileN);
           tma_load_2d(dst + 2 * kOperandTileBytes, &tm_gate, full, j * kBlockK, (2 * nb + 1) * kTileN);
         } else {
-          tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, nb * kTileN);
-          tma_load_2d(dst + 2 * kOperandTileBytes, &tm_up, full, j * kBlockK, nb * kTileN);
+          if (p.num_m_blocks == 1) {  // the weights pass through L2 once (25.2 -> 23.9 us at 128 x 4096 x 14336)
+            tma_load_2d_hint(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, nb * kTileN, read_once);
+            tma_load_2d_hint(dst + 2 * kOperandTileBytes, &tm_up, full, j * kBlockK, nb * kTileN, read_once);
+          } else {
+            tma_load_2d(dst + kOperandTileBytes, &tm_gate, full, j * kBlockK, nb * kTileN);
+            tma_load_2d(dst + 2 * kOperandTileBytes, &tm_up, full, j * kBlockK, nb * kTileN);
+          }
         }
       };
       auto load_x = [&](int st, int j, int mb) {
@@ -261,12 +269,19 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
       // K blocks of the first tile whose weights are loaded while the kernel in front still runs
       int early = 0;
       if constexpr (!kStreamK) {
-        if (p.weights_ready && static_cast<int>(blockIdx.x) < p.num_tiles) {
-          early = min(kTileStages, p.kb);
+        if (static_cast<int>(blockIdx.x) < p.num_tiles) {
+          early = p.weights_ready ? min(kTileStages, p.kb) : 0;
           int mb, nb;
           tile_coords(p, blockIdx.x, mb, nb);
           for (int j = 0; j < early; ++j)
             if (in_range(j, j, mb, nb)) load_weights(j, j, nb);
+          // where that is not known to be safe, they are only brought into L2
+          for (int j = 0; early == 0 && j < min(kTileStages, p.kb); ++j) {
+            if (!in_range(0, j, mb, nb)) continue;
+            tma_prefetch_2d(&tm_gate, j * kBlockK, (kSingle ? 2 * nb : nb) * kTileN);
+            if constexpr (!kSingle) tma_prefetch_2d(&tm_up, j * kBlockK, nb * kTileN);
+            else if (2 * nb + 1 < p.n_blocks128) tma_prefetch_2d(&tm_gate, j * kBlockK, (2 * nb + 1) * kTileN);
+          }
         }
       }
       pdl_wait();

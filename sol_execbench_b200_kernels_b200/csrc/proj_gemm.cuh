@@ -179,6 +179,15 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
+  if (warp == 0 && lane == 0 && unit < p.num_tiles) {
+    // the first tile's first weights on their way into L2 while the kernel in front drains
+    int tm, tn;
+    pj_tile_coords(p, unit, tm, tn);
+    const int wrow = tn * tile_n + static_cast<int>(rank) * b_rows;
+    for (int j = 0; j < min(static_cast<int>(stages), p.kb); ++j)
+      if (wrow < p.n && GU_IN_RANGE(wrow >= 0 && ((j * kPjBlockK * 2) & 15) == 0, kSitePjLoad))
+        tma_prefetch_2d(&tm_w, j * kPjBlockK, wrow);
+  }
   pdl_wait();
 
   WaitCtx ctx{abort_slot, false, kPair};
@@ -187,6 +196,8 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
     // ---------------- TMA producer: the whole warp walks the loop, one elected lane waits and issues ----------------
     const bool elected = elect_one() != 0u;
     const uint32_t full_base = kPair ? mapa_shared(bar_full, 0) : bar_full;
+    const uint64_t read_once = l2_policy_evict_first();
+    (void)read_once;
     uint32_t slots = 0;  // ring slots filled so far: stage = low part, barrier phase = the next bit
     for (int tile = unit; tile < p.num_tiles; tile += units) {
       int tm, tn;
@@ -213,7 +224,8 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
           } else {
             mbar_arrive_expect_tx(full, stage_bytes);
             tma_load_2d(dst, &tm_a, full, j * kPjBlockK, row0);
-            tma_load_2d(dst + kPjATileBytes, &tm_w, full, j * kPjBlockK, wrow0);
+            // one row tile: the weights pass through L2 once (evict-first: 93.5 us against 96.4 at M = 128)
+            tma_load_2d_hint(dst + kPjATileBytes, &tm_w, full, j * kPjBlockK, wrow0, read_once);
           }
         }
         __syncwarp();
