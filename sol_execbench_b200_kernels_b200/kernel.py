@@ -13,6 +13,8 @@ PyTorch is used for device memory, streams and nothing else.
 from __future__ import annotations
 
 import ctypes
+from contextlib import nullcontext
+from functools import lru_cache
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -76,7 +78,7 @@ def _check(expected, device) -> None:
     """Same checks as the reference's `_debug_validate` / pybind `run` (kernel.py:345-395,
     variants/cuda_cpp_v4/binding.cpp:26-72): shapes and dtypes first, then device and layout; always on."""
     for name, (t, shape, dtype) in expected.items():
-        if tuple(t.shape) != shape or t.dtype != dtype:
+        if t.shape != shape or t.dtype != dtype:
             raise ValueError(f"{name}: expected shape={shape}, dtype={dtype}; "
                              f"got shape={tuple(t.shape)}, dtype={t.dtype}")
     for name, (t, shape, dtype) in expected.items():
@@ -107,6 +109,31 @@ def _validate(x, scale_x, gate_w, scale_gate, up_w, scale_up, output) -> Tuple[i
     return m, k, n
 
 
+_ALREADY_CURRENT = nullcontext()
+
+
+def _on(device: torch.device):
+    """Context with `device` current; costs next to nothing when it already is."""
+    index = device.index
+    if index is None or index == torch.cuda.current_device():
+        return _ALREADY_CURRENT
+    return torch.cuda.device(device)
+
+
+def _stream_ptr(device: torch.device) -> int:
+    """The current stream of `device` as a cudaStream_t, without building a Stream object."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+@lru_cache(maxsize=4096)
+def _scratch_bytes(device_index: int, m: int, k: int, n: int, plan_id: int, whole_tiles: bool) -> int:
+    """Scratch a call needs: a function of the shape, the plan and the (current) device's SM count alone."""
+    if whole_tiles and (plan_id == PLAN_TILE or (plan_id == PLAN_AUTO and _cabi.lib.gu_select_plan(m, k, n) == PLAN_TILE)):
+        return 0  # the tile plan without scratch never cuts a tile along K
+    return _cabi.lib.gu_workspace_bytes(m, k, n, plan_id)
+
+
 def _workspace(device: torch.device, stream_ptr: int, nbytes: int) -> Optional[torch.Tensor]:
     if nbytes == 0:
         return None
@@ -126,12 +153,11 @@ def _workspace(device: torch.device, stream_ptr: int, nbytes: int) -> Optional[t
 def _launch(x, scale_x, gate_w, scale_gate, up_w, scale_up, output, plan: str, whole_tiles: bool = False) -> None:
     m, k, n = _validate(x, scale_x, gate_w, scale_gate, up_w, scale_up, output)
     plan_id = _PLANS[plan]
-    with torch.cuda.device(x.device):
-        stream_ptr = torch.cuda.current_stream(x.device).cuda_stream
-        nbytes = _cabi.lib.gu_workspace_bytes(m, k, n, plan_id)
-        if whole_tiles and (plan_id == PLAN_TILE or (plan_id == PLAN_AUTO and _cabi.lib.gu_select_plan(m, k, n) == PLAN_TILE)):
-            nbytes = 0  # the tile plan without scratch never cuts a tile along K
-        ws = _workspace(x.device, stream_ptr, nbytes)
+    device = x.device
+    with _on(device):
+        stream_ptr = _stream_ptr(device)
+        nbytes = _scratch_bytes(torch.cuda.current_device(), m, k, n, plan_id, whole_tiles)
+        ws = _workspace(device, stream_ptr, nbytes)
         pr = GuProblem(
             x.data_ptr(), scale_x.data_ptr(), gate_w.data_ptr(), scale_gate.data_ptr(),
             up_w.data_ptr(), scale_up.data_ptr(), output.data_ptr(),
@@ -141,7 +167,6 @@ def _launch(x, scale_x, gate_w, scale_gate, up_w, scale_up, output, plan: str, w
     _raise_for(code)
 
 
-@torch.no_grad()
 def run(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch.Tensor,
         up_proj_weight: torch.Tensor, scale_up: torch.Tensor, output: torch.Tensor) -> None:
     """output[M, N] (bf16) = SiLU(x @ gate^T) * (x @ up^T) with block-scaled e4m3 operands.
@@ -152,7 +177,6 @@ def run(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: torch.Tensor, 
     _launch(x, scale_x, gate_proj_weight, scale_gate, up_proj_weight, scale_up, output, "auto")
 
 
-@torch.no_grad()
 def run_with_plan(x, scale_x, gate_proj_weight, scale_gate, up_proj_weight, scale_up, output, plan: str,
                   whole_tiles: bool = False) -> None:
     """`run` with the kernel forced: 'auto', 'tile' (kernel and schedule by heuristic), 'tile_pair' / 'tile_pair_sk'
@@ -198,8 +222,8 @@ def run_gather(x: torch.Tensor, scale_x: torch.Tensor, gate_shard: torch.Tensor,
         raise ValueError(f"shard has {n_local} columns, expected {n_full} / {world}")
     _validate_inputs_only(x, scale_x, gate_shard, scale_gate_shard, up_shard, scale_up_shard, m, n_local)
     k = x.shape[1]
-    with torch.cuda.device(x.device):
-        stream_ptr = torch.cuda.current_stream(x.device).cuda_stream
+    with _on(x.device):
+        stream_ptr = _stream_ptr(x.device)
         ptrs = (ctypes.c_void_p * world)(*[int(p) for p in rank_output_ptrs])
         pr = GuProblem(
             x.data_ptr(), scale_x.data_ptr(), gate_shard.data_ptr(), scale_gate_shard.data_ptr(),
@@ -221,8 +245,8 @@ def run_fp8_output(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: tor
     m, k, n = _validate_inputs_only(x, scale_x, gate_proj_weight, scale_gate, up_proj_weight, scale_up)
     _check({"out_q": (out_q, (m, n), torch.float8_e4m3fn), "out_scale": (out_scale, (m, n // BLOCK), torch.float32)},
            x.device)
-    with torch.cuda.device(x.device):
-        stream_ptr = torch.cuda.current_stream(x.device).cuda_stream
+    with _on(x.device):
+        stream_ptr = _stream_ptr(x.device)
         pr = GuProblem(
             x.data_ptr(), scale_x.data_ptr(), gate_proj_weight.data_ptr(), scale_gate.data_ptr(),
             up_proj_weight.data_ptr(), scale_up.data_ptr(), None, m, k, n, n, None, 0, PLAN_TILE, 0)
@@ -230,7 +254,6 @@ def run_fp8_output(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: tor
     _raise_for(code)
 
 
-@torch.no_grad()
 def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch.Tensor, up_proj_weight: torch.Tensor,
               scale_up: torch.Tensor, down_proj_weight: torch.Tensor, scale_down: torch.Tensor,
               output: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -277,8 +300,8 @@ def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch
         down_proj_weight.data_ptr(), scale_down.data_ptr(), base + offsets[0], base + offsets[1], base + offsets[2],
         base + offsets[3], output.data_ptr(), m, k, n, h_out, x.stride(0), output.stride(0),
         1 if x.dtype == torch.float32 else 0, 0)
-    with torch.cuda.device(x.device):
-        stream_ptr = torch.cuda.current_stream(x.device).cuda_stream
+    with _on(x.device):
+        stream_ptr = _stream_ptr(x.device)
         code = _cabi.lib.gu_mlp_block(ctypes.byref(block), stream_ptr)
     _raise_for(code)
     return output
@@ -306,8 +329,8 @@ def blockwise_gemm(a: torch.Tensor, scale_a: torch.Tensor, b: torch.Tensor, scal
     _check(expected, a.device)
     if output.stride(1) != 1 or output.stride(0) < n:
         raise ValueError("output must be row-major with unit column stride")
-    with torch.cuda.device(a.device):
-        stream_ptr = torch.cuda.current_stream(a.device).cuda_stream
+    with _on(a.device):
+        stream_ptr = _stream_ptr(a.device)
         code = _cabi.lib.gu_blockwise_gemm(a.data_ptr(), scale_a.data_ptr(), b.data_ptr(), scale_b.data_ptr(),
                                            output.data_ptr(), m, k, n, output.stride(0), stream_ptr)
     _raise_for(code)
@@ -333,8 +356,8 @@ def blockwise_gemm_scatter(a: torch.Tensor, scale_a: torch.Tensor, b: torch.Tens
         "b": (b, (n, k), torch.float8_e4m3fn), "scale_b": (scale_b, (n // BLOCK, k // BLOCK), torch.float32),
     }
     _check(expected, a.device)
-    with torch.cuda.device(a.device):
-        stream_ptr = torch.cuda.current_stream(a.device).cuda_stream
+    with _on(a.device):
+        stream_ptr = _stream_ptr(a.device)
         ptrs = (ctypes.c_void_p * world)(*[int(p) for p in rank_slot_ptrs])
         code = _cabi.lib.gu_blockwise_gemm_scatter(a.data_ptr(), scale_a.data_ptr(), b.data_ptr(),
                                                    scale_b.data_ptr(), ptrs, world, rank, m, k, n, stream_ptr)
@@ -400,8 +423,8 @@ def quantize_activation(x: torch.Tensor, q: Optional[torch.Tensor] = None,
     for name, t, shape, dtype in (("q", q, (m, k), torch.float8_e4m3fn), ("scale", scale, (m, k // BLOCK), torch.float32)):
         if tuple(t.shape) != shape or t.dtype != dtype or t.device != x.device or not t.is_contiguous():
             raise ValueError(f"{name}: expected contiguous shape={shape}, dtype={dtype} on {x.device}")
-    with torch.cuda.device(x.device):
-        stream_ptr = torch.cuda.current_stream(x.device).cuda_stream
+    with _on(x.device):
+        stream_ptr = _stream_ptr(x.device)
         code = _cabi.lib.gu_quantize_activation(x.data_ptr(), 1 if x.dtype == torch.float32 else 0, x.stride(0),
                                                 q.data_ptr(), scale.data_ptr(), m, k, stream_ptr)
     _raise_for(code)

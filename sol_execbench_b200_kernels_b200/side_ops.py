@@ -13,6 +13,7 @@ from typing import Tuple
 import torch
 
 from . import _sideops_cabi as _so
+from .kernel import _on, _stream_ptr
 
 HEAD_DIM = 128
 CONV_TAPS = 4
@@ -24,15 +25,24 @@ def _need(cond: bool, msg: str) -> None:
         raise ValueError(msg)
 
 
+def _check_dtype(t: torch.Tensor, name: str, device, dtype, dtype_name: str, same: str) -> None:
+    # (messages are put together only when they are needed: a dozen of these checks run per call)
+    if not isinstance(t, torch.Tensor):
+        raise ValueError(f"{name} must be a tensor")
+    if t.dtype != dtype:
+        raise ValueError(f"{name} must have {dtype_name} dtype")
+    if not t.is_contiguous():
+        raise ValueError(f"{name} must be contiguous")
+    if not t.is_cuda:
+        raise ValueError(f"{name} must be a CUDA tensor")
+    if t.device != device:
+        raise ValueError(f"all tensors must {same} the same CUDA device")
+
+
 def _check_f32(t: torch.Tensor, name: str, device) -> None:
-    _need(isinstance(t, torch.Tensor), f"{name} must be a tensor")
-    _need(t.dtype == torch.float32, f"{name} must have float32 dtype")
-    _need(t.is_contiguous(), f"{name} must be contiguous")
-    _need(t.is_cuda, f"{name} must be a CUDA tensor")
-    _need(t.device == device, "all tensors must use the same CUDA device")
+    _check_dtype(t, name, device, torch.float32, "float32", "use")
 
 
-@torch.no_grad()
 def rmsnorm_qk(query: torch.Tensor, key: torch.Tensor, weight_q: torch.Tensor, weight_k: torch.Tensor, eps: float,
                query_norm: torch.Tensor, key_norm: torch.Tensor) -> None:
     """Per-head RMSNorm of query and key, one launch: out = x * rsqrt(mean(x^2, -1) + eps) * weight[head].
@@ -54,21 +64,16 @@ def rmsnorm_qk(query: torch.Tensor, key: torch.Tensor, weight_q: torch.Tensor, w
     tokens = query.numel() // (heads * HEAD_DIM)
     if tokens == 0:
         return
-    with torch.cuda.device(query.device):
-        stream = torch.cuda.current_stream(query.device).cuda_stream
+    with _on(query.device):
+        stream = _stream_ptr(query.device)
         _so.check(_so.lib.so_rmsnorm_qk(query.data_ptr(), key.data_ptr(), weight_q.data_ptr(), weight_k.data_ptr(),
                                         float(eps), query_norm.data_ptr(), key_norm.data_ptr(), tokens, heads, stream))
 
 
 def _check_bf16(t: torch.Tensor, name: str, device) -> None:
-    _need(isinstance(t, torch.Tensor), f"{name} must be a tensor")
-    _need(t.dtype == torch.bfloat16, f"{name} must have bfloat16 dtype")
-    _need(t.is_contiguous(), f"{name} must be contiguous")
-    _need(t.is_cuda, f"{name} must be a CUDA tensor")
-    _need(t.device == device, "all tensors must be on the same CUDA device")
+    _check_dtype(t, name, device, torch.bfloat16, "bfloat16", "be on")
 
 
-@torch.no_grad()
 def mamba_conv1d_tail(projected: torch.Tensor, attention_mask: torch.Tensor, conv1d_weight: torch.Tensor,
                       conv1d_bias: torch.Tensor, output_hidden_states: torch.Tensor) -> None:
     """Mask, depthwise causal conv (4 taps) + bias, SiLU, mask, transposed to [B, channels, L]; all bf16.
@@ -93,15 +98,14 @@ def mamba_conv1d_tail(projected: torch.Tensor, attention_mask: torch.Tensor, con
         _check_bf16(t, name, projected.device)
     if batch == 0 or sequence == 0:
         return
-    with torch.cuda.device(projected.device):
-        stream = torch.cuda.current_stream(projected.device).cuda_stream
+    with _on(projected.device):
+        stream = _stream_ptr(projected.device)
         _so.check(_so.lib.so_mamba_conv1d_tail(projected.data_ptr(), attention_mask.data_ptr(),
                                                conv1d_weight.data_ptr(), conv1d_bias.data_ptr(),
                                                output_hidden_states.data_ptr(), batch, sequence, channels, width,
                                                stream))
 
 
-@torch.no_grad()
 def mamba_in_proj(hidden_states: torch.Tensor, in_proj_weight: torch.Tensor, in_proj_bias: torch.Tensor,
                   projected: torch.Tensor) -> None:
     """projected[..., N] = bf16(hidden_states[..., K] . in_proj_weight[N, K]^T + in_proj_bias[N]), fp32 accumulation.
@@ -123,8 +127,8 @@ def mamba_in_proj(hidden_states: torch.Tensor, in_proj_weight: torch.Tensor, in_
     m = hidden_states.numel() // k
     if m == 0:
         return
-    with torch.cuda.device(hidden_states.device):
-        stream = torch.cuda.current_stream(hidden_states.device).cuda_stream
+    with _on(hidden_states.device):
+        stream = _stream_ptr(hidden_states.device)
         _so.check(_so.lib.so_mamba_in_proj(hidden_states.data_ptr(), in_proj_weight.data_ptr(),
                                            in_proj_bias.data_ptr(), projected.data_ptr(), m, k, n, stream))
 
