@@ -231,7 +231,7 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
   WaitCtx ctx{abort_slot, false, false};
 
   if (warp < 4) {
-    reg_dealloc<64>();
+    reg_dealloc<56>();
     if (warp == 0 && lane == 0) {
       // ------------------------------ TMA producer ------------------------------
       int stage = 0;
@@ -330,7 +330,7 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
       }
     }
   } else {
-    reg_alloc<216>();
+    reg_alloc<224>();
     // ------------------------------- consumers --------------------------------
     pdl_wait();  // the scales of x come from the kernel in front; the stores may overwrite what it reads
     const int quarter = warp & 3;          // TMEM lane quarter this warp may read
@@ -369,9 +369,32 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
         sx0 = ld_dep(sx_row); sg0 = ld_dep(sg_row); su0 = ld_dep(su_row);
         if (p.kb > 1) { sx1 = ld_dep(sx_row + 1); sg1 = ld_dep(sg_row + 1); su1 = ld_dep(su_row + 1); }
       };
-      if (tile < p.num_tiles) start_tile(tile);
-
+      bool fresh = true;  // no epilogue has fetched the tile's first scales
       while (tile < p.num_tiles) {
+        if (fresh) start_tile(tile);
+        fresh = false;
+        // A warp whose 32 token rows lie past M (in the last block of a ragged M) hands the stages back and meets the
+        // epilogue's barriers, nothing else: such a tile costs little more than its MMAs.  Never the first quarter, which
+        // has the storing threads.
+        if (mb * kTileM + quarter * 32 >= p.m) {
+          for (int j = 0; j < p.kb; ++j) {
+            mbar_wait(ctx, my_acc_full + 8 * acc, acc_phase, kWaitTileAccFull);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(my_acc_empty + 8 * acc);
+            acc ^= 1;
+            if (acc == 0) acc_phase ^= 1u;
+          }
+          if constexpr (kFp8Out) {
+            named_bar_sync(3, 256);
+            named_bar_sync(3, 256);
+          } else {
+#pragma unroll
+            for (int b = 0; b < (kSingle ? 4 : 2); ++b) named_bar_sync(1 + half, 128);
+          }
+          tile += gridDim.x;
+          fresh = true;
+          continue;
+        }
         float2 g[32], u[32];  // 64 gate + 64 up running sums
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
