@@ -301,6 +301,9 @@ __device__ __forceinline__ void tile_kernel_body(const CUtensorMap& tm_x, const 
     } else if (warp == 1 && lane == 0) {
       // ------------------------------- MMA issuer -------------------------------
       constexpr uint32_t idesc = umma_idesc_e4m3_f32(kTileM, 2 * kTileN);
+      // no MMA can start before X is loaded, which is after this; a bounded wait begun earlier would count the time of
+      // the kernel in front
+      pdl_wait();
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       TileWalk<kStreamK> walk(p, blockIdx.x, gridDim.x);

@@ -50,6 +50,51 @@ def test_bounded_wait_runs_out_reports_and_leaves_the_context_usable():
         assert st["max_abs"] <= 2e-2 and st["rel_l2"] <= 1e-4, (shape, plan, st)
 
 
+def test_time_limit_of_a_wait_does_not_run_during_the_kernel_in_front():
+    """A launch moves in while the kernel in front still runs.  Its waits start to count when that kernel has ended: with
+    a limit far below the time the kernel in front takes, the launch behind it still gives its result.  The kernel in
+    front is one CTA that walks 65536 K blocks (about 20 ms, no single wait of it longer than a few microseconds), so
+    the other SMs are free for the launch behind it from the start."""
+    import sol_execbench_b200_kernels_b200 as pkg
+    from sol_execbench_b200_kernels_b200 import _cabi
+
+    k = 1 << 23
+    dev = torch.device("cuda:0")
+
+    def e4m3(rows):
+        return torch.zeros(rows, k, dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
+
+    slow = (e4m3(1), torch.ones(1, k // 128, device=dev), e4m3(128), torch.ones(1, k // 128, device=dev), e4m3(128),
+            torch.ones(1, k // 128, device=dev), torch.empty(1, 128, dtype=torch.bfloat16, device=dev))
+    behind = []
+    for shape, plan in (((100, 2048, 1024), "tile_dp"), ((100, 2048, 1024), "tile"), ((300, 2048, 1024), "tile_pair"),
+                        ((16, 2048, 1024), "stream")):      # "tile" cuts these eight tiles along K
+        args = W.make_inputs(*shape, seed=shape[0], device=dev).args()
+        want = torch.empty(shape[0], shape[2], dtype=torch.bfloat16, device=dev)
+        pkg.run_with_plan(*args, want, plan)
+        behind.append((args, want, plan))
+    pkg.run_with_plan(*slow, "tile_dp")
+    torch.cuda.synchronize()
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    begin.record()
+    pkg.run_with_plan(*slow, "tile_dp")
+    end.record()
+    torch.cuda.synchronize()
+    limit_ms = begin.elapsed_time(end) / 20
+    assert limit_ms > 0.1 and pkg.last_status(clear=True) == (0, 0)
+    assert _cabi.lib.gu_set_wait_limit_ns(int(limit_ms * 1e6)) == 0
+    try:
+        for args, want, plan in behind:
+            out = torch.full_like(want, 7.0)
+            pkg.run_with_plan(*slow, "tile_dp")
+            pkg.run_with_plan(*args, out, plan)
+            torch.cuda.synchronize()
+            assert pkg.last_status(clear=True) == (0, 0), plan
+            assert torch.equal(out, want), plan
+    finally:
+        assert _cabi.lib.gu_set_wait_limit_ns(0) == 0
+
+
 def test_wait_limit_setter_round_trip():
     from sol_execbench_b200_kernels_b200 import _cabi
 
