@@ -52,7 +52,7 @@ class GuMlp(Structure):
     _fields_ = [(name, c_void_p) for name in ("x", "gate_w", "scale_gate", "up_w", "scale_up", "down_w", "scale_down",
                                               "x_q", "x_scale", "mid_q", "mid_scale", "output")]
     _fields_ += [(name, c_int64) for name in ("m", "k", "n", "h_out", "ld_x", "ld_output")]
-    _fields_ += [("x_is_f32", c_int32), ("reserved", c_int32)]
+    _fields_ += [("x_is_f32", c_int32), ("whole_tiles", c_int32)]
 
 
 class GateUpError(RuntimeError):

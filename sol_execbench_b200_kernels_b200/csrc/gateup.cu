@@ -699,8 +699,8 @@ int quantize_launch(const void* x, int x_is_f32, int64_t ld_x, void* q, float* s
 }
 
 // `chained`: a step of gu_mlp_block — the kernel in front is the block's own quantiser, so the weights were complete
-// before it began, and tiles may be cut along K.
-int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chained, void* stream_v) {
+// before it began.  `cut`: tiles may be cut along K.
+int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chained, bool cut, void* stream_v) {
   if (!pr || !out_q || !out_scale) return GU_EINVAL_NULL;
   if (!pr->x || !pr->scale_x || !pr->gate_w || !pr->scale_gate || !pr->up_w || !pr->scale_up) return GU_EINVAL_NULL;
   if (!shape_ok(pr->m, pr->k, pr->n)) return GU_EINVAL_SHAPE;
@@ -718,7 +718,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
   if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
 
-  if (chained) {
+  if (cut) {
     const int splits = split_ctas(*dev, (m + kTileM - 1) / kTileM * (n / kTileN), k / 128);
     if (splits > 1) {
       SplitParams sp;
@@ -729,7 +729,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
       sp.out = out_q;
       sp.scale_out = out_scale;
       sp.ld_out = n;
-      sp.weights_ready = 1;
+      sp.weights_ready = chained ? 1 : 0;
       return launch_split<kSplitFp8>(sp, m, k, n, n / kTileN, splits, tm_x, tm_g, tm_u, static_cast<cudaStream_t>(stream_v));
     }
   }
@@ -774,7 +774,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
 }
 
 int gemm_launch(const void* a, const float* scale_a, const void* b, const float* scale_b, void* c, int64_t m,
-                int64_t k, int64_t n, int64_t ld_c, bool chained, void* stream_v) {
+                int64_t k, int64_t n, int64_t ld_c, bool chained, bool cut, void* stream_v) {
   if (!a || !scale_a || !b || !scale_b || !c) return GU_EINVAL_NULL;
   if (!shape_ok(m, k, n) || ld_c < n) return GU_EINVAL_SHAPE;
   if (!aligned16(a) || !aligned16(b) || !aligned16(c) || (reinterpret_cast<uintptr_t>(scale_a) & 3u) ||
@@ -789,7 +789,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
   if ((rc = get_map(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, n, m, ld_c * 2, 64, 128)) != GU_OK) return rc;
 
-  if (chained) {
+  if (cut) {
     const int64_t col_tiles = (n / 128 + 1) / 2;
     const int splits = split_ctas(*dev, (m + kTileM - 1) / kTileM * col_tiles, k / 128);
     if (splits > 1) {
@@ -800,7 +800,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
       sp.scale_up = scale_b;
       sp.out = c;
       sp.ld_out = ld_c;
-      sp.weights_ready = 1;
+      sp.weights_ready = chained ? 1 : 0;
       return launch_split<kSplitGemm>(sp, m, k, n, col_tiles, splits, tm_a, tm_b, tm_b, static_cast<cudaStream_t>(stream_v));
     }
   }
@@ -1266,12 +1266,12 @@ int gu_quantize_activation(const void* x, int x_is_f32, int64_t ld_x, void* q, f
 }
 
 int gu_run_fp8out(const gu_problem* pr, void* out_q, float* out_scale, void* stream) {
-  return gu::fp8out_launch(pr, out_q, out_scale, false, stream);
+  return gu::fp8out_launch(pr, out_q, out_scale, false, false, stream);
 }
 
 int gu_blockwise_gemm(const void* a, const float* scale_a, const void* b, const float* scale_b, void* c, int64_t m,
                       int64_t k, int64_t n, int64_t ld_c, void* stream) {
-  return gu::gemm_launch(a, scale_a, b, scale_b, c, m, k, n, ld_c, false, stream);
+  return gu::gemm_launch(a, scale_a, b, scale_b, c, m, k, n, ld_c, false, false, stream);
 }
 
 int gu_mlp_block(const gu_mlp* b, void* stream) {
@@ -1303,9 +1303,10 @@ int gu_mlp_block(const gu_mlp* b, void* stream) {
   pr.m = b->m;
   pr.k = b->k;
   pr.n = b->n;
-  if ((rc = gu::fp8out_launch(&pr, b->mid_q, b->mid_scale, true, stream)) != GU_OK) return rc;
+  const bool cut = b->whole_tiles == 0;
+  if ((rc = gu::fp8out_launch(&pr, b->mid_q, b->mid_scale, true, cut, stream)) != GU_OK) return rc;
   return gu::gemm_launch(b->mid_q, b->mid_scale, b->down_w, b->scale_down, b->output, b->m, b->n, b->h_out, b->ld_output, true,
-                         stream);
+                         cut, stream);
 }
 
 int gu_last_status(int* detail, int clear) {

@@ -256,12 +256,14 @@ def run_fp8_output(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: tor
 
 def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch.Tensor, up_proj_weight: torch.Tensor,
               scale_up: torch.Tensor, down_proj_weight: torch.Tensor, scale_down: torch.Tensor,
-              output: Optional[torch.Tensor] = None) -> torch.Tensor:
+              output: Optional[torch.Tensor] = None, whole_tiles: bool = False) -> torch.Tensor:
     """bf16 / fp32 activations [M, H] -> bf16 [M, H_out]: quantise, gate/up + SwiGLU (e4m3 out), down projection.
 
     One call into the library, three launches (the steps of `quantize_activation`, `run_fp8_output` and
     `blockwise_gemm`).  `down_proj_weight` is e4m3 [H_out, N] with scales [H_out/128, N/128].  The intermediate [M, N]
-    exists only as e4m3 + scales.  With few tokens the library cuts tiles along K (see gu_mlp_block in gateup.h).
+    exists only as e4m3 + scales.  With few tokens the library cuts tiles along K (see gu_mlp_block in gateup.h);
+    `whole_tiles=True` keeps it from that, as in `run_with_plan`: the bits of an output row then do not depend on how many
+    other rows the call has, and equal those of the three steps called one after the other.
     """
     m, k = _activation_shape(x)
     if gate_proj_weight.dim() != 2 or up_proj_weight.dim() != 2:
@@ -299,7 +301,7 @@ def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch
         x.data_ptr(), gate_proj_weight.data_ptr(), scale_gate.data_ptr(), up_proj_weight.data_ptr(), scale_up.data_ptr(),
         down_proj_weight.data_ptr(), scale_down.data_ptr(), base + offsets[0], base + offsets[1], base + offsets[2],
         base + offsets[3], output.data_ptr(), m, k, n, h_out, x.stride(0), output.stride(0),
-        1 if x.dtype == torch.float32 else 0, 0)
+        1 if x.dtype == torch.float32 else 0, 1 if whole_tiles else 0)
     with _on(x.device):
         stream_ptr = _stream_ptr(x.device)
         code = _cabi.lib.gu_mlp_block(ctypes.byref(block), stream_ptr)

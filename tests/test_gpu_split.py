@@ -70,6 +70,29 @@ def test_mlp_block_cut_along_k(m, kb, nb, hb, dtype):
     assert bool((wide[m] == 7.0).all()) and bool((wide[:, h:] == 7.0).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_mlp_block_with_whole_tiles_gives_rows_that_do_not_depend_on_the_batch(dtype):
+    """512 tokens run on CTA pairs, 300 on lone CTAs, and by itself the library would cut both steps of the smaller calls
+    along K."""
+    import sol_execbench_b200_kernels_b200 as pkg
+
+    k, n, h = 2048, 2304, 2048
+    g = torch.Generator(device="cuda:0").manual_seed(9)
+    x = torch.randn(512, k, generator=g, device="cuda:0").to(dtype)
+    weights = []
+    for rows, cols in ((n, k), (n, k), (h, n)):
+        weights += W.quantize_weight_128x128(torch.randn(rows, cols, generator=g, device="cuda:0") * 0.02)
+    xq, sx = pkg.quantize_activation(x)
+    mid_q = torch.empty(512, n, dtype=torch.float8_e4m3fn, device="cuda:0")
+    mid_s = torch.empty(512, n // 128, device="cuda:0")
+    pkg.run_fp8_output(xq, sx, *weights[:4], mid_q, mid_s)
+    ref = torch.empty(512, h, dtype=torch.bfloat16, device="cuda:0")
+    pkg.blockwise_gemm(mid_q, mid_s, *weights[4:], ref)
+    for m in (512, 300, 129, 128, 31, 1):
+        assert torch.equal(pkg.mlp_block(x[:m], *weights, whole_tiles=True), ref[:m]), m
+    assert pkg.last_status()[0] == 0
+
+
 def test_mlp_block_in_a_graph_and_after_a_weight_update():
     """The block's kernels start before the ones in front of them have ended: weights written just before the call have
     to be the ones that count, in eager calls and in replays."""
