@@ -23,9 +23,11 @@ GU_ESTATIC_LIMIT = -9
 GU_EBOUNDS = -10
 
 PLAN_AUTO, PLAN_TILE, PLAN_STREAM, PLAN_TILE_DP, PLAN_TILE_SK, PLAN_TILE_PAIR, PLAN_TILE_PAIR_SK = 0, 1, 2, 3, 4, 5, 6
-OP_GATEUP, OP_GATEUP_FP8, OP_GEMM = 0, 1, 2
+PLAN_TILE_SPLIT = 8
+OP_GATEUP, OP_GATEUP_FP8, OP_GEMM, OP_MLP_GATEUP, OP_MLP_DOWN = 0, 1, 2, 4, 5
 PLAN_NAMES = {PLAN_AUTO: "auto", PLAN_TILE: "tile", PLAN_STREAM: "stream", PLAN_TILE_DP: "tile_dp",
-              PLAN_TILE_SK: "tile_sk", PLAN_TILE_PAIR: "tile_pair", PLAN_TILE_PAIR_SK: "tile_pair_sk"}
+              PLAN_TILE_SK: "tile_sk", PLAN_TILE_PAIR: "tile_pair", PLAN_TILE_PAIR_SK: "tile_pair_sk",
+              PLAN_TILE_SPLIT: "tile_split"}
 
 EXPORTS = (
     "gu_version", "gu_error_string", "gu_select_plan", "gu_select_tile_kernel", "gu_workspace_bytes", "gu_workspace_init",

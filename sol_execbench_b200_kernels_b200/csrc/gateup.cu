@@ -621,11 +621,23 @@ int encode_map_uncached(CUtensorMap* out, const void* ptr, uint64_t cols, uint64
 // so few 128-token tiles that most SMs would have none: as many CTAs per tile as can be resident together, each with
 // at least kSplitMinBlocks K blocks, and not below kSplitMinTotal, where a tile is over before a cut has paid.
 constexpr int64_t kSplitMinBlocks = 4, kSplitMinTotal = 12;
-int split_ctas(const DeviceInfo& dev, int64_t tiles, int64_t kb) {
-  if (kb < kSplitMinTotal) return 1;
-  for (int c = kSplitMaxCtas; c >= 2; --c)
-    if (tiles <= dev.split_clusters[c] && kb >= kSplitMinBlocks * c) return c;
-  return 1;
+int64_t split_tiles(int64_t m, int64_t col_tiles) { return (m + kTileM - 1) / kTileM * col_tiles; }
+// Whether the rule cuts at all; `pairs`: clusters of two CTAs that are resident at once (the largest count of any size).
+bool prefers_split(int64_t m, int64_t kb, int64_t col_tiles, int pairs) {
+  return kb >= kSplitMinTotal && split_tiles(m, col_tiles) <= pairs;
+}
+int split_ctas(const DeviceInfo& dev, int64_t m, int64_t kb, int64_t col_tiles) {
+  if (!prefers_split(m, kb, col_tiles, dev.split_clusters[2])) return 1;
+  for (int c = kSplitMaxCtas; c > 2; --c)
+    if (split_tiles(m, col_tiles) <= dev.split_clusters[c] && kb >= kSplitMinBlocks * c) return c;
+  return 2;
+}
+// For GU_PLAN_TILE_SPLIT: any count of tiles and K blocks, as long as every CTA has a block; 1 where it cannot run.
+int forced_split_ctas(const DeviceInfo& dev, int64_t m, int64_t kb, int64_t col_tiles) {
+  if (kb < 2 || dev.split_clusters[2] < 1 || split_tiles(m, col_tiles) * kb >= (1ll << 31)) return 1;
+  for (int c = kSplitMaxCtas; c > 2; --c)
+    if (split_tiles(m, col_tiles) <= dev.split_clusters[c] && kb >= c) return c;
+  return 2;
 }
 
 // `p` comes with its pointers; the map of x has boxes of x_box_rows(m) rows.
@@ -719,7 +731,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
   if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
 
   if (cut) {
-    const int splits = split_ctas(*dev, (m + kTileM - 1) / kTileM * (n / kTileN), k / 128);
+    const int splits = split_ctas(*dev, m, k / 128, n / kTileN);
     if (splits > 1) {
       SplitParams sp;
       std::memset(&sp, 0, sizeof(sp));
@@ -791,7 +803,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
 
   if (cut) {
     const int64_t col_tiles = (n / 128 + 1) / 2;
-    const int splits = split_ctas(*dev, (m + kTileM - 1) / kTileM * col_tiles, k / 128);
+    const int splits = split_ctas(*dev, m, k / 128, col_tiles);
     if (splits > 1) {
       SplitParams sp;
       std::memset(&sp, 0, sizeof(sp));
@@ -909,9 +921,13 @@ int gu_select_plan(int64_t m, int64_t k, int64_t n) {
 
 int gu_select_tile_kernel(int op, int64_t m, int64_t k, int64_t n, int with_workspace) {
   if (!gu::shape_ok(m, k, n)) return GU_EINVAL_SHAPE;
+  const bool in_mlp = op == GU_OP_MLP_GATEUP || op == GU_OP_MLP_DOWN;
+  if (in_mlp) op = op == GU_OP_MLP_GATEUP ? GU_OP_GATEUP_FP8 : GU_OP_GEMM;
   if (op != GU_OP_GATEUP && op != GU_OP_GATEUP_FP8 && op != GU_OP_GEMM) return GU_EINVAL_PLAN;
   const int sms = gu::sm_count_or_default(), clusters = sms / 2;
   const int64_t col_tiles = op == GU_OP_GEMM ? (n / 128 + 1) / 2 : n / gu::kTileN;
+  if (with_workspace && (in_mlp || op == GU_OP_GATEUP) && gu::prefers_split(m, k / 128, col_tiles, clusters))
+    return GU_PLAN_TILE_SPLIT;
   if (gu::tile_prefers_lone(op, m, k / 128, col_tiles, sms, clusters, with_workspace != 0)) {
     const bool cut = op == GU_OP_GATEUP && with_workspace && m <= gu::kTileM && gu::tile_prefers_stream_k(m, k, n, sms);
     return cut ? GU_PLAN_TILE_SK : GU_PLAN_TILE_DP;
@@ -933,9 +949,7 @@ size_t gu_workspace_bytes(int64_t m, int64_t k, int64_t n, int plan) {
     // what the tile plan would launch on a B200 (one cluster per two SMs): scratch only where stream-K is chosen
     const int clusters = gu::sm_count_or_default() / 2;
     const int64_t tiles = ((m + 255) / 256) * (n / 128);
-    gu::DeviceInfo like_b200;
-    for (int c = 2; c <= gu::kSplitMaxCtas; ++c) like_b200.split_clusters[c] = gu::sm_count_or_default() / c;
-    if (gu::split_ctas(like_b200, (m + gu::kTileM - 1) / gu::kTileM * (n / gu::kTileN), k / 128) > 1) return gu::kStreamFlagBytes;
+    if (gu::prefers_split(m, k / 128, n / gu::kTileN, clusters)) return gu::kStreamFlagBytes;
     if (m > gu::kTileM && tiles < (1ll << 31) && gu::pair_prefers_stream_k(static_cast<int>(tiles), clusters) &&
         !gu::tile_prefers_lone(gu::kOpGateUp, m, k / 128, n / gu::kTileN, gu::sm_count_or_default(), clusters, true))
       return gu::tile_stream_k_bytes();
@@ -956,17 +970,21 @@ int gu_run(const gu_problem* pr, void* stream_v) {
   int plan = pr->plan;
   if (plan == GU_PLAN_AUTO) plan = gu_select_plan(pr->m, pr->k, pr->n);
   if (plan != GU_PLAN_TILE && plan != GU_PLAN_STREAM && plan != GU_PLAN_TILE_DP && plan != GU_PLAN_TILE_SK &&
-      plan != GU_PLAN_TILE_PAIR && plan != GU_PLAN_TILE_PAIR_SK)
+      plan != GU_PLAN_TILE_PAIR && plan != GU_PLAN_TILE_PAIR_SK && plan != GU_PLAN_TILE_SPLIT)
     return GU_EINVAL_PLAN;
   gu::DeviceInfo* dev = nullptr;
   if ((rc = gu::device_info(&dev)) != GU_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   if (plan == GU_PLAN_TILE_PAIR) return gu::launch_pair(pr, *dev, stream, 0);
   if (plan == GU_PLAN_TILE_PAIR_SK) return gu::launch_pair(pr, *dev, stream, 1);
+  if (plan == GU_PLAN_TILE_SPLIT) {
+    const int splits = gu::forced_split_ctas(*dev, pr->m, pr->k / 128, pr->n / gu::kTileN);
+    return splits > 1 ? gu::launch_split_run(pr, splits, stream) : GU_EINVAL_PLAN;
+  }
   const bool have_ws = pr->workspace && pr->workspace_bytes >= gu::tile_stream_k_bytes() && gu::aligned16(pr->workspace);
   // (scratch stands for leave to cut tiles along K; this kernel needs none of it)
   if (plan == GU_PLAN_TILE && pr->workspace && pr->workspace_bytes >= gu::kStreamFlagBytes) {
-    const int splits = gu::split_ctas(*dev, (pr->m + gu::kTileM - 1) / gu::kTileM * (pr->n / gu::kTileN), pr->k / 128);
+    const int splits = gu::split_ctas(*dev, pr->m, pr->k / 128, pr->n / gu::kTileN);
     if (splits > 1) return gu::launch_split_run(pr, splits, stream);
   }
   if (plan == GU_PLAN_TILE && pr->m > gu::kTileM) {

@@ -21,11 +21,12 @@ import torch
 
 from . import _cabi
 from ._cabi import (PLAN_AUTO, PLAN_STREAM, PLAN_TILE, PLAN_TILE_DP, PLAN_TILE_PAIR, PLAN_TILE_PAIR_SK, PLAN_TILE_SK,
-                    GuProblem)
+                    PLAN_TILE_SPLIT, GuProblem)
 
 BLOCK = 128
 _PLANS = {"auto": PLAN_AUTO, "tile": PLAN_TILE, "stream": PLAN_STREAM, "tile_dp": PLAN_TILE_DP, "tile_sk": PLAN_TILE_SK,
-          "tile_pair": PLAN_TILE_PAIR, "tile_pair_sk": PLAN_TILE_PAIR_SK}
+          "tile_pair": PLAN_TILE_PAIR, "tile_pair_sk": PLAN_TILE_PAIR_SK,
+          "tile_split": PLAN_TILE_SPLIT}
 
 # Scratch for the stream-K hand-off, one buffer per (device, stream): it is
 # written and consumed inside a single call and carries no result across calls.
@@ -180,7 +181,8 @@ def run(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: torch.Tensor, 
 def run_with_plan(x, scale_x, gate_proj_weight, scale_gate, up_proj_weight, scale_up, output, plan: str,
                   whole_tiles: bool = False) -> None:
     """`run` with the kernel forced: 'auto', 'tile' (kernel and schedule by heuristic), 'tile_pair' / 'tile_pair_sk'
-    (CTA-pair kernel, whole tiles / stream-K schedule), 'tile_dp' / 'tile_sk' (lone-CTA kernel, likewise) or 'stream'.
+    (CTA-pair kernel, whole tiles / stream-K schedule), 'tile_dp' / 'tile_sk' (lone-CTA kernel, likewise), 'tile_split'
+    (a cluster of CTAs per tile; K >= 256) or 'stream'.
 
     `whole_tiles=True` keeps the tile plan from cutting any tile along K (it is given no scratch, and then runs its
     data-parallel schedule): the bits of an output row then do not depend on how many other rows the call has, so a

@@ -14,13 +14,19 @@ def _close(out, ref, rel_limit, what):
 
 
 # tokens at the edges of a warp's 32 rows and of the 128-row tile; K blocks that no cluster size divides; one column
-# block (8 CTAs) up to as many tiles as still leave two CTAs each
-@pytest.mark.parametrize("m,kb,nb", [(1, 33, 1), (31, 56, 18), (33, 32, 18), (128, 35, 13), (129, 40, 9), (200, 17, 30),
-                                     (257, 32, 24), (7, 8, 74), (64, 12, 48), (5, 64, 25)])
-def test_gateup_cut_along_k(m, kb, nb):
+# block (8 CTAs) up to as many tiles as still leave two CTAs each (74 on a B200), and one more; fewer K blocks than the
+# rule cuts
+@pytest.mark.parametrize("m,kb,nb,cut", [
+    (1, 33, 1, True), (31, 56, 18, True), (33, 32, 18, True), (128, 35, 13, True), (129, 40, 9, True), (200, 17, 30, True),
+    (257, 32, 24, True), (64, 12, 48, True), (5, 64, 25, True), (7, 12, 74, True), (130, 32, 37, True),
+    (7, 8, 74, False), (33, 11, 18, False), (7, 12, 75, False), (257, 32, 25, False)])
+def test_gateup_cut_along_k(m, kb, nb, cut):
     import sol_execbench_b200_kernels_b200 as pkg
+    from sol_execbench_b200_kernels_b200 import _cabi
 
     k, n = 128 * kb, 128 * nb
+    choice = _cabi.lib.gu_select_tile_kernel(_cabi.OP_GATEUP, m, k, n, 1)
+    assert choice == _cabi.PLAN_TILE_SPLIT if cut else choice in (_cabi.PLAN_TILE_DP, _cabi.PLAN_TILE_PAIR)
     inp = W.make_inputs(m, k, n, seed=m, device="cuda:0")
     whole = torch.empty(m, n, dtype=torch.bfloat16, device="cuda:0")
     pkg.run_with_plan(*inp.args(), whole, "tile_dp")
@@ -30,14 +36,28 @@ def test_gateup_cut_along_k(m, kb, nb):
     pkg.run_with_plan(*inp.args(), again, "tile")
     kept = torch.empty_like(whole)
     pkg.run_with_plan(*inp.args(), kept, "tile", whole_tiles=True)
+    forced = torch.empty_like(whole)
+    pkg.run_with_plan(*inp.args(), forced, "tile_split")
     torch.cuda.synchronize()
     assert pkg.last_status()[0] == 0
     # up to eight fp32 partial sums joined: a bf16 rounding flips where a sum is within 2^-24 * 8 of a tie
-    _close(wide[:m, :n], whole, 1e-4, (m, k, n))
-    assert float((wide[:m, :n] != whole).float().mean()) <= 5e-3
+    for out in (wide[:m, :n], forced):
+        _close(out, whole, 1e-4, (m, k, n))
+        assert float((out != whole).float().mean()) <= 5e-3
+    # the kernel that the choice names is the one that ran: joined sums round differently somewhere, whole tiles nowhere
+    assert not cut or m * n < 1 << 15 or not torch.equal(wide[:m, :n], whole)
+    assert cut or torch.equal(wide[:m, :n], whole)
     assert torch.equal(wide[:m, :n], again)  # the order of the sums is fixed
     assert torch.equal(kept, whole)
     assert bool((wide[m] == 7.0).all()) and bool((wide[:, n:] == 7.0).all())
+
+
+def test_forced_split_needs_two_k_blocks():
+    import sol_execbench_b200_kernels_b200 as pkg
+
+    inp = W.make_inputs(4, 128, 256, seed=1, device="cuda:0")
+    with pytest.raises(ValueError, match="plan"):
+        pkg.run_with_plan(*inp.args(), torch.empty(4, 256, dtype=torch.bfloat16, device="cuda:0"), "tile_split")
 
 
 @pytest.mark.parametrize("m,kb,nb,hb", [(1, 4, 40, 1), (8, 32, 112, 32), (8, 9, 33, 3), (31, 7, 18, 5), (128, 16, 35, 16),

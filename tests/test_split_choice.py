@@ -1,0 +1,38 @@
+"""Where tiles are cut along K in clusters, pinned on the CPU (148 SMs, so 74 clusters of two CTAs, are assumed there)."""
+import pytest
+
+from sol_execbench_b200_kernels_b200 import _cabi
+
+
+def _choice(op, m, k, n, leave):
+    return _cabi.PLAN_NAMES[_cabi.lib.gu_select_tile_kernel(op, m, k, n, leave)]
+
+
+@pytest.mark.parametrize("m,kb,nb,cut", [
+    (128, 56, 18, True), (451, 56, 18, True), (1, 12, 74, True), (128, 32, 74, True),
+    (1, 12, 75, False), (129, 32, 37, True), (129, 32, 38, False),  # 74 and 76 tiles
+    (1, 11, 74, False), (1, 12, 1, True), (600, 32, 14, True), (600, 32, 15, False),
+])
+def test_gateup_tiles_cut_in_clusters(m, kb, nb, cut):
+    k, n = 128 * kb, 128 * nb
+    assert (_choice(_cabi.OP_GATEUP, m, k, n, 1) == "tile_split") == cut
+    assert _choice(_cabi.OP_MLP_GATEUP, m, k, n, 1) == ("tile_split" if cut else _choice(_cabi.OP_GATEUP_FP8, m, k, n, 1))
+    # without leave to cut, and in a call that never cuts, tiles are whole
+    assert _choice(_cabi.OP_GATEUP, m, k, n, 0) in ("tile_dp", "tile_pair")
+    assert _choice(_cabi.OP_MLP_GATEUP, m, k, n, 0) == _choice(_cabi.OP_GATEUP_FP8, m, k, n, 0)
+    assert _choice(_cabi.OP_GATEUP_FP8, m, k, n, 1) in ("tile_dp", "tile_pair")
+
+
+@pytest.mark.parametrize("m,k,h,cut", [
+    (8, 14336, 4096, True), (515, 14336, 4096, False), (512, 14336, 4096, True), (8, 1536, 37 * 256, True),
+    (8, 1536, 74 * 256, True), (8, 1536, 74 * 256 + 128, False), (8, 1536, 73 * 256 + 128, True), (8, 1408, 4096, False),
+])
+def test_down_projection_tiles_cut_in_clusters(m, k, h, cut):
+    assert (_choice(_cabi.OP_MLP_DOWN, m, k, h, 1) == "tile_split") == cut
+    assert _choice(_cabi.OP_MLP_DOWN, m, k, h, 0) == _choice(_cabi.OP_GEMM, m, k, h, 1) != "tile_split"
+
+
+def test_unassigned_ops_and_plans_stay_refused():
+    assert _cabi.lib.gu_select_tile_kernel(3, 256, 128, 128, 1) == _cabi.GU_EINVAL_PLAN
+    assert _cabi.lib.gu_select_tile_kernel(6, 256, 128, 128, 1) == _cabi.GU_EINVAL_PLAN
+    assert _cabi.lib.gu_select_tile_kernel(_cabi.OP_MLP_DOWN, 4, 100, 128, 1) == _cabi.GU_EINVAL_SHAPE
