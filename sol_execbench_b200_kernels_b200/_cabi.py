@@ -46,7 +46,7 @@ class GuProblem(Structure):
         ("m", c_int64), ("k", c_int64), ("n", c_int64),
         ("ld_output", c_int64),
         ("workspace", c_void_p), ("workspace_bytes", c_size_t),
-        ("plan", c_int32), ("reserved", c_int32),
+        ("plan", c_int32), ("cut_k", c_int32),
     ]
 
 

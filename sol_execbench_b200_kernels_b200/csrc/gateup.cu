@@ -946,10 +946,10 @@ size_t gu_workspace_bytes(int64_t m, int64_t k, int64_t n, int plan) {
     return gu::kStreamFlagBytes + size_t(gu::kStreamMaxGrid) * 2 * gu::stream_mpad(m) * 128 * sizeof(float);
   if (plan == GU_PLAN_TILE_SK || plan == GU_PLAN_TILE_PAIR_SK) return gu::tile_stream_k_bytes();
   if (plan == GU_PLAN_TILE) {
-    // what the tile plan would launch on a B200 (one cluster per two SMs): scratch only where stream-K is chosen
+    // what the tile plan would launch on a B200 (one cluster per two SMs): scratch only where stream-K is chosen (tiles
+    // that are cut in clusters need none)
     const int clusters = gu::sm_count_or_default() / 2;
     const int64_t tiles = ((m + 255) / 256) * (n / 128);
-    if (gu::prefers_split(m, k / 128, n / gu::kTileN, clusters)) return gu::kStreamFlagBytes;
     if (m > gu::kTileM && tiles < (1ll << 31) && gu::pair_prefers_stream_k(static_cast<int>(tiles), clusters) &&
         !gu::tile_prefers_lone(gu::kOpGateUp, m, k / 128, n / gu::kTileN, gu::sm_count_or_default(), clusters, true))
       return gu::tile_stream_k_bytes();
@@ -982,8 +982,8 @@ int gu_run(const gu_problem* pr, void* stream_v) {
     return splits > 1 ? gu::launch_split_run(pr, splits, stream) : GU_EINVAL_PLAN;
   }
   const bool have_ws = pr->workspace && pr->workspace_bytes >= gu::tile_stream_k_bytes() && gu::aligned16(pr->workspace);
-  // (scratch stands for leave to cut tiles along K; this kernel needs none of it)
-  if (plan == GU_PLAN_TILE && pr->workspace && pr->workspace_bytes >= gu::kStreamFlagBytes) {
+  // (a caller that passes scratch allows the cut too; this kernel needs none of it)
+  if (plan == GU_PLAN_TILE && (pr->cut_k || (pr->workspace && pr->workspace_bytes >= gu::kStreamFlagBytes))) {
     const int splits = gu::split_ctas(*dev, pr->m, pr->k / 128, pr->n / gu::kTileN);
     if (splits > 1) return gu::launch_split_run(pr, splits, stream);
   }

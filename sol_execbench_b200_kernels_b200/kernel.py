@@ -131,7 +131,7 @@ def _stream_ptr(device: torch.device) -> int:
 def _scratch_bytes(device_index: int, m: int, k: int, n: int, plan_id: int, whole_tiles: bool) -> int:
     """Scratch a call needs: a function of the shape, the plan and the (current) device's SM count alone."""
     if whole_tiles and (plan_id == PLAN_TILE or (plan_id == PLAN_AUTO and _cabi.lib.gu_select_plan(m, k, n) == PLAN_TILE)):
-        return 0  # the tile plan without scratch never cuts a tile along K
+        return 0  # without scratch, and without leave to cut in clusters, the tile plan keeps whole tiles
     return _cabi.lib.gu_workspace_bytes(m, k, n, plan_id)
 
 
@@ -163,7 +163,7 @@ def _launch(x, scale_x, gate_w, scale_gate, up_w, scale_up, output, plan: str, w
             x.data_ptr(), scale_x.data_ptr(), gate_w.data_ptr(), scale_gate.data_ptr(),
             up_w.data_ptr(), scale_up.data_ptr(), output.data_ptr(),
             m, k, n, output.stride(0),
-            ws.data_ptr() if ws is not None else None, nbytes, plan_id, 0)
+            ws.data_ptr() if ws is not None else None, nbytes, plan_id, 0 if whole_tiles else 1)
         code = _cabi.lib.gu_run(ctypes.byref(pr), stream_ptr)
     _raise_for(code)
 
@@ -184,8 +184,8 @@ def run_with_plan(x, scale_x, gate_proj_weight, scale_gate, up_proj_weight, scal
     (CTA-pair kernel, whole tiles / stream-K schedule), 'tile_dp' / 'tile_sk' (lone-CTA kernel, likewise), 'tile_split'
     (a cluster of CTAs per tile; K >= 256) or 'stream'.
 
-    `whole_tiles=True` keeps the tile plan from cutting any tile along K (it is given no scratch, and then runs its
-    data-parallel schedule): the bits of an output row then do not depend on how many other rows the call has, so a
+    `whole_tiles=True` keeps the tile plan from cutting any tile along K (it is given neither scratch nor leave to, and
+    then runs its data-parallel schedule): the bits of an output row then do not depend on how many other rows the call has, so a
     caller that splits M into chunks gets the result of the unsplit call bit for bit."""
     if plan not in _PLANS:
         raise ValueError(f"unknown plan {plan!r}")

@@ -84,6 +84,7 @@ void run(const torch::Tensor& x, const torch::Tensor& scale_x, const torch::Tens
   pr.n = n;
   pr.ld_output = n;
   pr.plan = GU_PLAN_AUTO;
+  pr.cut_k = 1;
   torch::Tensor ws;
   const size_t need = gu_workspace_bytes(m, k, n, GU_PLAN_AUTO);
   if (need != 0) {

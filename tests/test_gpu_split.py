@@ -52,6 +52,43 @@ def test_gateup_cut_along_k(m, kb, nb, cut):
     assert bool((wide[m] == 7.0).all()) and bool((wide[:, n:] == 7.0).all())
 
 
+def test_leave_to_cut_is_the_callers():
+    """Through the C entry point: no tile is cut without scratch and without `cut_k`; either allows it, with the same bits;
+    and `run`, which allows it, takes no scratch for it."""
+    import ctypes
+
+    import sol_execbench_b200_kernels_b200 as pkg
+    from sol_execbench_b200_kernels_b200 import _cabi, kernel
+
+    m, k, n = 128, 7168, 2304
+    args = W.make_inputs(m, k, n, seed=4, device="cuda:0").args()
+    stream = torch.cuda.current_stream().cuda_stream
+    scratch = torch.zeros(4096, dtype=torch.uint8, device="cuda:0")
+
+    def call(cut_k, ws):
+        out = torch.empty(m, n, dtype=torch.bfloat16, device="cuda:0")
+        pr = _cabi.GuProblem(*[t.data_ptr() for t in args], out.data_ptr(), m, k, n, n, ws.data_ptr() if ws is not None else None,
+                             ws.numel() if ws is not None else 0, _cabi.PLAN_AUTO, cut_k)
+        _cabi.check(_cabi.lib.gu_run(ctypes.byref(pr), stream))
+        return out
+
+    whole, cut = (torch.empty(m, n, dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
+    pkg.run_with_plan(*args, whole, "tile_dp")
+    before = dict(kernel._WORKSPACES)
+    other = torch.cuda.Stream()
+    other.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(other):
+        pkg.run(*args, cut)
+    torch.cuda.synchronize()
+    assert kernel._WORKSPACES == before
+    assert not torch.equal(cut, whole)
+    assert torch.equal(call(0, None), whole)
+    assert torch.equal(call(1, None), cut)
+    assert torch.equal(call(0, scratch), cut)
+    assert not scratch.any()
+    assert pkg.last_status()[0] == 0
+
+
 def test_forced_split_needs_two_k_blocks():
     import sol_execbench_b200_kernels_b200 as pkg
 

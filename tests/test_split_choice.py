@@ -32,6 +32,14 @@ def test_down_projection_tiles_cut_in_clusters(m, k, h, cut):
     assert _choice(_cabi.OP_MLP_DOWN, m, k, h, 0) == _choice(_cabi.OP_GEMM, m, k, h, 1) != "tile_split"
 
 
+def test_no_scratch_is_asked_for_where_none_is_used():
+    lib = _cabi.lib
+    for m, k, n in [(128, 7168, 2304), (451, 7168, 2304), (256, 8192, 2048), (1, 4224, 128)]:
+        assert _choice(_cabi.OP_GATEUP, m, k, n, 1) == "tile_split"
+        for plan in (_cabi.PLAN_AUTO, _cabi.PLAN_TILE, _cabi.PLAN_TILE_SPLIT):
+            assert lib.gu_workspace_bytes(m, k, n, plan) == 0
+
+
 def test_unassigned_ops_and_plans_stay_refused():
     assert _cabi.lib.gu_select_tile_kernel(3, 256, 128, 128, 1) == _cabi.GU_EINVAL_PLAN
     assert _cabi.lib.gu_select_tile_kernel(6, 256, 128, 128, 1) == _cabi.GU_EINVAL_PLAN
