@@ -619,15 +619,32 @@ int encode_map_uncached(CUtensorMap* out, const void* ptr, uint64_t cols, uint64
 
 // CTAs per tile of the K-split kernel, or 1 where the other kernels are the better choice.  Worth it when a launch has
 // so few 128-token tiles that most SMs would have none: as many CTAs per tile as can be resident together, each with
-// at least kSplitMinBlocks K blocks, and not below kSplitMinTotal, where a tile is over before a cut has paid.
+// at least kSplitMinBlocks K blocks.
+//
+// The cut saves K blocks and costs the join, which grows with the token rows of a tile (a CTA hands over `rows` KiB), and
+// it saves the less the nearer the tiles by themselves come to pulling what HBM gives.  So the fewest K blocks that are
+// cut grow with both; they grow faster with the tiles behind the quantiser, where whole tiles too load their first
+// weights early, and are one or two fewer where several token blocks share their weights.  Measured on B200, us cut /
+// whole, (tokens, tiles, K blocks) of a gate/up launch: (8, 74, 12) 9.8 / 11.0, (64, 74, 12) 11.5 / 11.3, (64, 74, 16)
+// 12.8 / 13.6, (128, 18, 12) 10.3 / 10.5, (128, 37, 12) 11.6 / 10.9, (128, 37, 16) 12.6 / 12.8, (128, 50, 16) 13.0 / 13.3,
+// (128, 74, 12) 13.4 / 11.8, (128, 74, 16) 14.7 / 13.9, (128, 74, 24) 17.7 / 18.1, (256, 74, 16) 13.7 / 13.4,
+// (200, 74, 18) 14.0 / 14.3, (256, 74, 24) 16.4 / 17.4.  Inside the MLP block, us of the whole block: gate/up (128, 18,
+// 12) 27.7 / 27.4, (128, 37, 16) 41.9 / 40.4, (256, 36, 16) 37.7 / 38.6, (128, 37, 24) 43.5 / 44.9, (128, 74, 24) 65.6 /
+// 65.1, (128, 74, 32) 68.8 / 69.3, (64, 74, 16) 60.3 / 59.7, (64, 74, 24) 62.3 / 63.2; down (128, 74, 24) 28.5 / 28.5,
+// (256, 74, 24) 27.6 / 26.4, (256, 74, 32) 30.7 / 30.4, (256, 74, 56) 40.2 / 42.1.  Below 12 K blocks nothing is cut; there
+// a cut gains only with few rows ((8, 18, 8) 5.8 / 7.9).
 constexpr int64_t kSplitMinBlocks = 4, kSplitMinTotal = 12;
 int64_t split_tiles(int64_t m, int64_t col_tiles) { return (m + kTileM - 1) / kTileM * col_tiles; }
 // Whether the rule cuts at all; `pairs`: clusters of two CTAs that are resident at once (the largest count of any size).
-bool prefers_split(int64_t m, int64_t kb, int64_t col_tiles, int pairs) {
-  return kb >= kSplitMinTotal && split_tiles(m, col_tiles) <= pairs;
+bool prefers_split(int64_t m, int64_t kb, int64_t col_tiles, int pairs, bool chained) {
+  const int64_t tiles = split_tiles(m, col_tiles), rows = m < kTileM ? m : kTileM;
+  const bool several = m > kTileM;  // token blocks
+  // in 24ths: kb >= tiles / 6 + rows / 8 - 8.5 (several: - 10.5), chained kb >= tiles / 4 + rows / 8 - 9 (- 10)
+  const int64_t least = 3 * rows + (chained ? 6 * tiles - (several ? 240 : 216) : 4 * tiles - (several ? 252 : 204));
+  return tiles <= pairs && kb >= kSplitMinTotal && 24 * kb >= least;
 }
-int split_ctas(const DeviceInfo& dev, int64_t m, int64_t kb, int64_t col_tiles) {
-  if (!prefers_split(m, kb, col_tiles, dev.split_clusters[2])) return 1;
+int split_ctas(const DeviceInfo& dev, int64_t m, int64_t kb, int64_t col_tiles, bool chained) {
+  if (!prefers_split(m, kb, col_tiles, dev.split_clusters[2], chained)) return 1;
   for (int c = kSplitMaxCtas; c > 2; --c)
     if (split_tiles(m, col_tiles) <= dev.split_clusters[c] && kb >= kSplitMinBlocks * c) return c;
   return 2;
@@ -731,7 +748,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
   if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
 
   if (cut) {
-    const int splits = split_ctas(*dev, m, k / 128, n / kTileN);
+    const int splits = split_ctas(*dev, m, k / 128, n / kTileN, chained);
     if (splits > 1) {
       SplitParams sp;
       std::memset(&sp, 0, sizeof(sp));
@@ -803,7 +820,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
 
   if (cut) {
     const int64_t col_tiles = (n / 128 + 1) / 2;
-    const int splits = split_ctas(*dev, m, k / 128, col_tiles);
+    const int splits = split_ctas(*dev, m, k / 128, col_tiles, chained);
     if (splits > 1) {
       SplitParams sp;
       std::memset(&sp, 0, sizeof(sp));
@@ -926,7 +943,7 @@ int gu_select_tile_kernel(int op, int64_t m, int64_t k, int64_t n, int with_work
   if (op != GU_OP_GATEUP && op != GU_OP_GATEUP_FP8 && op != GU_OP_GEMM) return GU_EINVAL_PLAN;
   const int sms = gu::sm_count_or_default(), clusters = sms / 2;
   const int64_t col_tiles = op == GU_OP_GEMM ? (n / 128 + 1) / 2 : n / gu::kTileN;
-  if (with_workspace && (in_mlp || op == GU_OP_GATEUP) && gu::prefers_split(m, k / 128, col_tiles, clusters))
+  if (with_workspace && (in_mlp || op == GU_OP_GATEUP) && gu::prefers_split(m, k / 128, col_tiles, clusters, in_mlp))
     return GU_PLAN_TILE_SPLIT;
   if (gu::tile_prefers_lone(op, m, k / 128, col_tiles, sms, clusters, with_workspace != 0)) {
     const bool cut = op == GU_OP_GATEUP && with_workspace && m <= gu::kTileM && gu::tile_prefers_stream_k(m, k, n, sms);
@@ -984,7 +1001,7 @@ int gu_run(const gu_problem* pr, void* stream_v) {
   const bool have_ws = pr->workspace && pr->workspace_bytes >= gu::tile_stream_k_bytes() && gu::aligned16(pr->workspace);
   // (a caller that passes scratch allows the cut too; this kernel needs none of it)
   if (plan == GU_PLAN_TILE && (pr->cut_k || (pr->workspace && pr->workspace_bytes >= gu::kStreamFlagBytes))) {
-    const int splits = gu::split_ctas(*dev, pr->m, pr->k / 128, pr->n / gu::kTileN);
+    const int splits = gu::split_ctas(*dev, pr->m, pr->k / 128, pr->n / gu::kTileN, false);
     if (splits > 1) return gu::launch_split_run(pr, splits, stream);
   }
   if (plan == GU_PLAN_TILE && pr->m > gu::kTileM) {

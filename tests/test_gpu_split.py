@@ -19,7 +19,8 @@ def _close(out, ref, rel_limit, what):
 @pytest.mark.parametrize("m,kb,nb,cut", [
     (1, 33, 1, True), (31, 56, 18, True), (33, 32, 18, True), (128, 35, 13, True), (129, 40, 9, True), (200, 17, 30, True),
     (257, 32, 24, True), (64, 12, 48, True), (5, 64, 25, True), (7, 12, 74, True), (130, 32, 37, True),
-    (7, 8, 74, False), (33, 11, 18, False), (7, 12, 75, False), (257, 32, 25, False)])
+    (7, 8, 74, False), (33, 11, 18, False), (7, 12, 75, False), (257, 32, 25, False),
+    (200, 13, 30, False), (128, 12, 74, False)])
 def test_gateup_cut_along_k(m, kb, nb, cut):
     import sol_execbench_b200_kernels_b200 as pkg
     from sol_execbench_b200_kernels_b200 import _cabi

@@ -32,6 +32,24 @@ def test_down_projection_tiles_cut_in_clusters(m, k, h, cut):
     assert _choice(_cabi.OP_MLP_DOWN, m, k, h, 0) == _choice(_cabi.OP_GEMM, m, k, h, 1) != "tile_split"
 
 
+@pytest.mark.parametrize("op,m,kb,tiles,cut", [
+    # the faster side of the measurements beside the rule, and the rule's line itself
+    ("run", 8, 12, 74, True), ("run", 64, 16, 74, True), ("run", 200, 16, 50, True), ("run", 128, 12, 18, True),
+    ("run", 128, 12, 37, False), ("run", 128, 16, 37, True), ("run", 128, 16, 74, False), ("run", 128, 24, 74, True),
+    ("run", 256, 16, 74, False), ("run", 256, 24, 74, True), ("run", 128, 19, 74, False), ("run", 128, 20, 74, True),
+    ("run", 128, 16, 50, True), ("run", 96, 12, 74, False),
+    ("gateup", 128, 12, 37, False), ("gateup", 256, 16, 36, True), ("gateup", 128, 16, 37, False), ("gateup", 128, 24, 37, True),
+    ("gateup", 128, 24, 74, False), ("gateup", 128, 32, 74, True), ("gateup", 64, 16, 74, False),
+    ("gateup", 64, 24, 74, True), ("gateup", 128, 25, 74, False), ("gateup", 128, 26, 74, True),
+    ("down", 256, 24, 74, False), ("down", 256, 56, 74, True), ("down", 8, 12, 74, True), ("down", 128, 80, 74, True),
+])
+def test_cut_only_where_it_was_the_faster(op, m, kb, tiles, cut):
+    col_tiles = tiles // ((m + 127) // 128)
+    code = {"run": _cabi.OP_GATEUP, "gateup": _cabi.OP_MLP_GATEUP, "down": _cabi.OP_MLP_DOWN}[op]
+    n = col_tiles * (256 if op == "down" else 128)
+    assert (_choice(code, m, 128 * kb, n, 1) == "tile_split") == cut
+
+
 def test_no_scratch_is_asked_for_where_none_is_used():
     lib = _cabi.lib
     for m, k, n in [(128, 7168, 2304), (451, 7168, 2304), (256, 8192, 2048), (1, 4224, 128)]:
