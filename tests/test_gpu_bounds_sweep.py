@@ -5,10 +5,11 @@ built with -DGU_BOUNDS=1 (libgateup_bounds.so) every kernel tests each computed 
 ring / accumulator stage index against its extent before using it, records the first violation in the status word
 (`gu_last_status` -> GU_EBOUNDS) and skips the access.  This test runs every token count M = 1 ... 129 at
 K, N in {128, 256} through every plan that takes the shape — the lone-CTA tile kernel and its stream-K schedule, the
-CTA-pair kernel (forced also where the second CTA of a pair has no rows) and the weight-streaming kernel — inside
-that build, with canary rows and columns around the destination, against the CPU oracle; then a few larger shapes
-through the pair kernel's stream-K schedule, its FP8-output epilogue and its plain-GEMM mode.  A process binds one build
-of the library, so the sweep runs in a child process.
+CTA-pair kernel (forced also where the second CTA of a pair has no rows), the K-split kernel and the weight-streaming
+kernel — inside that build, with canary rows and columns around the destination, against the CPU oracle; then a few
+larger shapes through the pair kernel's stream-K schedule, its FP8-output epilogue and its plain-GEMM mode, the K-split
+kernel with up to eight CTAs per tile, and `mlp_block`, whose kernels load weights early.  A process binds one build of
+the library, so the sweep runs in a child process.
 """
 import os
 import subprocess
@@ -42,7 +43,7 @@ for k in (128, 256):
             inp = W.make_inputs(m, k, n, seed=1000 * k + 10 * n + m)
             ref = O.gateup_blockwise(*inp.args())
             g = inp.to(dev)
-            plans = ["tile_dp", "tile_pair", "tile_sk"] + (["stream"] if m <= 64 else [])
+            plans = ["tile_dp", "tile_pair", "tile_sk"] + (["stream"] if m <= 64 else []) + (["tile_split"] if k > 128 else [])
             for plan in plans:
                 wide.fill_(7.0)
                 view = wide[1:m + 1, 128:128 + n]
@@ -96,6 +97,54 @@ for shape in ((300, 256, 256), (129, 128, 384)):
     assert torch.equal(sc.cpu(), s_ref) and torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
     want = O.gemm_blockwise(q.cpu(), sc.cpu(), wq.cpu(), ws.cpu())
     assert O.error_stats(c, want)["rel_l2"] <= 1e-3
+# the K-split kernel: as `run` cuts few tiles (8, 3 and 2 CTAs per tile), and forced with one K block per CTA and with
+# more tiles than are resident at once
+for shape, plan in (((1, 4224, 128), "tile"), ((31, 7168, 384), "tile"), ((200, 2176, 1280), "tile"), ((64, 1536, 6144), "tile"),
+                    ((130, 4096, 4736), "tile"), ((17, 1024, 256), "tile_split"), ((129, 384, 9728), "tile_split")):
+    m, k, n = shape
+    assert plan != "tile" or _cabi.lib.gu_select_tile_kernel(_cabi.OP_GATEUP, m, k, n, 1) == _cabi.PLAN_TILE_SPLIT, shape
+    g = W.make_inputs(*shape, seed=m, device=dev)
+    ref = torch.empty(m, n, dtype=torch.bfloat16, device=dev)
+    pkg.run_with_plan(*g.args(), ref, "tile_dp")
+    wide = torch.full((m + 2, n + 256), 7.0, dtype=torch.bfloat16, device=dev)
+    view = wide[1:m + 1, 128:128 + n]
+    pkg.run_with_plan(*g.args(), view, plan)
+    launches += 2
+    torch.cuda.synchronize()
+    code, detail = pkg.last_status()
+    assert code == 0, f"{shape} {plan}: device status {code}, detail {detail:#x}"
+    st = O.error_stats(view.float().cpu(), ref.float().cpu())
+    assert st["finite"] and st["rel_l2"] <= 1e-3, (shape, st)
+    mask = torch.ones_like(wide, dtype=torch.bool)
+    mask[1:m + 1, 128:128 + n] = False
+    assert bool((wide[mask] == 7.0).all()), f"{shape} {plan}: wrote outside the destination"
+# mlp_block, cut and whole: (tokens, hidden, intermediate, output); both steps cut, one of them, pairs, lone CTAs, an odd
+# count of 128-column output blocks
+for m, k, n, h in ((1, 1664, 1536, 128), (33, 2048, 2304, 640), (8, 1024, 9600, 1152), (128, 1536, 2432, 384),
+                   (129, 384, 2176, 256), (300, 512, 4992, 2048), (515, 256, 384, 128)):
+    x = torch.randn(m, k, device=dev).to(torch.bfloat16)
+    ws = [t for r, c in ((n, k), (n, k), (h, n)) for t in W.quantize_weight_128x128(torch.randn(r, c, device=dev) * 0.03)]
+    xq, sx = pkg.quantize_activation(x)
+    q = torch.zeros(m, n, dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
+    sc = torch.zeros(m, n // 128, dtype=torch.float32, device=dev)
+    pkg.run_fp8_output(xq, sx, *ws[:4], q, sc)
+    ref = torch.empty(m, h, dtype=torch.bfloat16, device=dev)
+    pkg.blockwise_gemm(q, sc, *ws[4:], ref)
+    launches += 3
+    for whole in (True, False):
+        wide = torch.full((m + 2, h + 256), 7.0, dtype=torch.bfloat16, device=dev)
+        view = wide[1:m + 1, 128:128 + h]
+        pkg.mlp_block(x, *ws, view, whole_tiles=whole)
+        launches += 3
+        torch.cuda.synchronize()
+        code, detail = pkg.last_status()
+        assert code == 0, f"mlp_block {(m, k, n, h)} whole={whole}: device status {code}, detail {detail:#x}"
+        st = O.error_stats(view.float().cpu(), ref.float().cpu())
+        # (cut: an e4m3 rounding of the intermediate may move a step where a bf16 one flips)
+        assert torch.equal(view, ref) if whole else st["finite"] and st["rel_l2"] <= 2e-3, (m, k, n, h, whole, st)
+        mask = torch.ones_like(wide, dtype=torch.bool)
+        mask[1:m + 1, 128:128 + h] = False
+        assert bool((wide[mask] == 7.0).all()), f"mlp_block {(m, k, n, h)}: wrote outside the destination"
 print(f"swept {launches} launches under the range-checked build: status 0 throughout")
 """
 
@@ -122,11 +171,13 @@ dev = torch.device("cuda:0")
 side_ops.last_status()
 launches = 0
 g = torch.Generator().manual_seed(3)
+few = [1, 31, 33, 128, 129]
+# (small N: 64-column tiles up to 128 rows; the large ones give 96, 128, 160, 192, 224 and 256 columns, and two rounds)
 for k in (8, 64, 72, 200):
-    for n in (8, 248, 264, 520):
+    for n in (8, 248, 264, 520) + ((9480, 14216, 18952, 23688, 28424, 33160, 40008) if k in (8, 200) else ()):
         weight = (torch.randn(n, k, generator=g) * 0.1).to(torch.bfloat16).to(dev)
         bias = (torch.randn(n, generator=g) * 0.2).to(torch.bfloat16).to(dev)
-        for m in list(range(1, 131)) + [255, 256, 257, 300, 383, 384, 385, 511, 513]:
+        for m in few if n > 520 else list(range(1, 131)) + [255, 256, 257, 300, 383, 384, 385, 511, 513]:
             hidden = (torch.randn(m, k, generator=g) * 0.5).to(torch.bfloat16).to(dev)
             buf = torch.full((m + 2, n), 7.0, dtype=torch.bfloat16, device=dev)     # canary rows around the result
             out = buf[1:m + 1]

@@ -152,8 +152,8 @@ def test_mlp_block_with_whole_tiles_gives_rows_that_do_not_depend_on_the_batch(d
 
 
 def test_mlp_block_in_a_graph_and_after_a_weight_update():
-    """The block's kernels start before the ones in front of them have ended: weights written just before the call have
-    to be the ones that count, in eager calls and in replays."""
+    """Weights copied in just before the call have to be the ones that count, in eager calls and in replays.  (A copy never
+    lets its successor in early; a kernel that does is in front in test_gpu_overlap.py.)"""
     import sol_execbench_b200_kernels_b200 as pkg
 
     m, k, n = 8, 2048, 5632
