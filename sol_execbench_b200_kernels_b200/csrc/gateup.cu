@@ -224,35 +224,14 @@ unsigned int next_epoch() {
 }
 std::atomic<long long> g_launches{0};
 
-// One launch.  Every kernel of the path waits (pdl_wait) before it touches what an earlier kernel may have written or
-// still reads, so it is launched with the programmatic-serialisation attribute: its blocks move in and set themselves
-// up while the kernel in front drains.  `cluster` > 1 sets a cluster size that the kernel does not fix itself.
+// One launch of a kernel that calls pdl_wait, counted.
 template <typename... Params, typename... Args>
 int launch(void (*kernel)(Params...), int grid, int threads, uint32_t smem, cudaStream_t stream, int cluster,
            const Args&... args) {
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attrs[2];
-  std::memset(attrs, 0, sizeof(attrs));
-  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[0].val.programmaticStreamSerializationAllowed = 1;
-  attrs[1].id = cudaLaunchAttributeClusterDimension;
-  attrs[1].val.clusterDim.x = static_cast<unsigned>(cluster);
-  attrs[1].val.clusterDim.y = 1;
-  attrs[1].val.clusterDim.z = 1;
-  cfg.attrs = attrs;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return GU_ECUDA;
-  }
-  return GU_OK;
+  return launch_overlapping(kernel, dim3(static_cast<unsigned>(grid)), threads, smem, stream, cluster, args...) == cudaSuccess
+             ? GU_OK
+             : GU_ECUDA;
 }
 
 constexpr int kSmemBudget = 227 * 1024;
@@ -727,8 +706,8 @@ int quantize_launch(const void* x, int x_is_f32, int64_t ld_x, void* q, float* s
                  : launch(quantize_act_kernel<__nv_bfloat16, false>, g, t, 0, stream, 1, xh, qb, scale, nblk, ld_x, kb);
 }
 
-// `chained`: a step of gu_mlp_block — the kernel in front is the block's own quantiser, so the weights were complete
-// before it began.  `cut`: tiles may be cut along K.
+// `chained`: a step of gu_mlp_block.  The chain opens with the block's quantiser, which lets nothing start before all in
+// front of it has completed, so the weights of both steps are ready.  `cut`: tiles may be cut along K.
 int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chained, bool cut, void* stream_v) {
   if (!pr || !out_q || !out_scale) return GU_EINVAL_NULL;
   if (!pr->x || !pr->scale_x || !pr->gate_w || !pr->scale_gate || !pr->up_w || !pr->scale_up) return GU_EINVAL_NULL;
@@ -1338,6 +1317,7 @@ int gu_mlp_block(const gu_mlp* b, void* stream) {
   pr.m = b->m;
   pr.k = b->k;
   pr.n = b->n;
+  // both steps load weights early (`chained`), because the quantiser above is the first launch of the block
   const bool cut = b->whole_tiles == 0;
   if ((rc = gu::fp8out_launch(&pr, b->mid_q, b->mid_scale, true, cut, stream)) != GU_OK) return rc;
   return gu::gemm_launch(b->mid_q, b->mid_scale, b->down_w, b->scale_down, b->output, b->m, b->n, b->h_out, b->ld_output, true,

@@ -41,7 +41,8 @@ struct SplitParams {
   int m, kb;
   int num_m_blocks, n_blocks128;
   uint32_t x_bytes;         // bytes of an X box (see x_box_rows)
-  int weights_ready;        // the weights were complete before the kernel in front of this one began (see pdl_wait)
+  int weights_ready;        // the weights were complete before any kernel began that this one may overlap: a step of
+                            // gu_mlp_block behind its quantiser, and nothing else (see pdl_wait)
 };
 
 __device__ __forceinline__ float4 ld_shared_cluster_f32x4(uint32_t cluster_addr) {

@@ -95,7 +95,8 @@ struct TileParams {
   int blocks_per_owner;
   int slot_rows;
   uint32_t x_bytes;         // lone-CTA kernels: bytes of an X box (see x_box_rows)
-  int weights_ready;        // the weights were complete before the kernel in front of this one began (see pdl_wait)
+  int weights_ready;        // the weights were complete before any kernel began that this one may overlap: a step of
+                            // gu_mlp_block behind its quantiser, and nothing else (see pdl_wait)
   // stream-K schedule only
   unsigned int* flags;      // [gridDim.x] epoch of the last call that filled slot i
   float* partials;          // [gridDim.x][32][256] float4: values 4i..4i+3 of consumer thread t at [i * 256 + t]

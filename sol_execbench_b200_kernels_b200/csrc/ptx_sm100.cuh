@@ -367,12 +367,37 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_bar) {
 // the stream is still running: its blocks move in as the other's leave, and set up barriers, TMEM and descriptors.
 // pdl_wait() returns once every kernel in front has completed and its writes are visible; no thread touches memory
 // that another kernel may write (or still read) before it.  The one exception is weights that were complete before
-// the kernel in front began.  pdl_trigger() lets the next kernel start: from then on its blocks may take this grid's
-// place as its blocks leave.  A kernel that lets a successor prefetch weights triggers only after its own pdl_wait().
+// the kernels it may overlap began (`weights_ready`).  pdl_trigger() lets the next kernel start: from then on its blocks
+// may take this grid's place as its blocks leave.  Most kernels trigger first of all, so a kernel may overlap several in
+// front of it; the chain of overlaps ends at one that triggers after its own pdl_wait(), since nothing behind that one
+// starts before all in front of it has completed.  The quantiser is such a kernel, and `weights_ready` is right only in a
+// chain that it opens.  A bounded wait comes after pdl_wait(), or its limit counts the time of the kernels in front.
 // Both do nothing for a kernel launched without the attribute.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Host side: one launch with that attribute.  `cluster` > 1 sets a cluster size that the kernel does not fix itself.
+template <typename... Params, typename... Args>
+cudaError_t launch_overlapping(void (*kernel)(Params...), dim3 grid, int threads, uint32_t smem, cudaStream_t stream,
+                               int cluster, const Args&... args) {
+  cudaLaunchAttribute attrs[2] = {};
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attrs[1].val.clusterDim.y = 1;
+  attrs[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attrs;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
 // Load of a value that an earlier kernel wrote: volatile, so that it stays below pdl_wait(), and not through the
 // read-only path, which assumes that nothing writes the location while this kernel runs.
 __device__ __forceinline__ float ld_dep(const float* p) {

@@ -114,7 +114,7 @@ quantize_act_kernel(const T* x, uint8_t* __restrict__ q, float* __restrict__ sca
   constexpr int kQuantUnroll = quant_unroll<T>();
   const uint32_t half_warps = gridDim.x * (kQuantThreads / 16);
   pdl_wait();
-  pdl_trigger();  // only now: a successor may prefetch weights that a kernel in front of this one has written
+  pdl_trigger();  // only now: gu_mlp_block's launches load weights early that a kernel in front of this one may have written
   // the host keeps blocks + kQuantUnroll * half_warps below 2^32
   for (uint32_t b = blockIdx.x * (kQuantThreads / 16) + (threadIdx.x >> 4); b < blocks; b += half_warps * kQuantUnroll) {
     Raw8<T> raw[kQuantUnroll];

@@ -374,29 +374,11 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 
 constexpr uint32_t kPjSmemBudget = 227 * 1024;
 
-// One launch with the programmatic-serialisation attribute (see pdl_wait): the kernel's blocks move in while the kernel
-// in front drains.
+// One launch of a kernel that calls pdl_wait, counted.
 template <typename... Params, typename... Args>
 int launch(void (*kernel)(Params...), dim3 grid, int threads, uint32_t smem, cudaStream_t stream, const Args&... args) {
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  std::memset(&attr, 0, sizeof(attr));
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return SO_ECUDA;
-  }
-  return SO_OK;
+  return gu::launch_overlapping(kernel, grid, threads, smem, stream, 1, args...) == cudaSuccess ? SO_OK : SO_ECUDA;
 }
 
 // resolved through the runtime, so the library has no link-time dependency on the driver library
