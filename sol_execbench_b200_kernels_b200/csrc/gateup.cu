@@ -902,11 +902,11 @@ int gu_select_plan(int64_t m, int64_t k, int64_t n) {
   // but loses on mid-sized ones (K=4096, N=14336: 34.6 us against 28.8 us); from 33 tokens on the tile kernel
   // is faster everywhere (its consumers do one FMA per element, the streaming kernel's do two).
   // Where one round of 128-column tiles fills the device (85 % of the SMs or more), the tile kernel streams as well as
-  // the equal unit ranges do and hands nothing over: us at M = 8, tile / stream, (K, N) = (8192, 17920) 50.5 / 54.8,
-  // (7168, 18432) 45.6 / 50.6, (6144, 16384) 38.0 / 39.9; at M = 24 50.9 / 61.6 and 46.2 / 57.8 for the first two.  Below
-  // 40 K blocks its epilogue weighs more, up to 8 tokens: (3584, 18944) M = 1 24.2 / 23.4, M = 8 25.1 / 25.2, M = 16
-  // 25.4 / 26.4.  With a round three quarters full streaming is ahead: (8192, 14336) M = 8 46.8 / 44.5, (4096, 11008)
-  // 22.1 / 19.3.
+  // the equal unit ranges do and hands nothing over: us of device time at M = 8, tile / stream, (K, N) = (8192, 17920)
+  // 50.0 / 50.1, (7168, 18432) 43.8 / 45.0, (6144, 16384) 35.4 / 36.3; at M = 24 50.8 / 53.9 and 44.0 / 48.5 for the first
+  // two.  With a round three quarters full streaming is ahead: (8192, 14336) M = 8 41.9 / 40.8, (4096, 11008) 21.8 / 20.8.
+  // The line at 40 K blocks and 8 tokens was drawn on eager calls ((3584, 18944) M = 1 24.2 / 23.4, M = 16 25.4 / 26.4);
+  // of device time tiles take less there too (M = 1 23.9 / 24.8, M = 16 23.9 / 25.3).
   const int64_t weight_bytes = 2 * n * k, tiles = n / gu::kTileN, sms = gu::sm_count_or_default();
   if (tiles <= sms && 20 * tiles >= 17 * sms && (k / 128 >= 40 || m > 8)) return GU_PLAN_TILE;
   const bool can_stream = m <= 64 && gu::stream_stages(gu::stream_mpad(m), k / 128) > 0;
