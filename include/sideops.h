@@ -71,6 +71,18 @@ int so_mamba_in_proj(const void* hidden, const void* weight, const void* bias, v
                      int64_t n, void* stream);
 
 /*
+ * Both of the above in one call, the convolution in the projection's epilogue above 128 rows: hidden [batch, sequence, k],
+ * weight [n, k], bias [n], attention_mask [batch, sequence], conv_weight [channels, 4], conv_bias [channels] -> output
+ * [batch, channels, sequence], and projected [batch, sequence, n] with the gate in columns [channels, n).  Its columns
+ * [0, channels) are scratch: above 128 rows only those next to a multiple of 128 (in the flattened batch x sequence) are
+ * written, for a second, small launch that computes the positions whose taps reach over such a multiple.  Roundings as in
+ * the two calls above, sizes and alignments what both take.
+ */
+int so_mamba_in_proj_conv(const void* hidden, const void* weight, const void* bias, void* projected,
+                          const void* attention_mask, const void* conv_weight, const void* conv_bias, void* output,
+                          int64_t batch, int64_t sequence, int64_t k, int64_t n, int64_t channels, void* stream);
+
+/*
  * Synchronises the device and returns SO_OK, or SO_ETIMEOUT if a bounded wait inside so_mamba_in_proj ran out since
  * the status was last cleared (`detail`: wait id << 24 | block), or SO_EBOUNDS (range-checked build); `clear` != 0
  * resets it.

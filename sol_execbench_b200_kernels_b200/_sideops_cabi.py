@@ -9,7 +9,7 @@ from . import build as _build
 SO_OK, SO_EINVAL_NULL, SO_EINVAL_SHAPE, SO_EINVAL_ALIGN, SO_ECUDA, SO_EDEVICE, SO_ETIMEOUT, SO_EBOUNDS = (
     0, -1, -2, -3, -4, -5, -6, -7)
 
-EXPORTS = ("so_version", "so_error_string", "so_rmsnorm_qk", "so_mamba_conv1d_tail", "so_mamba_in_proj", "so_last_status",
+EXPORTS = ("so_version", "so_error_string", "so_rmsnorm_qk", "so_mamba_conv1d_tail", "so_mamba_in_proj", "so_mamba_in_proj_conv", "so_last_status",
            "so_is_range_checked_build", "so_set_wait_limit_ns", "so_launch_count")
 
 
@@ -37,6 +37,8 @@ def _load() -> ctypes.CDLL:
                                          c_int64, c_void_p]
     lib.so_mamba_in_proj.restype = c_int
     lib.so_mamba_in_proj.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_void_p]
+    lib.so_mamba_in_proj_conv.restype = c_int
+    lib.so_mamba_in_proj_conv.argtypes = [c_void_p] * 8 + [c_int64] * 5 + [c_void_p]
     lib.so_last_status.restype = c_int
     lib.so_last_status.argtypes = [POINTER(c_int), c_int]
     lib.so_is_range_checked_build.restype = c_int

@@ -28,7 +28,7 @@
 // shared::cluster addresses (remote mbarrier.arrive, TMA completion bytes, tcgen05.commit).  No multicast form.
 #pragma once
 
-#include "ptx_sm100.cuh"
+#include "mamba_conv.cuh"
 
 namespace so {
 
@@ -59,7 +59,8 @@ struct PjCfg {
 
 enum : unsigned { kWaitPjSlot = 40, kWaitPjFull = 41, kWaitPjAccFree = 42, kWaitPjAccFull = 43 };
 // sites of the range-checked debug build (-DGU_BOUNDS=1, see GU_IN_RANGE)
-enum : unsigned { kSitePjLoad = 49, kSitePjStage = 50, kSitePjStore = 51, kSitePjBias = 52, kSitePjTile = 53 };
+enum : unsigned { kSitePjLoad = 49, kSitePjStage = 50, kSitePjStore = 51, kSitePjBias = 52, kSitePjTile = 53,
+                  kSitePjConv = 54 };
 
 struct ProjParams {
   const __nv_bfloat16* bias;  // [N]
@@ -69,6 +70,27 @@ struct ProjParams {
   int group_m;                // raster: tiles walk `group_m` row tiles at a time, row tile fastest
   int tile_n, stages;         // lone CTAs: columns per tile (a multiple of 32, at most 256) and ring depth
   int staging_in_ring;        // lone CTAs: no CTA has a second tile, so the staging tiles may lie in the idle ring
+};
+
+// The convolution tail in the epilogue (CTA pairs only): the first `channels` columns are not stored as they are but masked,
+// convolved along the sequence, gated and written transposed.
+//
+// What it saves is the round trip of half of the projection through HBM and most of a launch (the tail by itself takes
+// 37.8 us at 2 x 1000 tokens).  The arithmetic is the tail's, some 5000 issue slots per warp and 256-column tile, and hides
+// behind the next tile's 65 000 cycles of MMAs; column tiles run in ascending order, so the tiles at the end of a group of
+// row tiles, which nothing hides, are gate tiles.  (Not so with one round of tiles: 1 x 128 tokens on lone CTAs took 104 us
+// this way and takes 99 with the tail behind.)  A lane holds one token row of 64 channels, so the taps at l-1, l-2, l-3 are
+// its neighbours' values (shuffles; the three lanes at a warp's edge read what the warp above left in shared memory), and
+// a channel's 32 positions are one 64-byte store per warp, whatever the alignment of the rows.  The first three rows of a
+// CTA's 128 need rows of another CTA: those outputs are left to mamba_conv1d_edges_kernel, and the three rows on either
+// side of each edge are stored into `projected` for it.  (Overlapping the row blocks by three instead would add a block
+// in 42, a whole round of tiles at some sizes.)
+struct ConvParams {
+  const uint16_t* mask;          // [M] bf16 bits
+  const __nv_bfloat16* weight;   // [channels, 4]
+  const __nv_bfloat16* bias;     // [channels]
+  uint16_t* out;                 // [batch, channels, sequence] bf16 bits
+  int sequence, channels;
 };
 
 // Instruction descriptor, kind::f16: D fp32 (bits 4-5 = 1), A and B bf16 (format 1 at bits 7-9 and 10-12), both
@@ -116,9 +138,63 @@ __device__ __forceinline__ void pj_tile_coords(const ProjParams& p, int tile, in
   tn = within / rows;
 }
 
-template <bool kPair>
-__device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CUtensorMap& tm_w,
-                                               const CUtensorMap& tm_out, const ProjParams& p) {
+// What a chunk of 64 channels leaves in shared memory (in its staging tile, which it does not use otherwise):
+constexpr uint32_t kConvHaloBytes = 4 * 3 * 128;  // [warp][row 29, 30, 31][64 channels]: masked rows for the warp below
+constexpr uint32_t kConvTapBytes = 32 * 16;       // [channel pair] taps, then [channel pair] bias (4 bytes)
+
+// One token row of 32 channels (16 packed words `x`, masked) -> 32 outputs.  `halo`: these channels of the three rows above
+// this warp's first, 128 bytes per row; `taps` / `biases`: of these channels; `hist`: rows of history that the lane's
+// position has, at most 3.
+__device__ __forceinline__ void conv_row_32(long long sequence, const uint32_t (&x)[16], const uint8_t* halo, const uint4* taps,
+                                            const uint4* biases, int lane, int hist, bool keep, bool store, uint16_t* dst) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {  // 4 words = 8 channels
+    const uint4 bq = biases[g];
+    const uint32_t bias[4] = {bq.x, bq.y, bq.z, bq.w};
+    uint32_t prev[3][4];  // [k - 1]: the values k positions back
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) {
+      uint4 edge = make_uint4(0u, 0u, 0u, 0u);
+      if (lane < k) edge = *reinterpret_cast<const uint4*>(halo + (3 + lane - k) * 128 + 16 * g);
+      const uint32_t e[4] = {edge.x, edge.y, edge.z, edge.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, x[4 * g + i], k);
+        prev[k - 1][i] = hist >= k ? (lane < k ? e[i] : up) : 0u;
+      }
+    }
+    uint32_t conv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 w[4];
+      unpack_taps(taps[4 * g + i], w);
+      conv[i] = conv_pair(bf16x2_to_float2(prev[2][i]), bf16x2_to_float2(prev[1][i]), bf16x2_to_float2(prev[0][i]),
+                          bf16x2_to_float2(x[4 * g + i]), w, bf16x2_to_float2(bias[i]));
+    }
+    __nv_bfloat162 lowest = *reinterpret_cast<const __nv_bfloat162*>(&conv[0]);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) lowest = __hmin2(lowest, *reinterpret_cast<const __nv_bfloat162*>(&conv[i]));
+    const bool small = __hbge2(lowest, __floats2bfloat162_rn(-20.f, -20.f));
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      uint32_t r[2];
+      silu_2x2(conv[i], conv[i + 1], small, r[0], r[1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (!keep) r[h] = 0u;
+        if (store) {
+          __stcs(reinterpret_cast<unsigned short*>(dst), static_cast<unsigned short>(r[h]));
+          __stcs(reinterpret_cast<unsigned short*>(dst + sequence), static_cast<unsigned short>(r[h] >> 16));
+        }
+        dst += 2 * sequence;
+      }
+    }
+  }
+}
+
+template <bool kPair, bool kConv>
+__device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const CUtensorMap& tm_out,
+                                               const ProjParams& p, const ConvParams* cv) {
   using Cfg = PjCfg<kPair>;
   extern __shared__ uint8_t smem_raw[];
   // operand tiles need 1024-byte alignment for the 128-byte swizzle pattern; both CTAs of a pair get the same offsets
@@ -294,6 +370,35 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
       const int col0 = tn * tile_n;
       const int chunks = (tile_n + 63) / 64;
       const uint32_t acc = tiles_done & 1u, acc_phase = (tiles_done >> 1) & 1u;
+      // (convolution) this lane's row: its mask, position and destination
+      uint32_t mask2 = 0u;
+      int hist = 0;
+      bool keep = false, conv_store = false, edge_row = false;
+      uint16_t* conv_out = nullptr;
+      if constexpr (kConv) {
+        if (row0 + row < p.m && col0 < cv->channels) {
+          const int r = row0 + row, b = r / cv->sequence, l = r - b * cv->sequence;
+          const uint32_t mb = ld_dep(cv->mask + r);
+          mask2 = mb | (mb << 16);
+          keep = conv_keeps(mb);
+          hist = min(l, kConvTaps - 1);
+          conv_store = hist <= row;  // all its taps lie among this CTA's rows
+          edge_row = row < kConvTaps - 1 || row >= kPjTileM - (kConvTaps - 1);  // stored for mamba_conv1d_edges_kernel
+          conv_out = cv->out + static_cast<long long>(b) * cv->channels * cv->sequence + l;
+        }
+      }
+      // taps and bias of a chunk, a channel pair per thread, fetched one chunk ahead (read where they are used they cost
+      // an L2 latency per eight channels: 1 x 512 tokens took 266 us that way)
+      uint4 taps_next = make_uint4(0u, 0u, 0u, 0u);
+      uint32_t cbias_next = 0u;
+      auto fetch_taps = [&](int first) {
+        const int ch = first + 2 * (et & 31);
+        if (kConv && ch < cv->channels) {
+          if (et < 32) taps_next = ld_dep(reinterpret_cast<const uint4*>(cv->weight + static_cast<long long>(ch) * kConvTaps));
+          else if (et < 64) cbias_next = ld_dep(reinterpret_cast<const uint32_t*>(cv->bias + ch));
+        }
+      };
+      fetch_taps(col0);
       const bool ok = pj_wait_elected(ctx, lane == 0, bar_acc_full + 8 * acc, acc_phase, kWaitPjAccFull);
       tc_fence_after();
 #pragma unroll 1
@@ -322,6 +427,46 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
         // the staging tile of this chunk was last read by the store issued two chunks ago
         if (et == 0) tma_store_wait_read1();
         named_bar_sync(1, 128);
+        if constexpr (kConv) {
+          if (colc < cv->channels) {  // all 64 columns are channels: both are multiples of 64
+            uint32_t x[2][16];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const uint32_t bw[4] = {bq[q].x, bq[q].y, bq[q].z, bq[q].w};
+              uint32_t o[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float b_lo = __uint_as_float(bw[i] << 16), b_hi = __uint_as_float(bw[i] & 0xffff0000u);
+                o[i] = pack_bf16x2(v[8 * q + 2 * i] + b_lo, v[8 * q + 2 * i + 1] + b_hi);
+                x[q >> 2][4 * (q & 3) + i] = mask_mul_bf16x2(o[i], mask2);
+              }
+              if (edge_row && ok && !ctx.aborted && GU_IN_RANGE(row0 + row >= 0 && row0 + row < p.m && colc + 8 * q + 8 <= p.n, kSitePjStore))
+                *reinterpret_cast<uint4*>(p.out + static_cast<size_t>(row0 + row) * p.n + colc + 8 * q) =
+                    make_uint4(o[0], o[1], o[2], o[3]);
+            }
+            uint8_t* halo = stag_gen + (c & 1) * kPjOutChunkBytes;
+            uint4* taps = reinterpret_cast<uint4*>(halo + kConvHaloBytes);
+            uint32_t* biases = reinterpret_cast<uint32_t*>(halo + kConvHaloBytes + kConvTapBytes);
+            if (et < 32) taps[et] = taps_next;
+            else if (et < 64) biases[et - 32] = cbias_next;
+            if (c + 1 < chunks) fetch_taps(colc + 64);
+            if (lane >= 29)
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                *reinterpret_cast<uint4*>(halo + (quarter * 3 + lane - 29) * 128 + 16 * q) =
+                    make_uint4(x[q >> 2][4 * (q & 3)], x[q >> 2][4 * (q & 3) + 1], x[q >> 2][4 * (q & 3) + 2], x[q >> 2][4 * (q & 3) + 3]);
+            named_bar_sync(2, 128);
+            const bool store = conv_store && ok && !ctx.aborted &&
+                               GU_IN_RANGE(row0 + row >= 0 && row0 + row < p.m && colc >= 0 && colc + 64 <= cv->channels, kSitePjConv);
+            const uint8_t* above = halo + (quarter == 0 ? 0 : quarter - 1) * 3 * 128;  // (the first warp's edge is not stored)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              conv_row_32(cv->sequence, x[h], above + 64 * h, taps + 16 * h, reinterpret_cast<const uint4*>(biases) + 4 * h, lane, hist,
+                          keep, store, conv_out + static_cast<long long>(colc + 32 * h) * cv->sequence);
+            if (et == 0) tma_store_commit();  // an empty group: one per chunk, see below
+            continue;
+          }
+        }
         uint8_t* dst_row = stag_gen + (c & 1) * kPjOutChunkBytes + row * 128;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -378,13 +523,20 @@ __device__ __forceinline__ void proj_gemm_body(const CUtensorMap& tm_a, const CU
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPjThreads, 1)
 proj_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                       const __grid_constant__ CUtensorMap tm_out, const ProjParams p) {
-  proj_gemm_body<true>(tm_a, tm_w, tm_out, p);
+  proj_gemm_body<true, false>(tm_a, tm_w, tm_out, p, nullptr);
 }
 
 __global__ void __launch_bounds__(kPjThreads, 1)
 proj_gemm_lone_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                       const __grid_constant__ CUtensorMap tm_out, const ProjParams p) {
-  proj_gemm_body<false>(tm_a, tm_w, tm_out, p);
+  proj_gemm_body<false, false>(tm_a, tm_w, tm_out, p, nullptr);
+}
+
+// With the convolution tail in the epilogue (see ConvParams).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPjThreads, 1)
+proj_conv_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
+                      const __grid_constant__ CUtensorMap tm_out, const ProjParams p, const ConvParams cv) {
+  proj_gemm_body<true, true>(tm_a, tm_w, tm_out, p, &cv);
 }
 
 }  // namespace so

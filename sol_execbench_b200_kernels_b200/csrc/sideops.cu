@@ -12,6 +12,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "mamba_conv.cuh"
 #include "proj_gemm.cuh"
 
 namespace so {
@@ -104,81 +105,10 @@ rmsnorm_qk_kernel(const float4* __restrict__ query, const float4* __restrict__ k
 // ------------------------------------------------------------------------------------------------------------
 constexpr int kConvChannels = 64;
 constexpr int kConvPositions = 128;
-constexpr int kConvTaps = 4;
 constexpr int kConvRows = kConvPositions + kConvTaps - 1;  // 131
 constexpr int kConvThreads = 256;
 constexpr int kConvOutPitch = kConvPositions / 2 + 2;  // words; even, so that rows stay 8-byte aligned for the 64-bit reads of the store phase
 constexpr int kConvRun = kConvPositions / (kConvThreads / 32);  // positions per warp = 16
-
-__device__ __forceinline__ float ex2_approx(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float2 bf16x2_to_float2(uint32_t w) {
-  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-}
-__device__ __forceinline__ uint32_t float2_to_bf16x2(float2 v) {
-  uint32_t r;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v.y), "f"(v.x));
-  return r;
-}
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-// bf16(a * m) for both halves of a packed word; the fp32 product of two bf16 values is exact, so this is the
-// single rounding of the eager masked multiply
-__device__ __forceinline__ uint32_t mask_mul_bf16x2(uint32_t a, uint32_t m2) { return mul_bf16x2(a, m2); }
-
-// convolution + bias for one position of a channel pair, rounded to bf16 (packed)
-__device__ __forceinline__ uint32_t conv_pair(float2 x0, float2 x1, float2 x2, float2 x3, const float2 (&w)[4],
-                                              float2 bias) {
-  float2 acc = __fmul2_rn(x0, w[0]);
-  acc = __ffma2_rn(x1, w[1], acc);
-  acc = __ffma2_rn(x2, w[2], acc);
-  acc = __ffma2_rn(x3, w[3], acc);
-  acc = __fadd2_rn(acc, bias);
-  return float2_to_bf16x2(acc);
-}
-
-// sigmoid of one value in full relative accuracy at any magnitude: e = 2^(-|x| log2 e) with log2 e split into a
-// 16-bit head (its product with an 8-bit bf16 significand is exact in fp32) and a tail applied as a first-order
-// factor; 1/(1+e) for x >= 0, e/(1+e) for x < 0
-__device__ __noinline__ float sigmoid_wide(float x) {
-  constexpr float kLog2eHead = 1.44268798828125f;      // 0x3fb8aa00
-  constexpr float kLog2eTailLn2 = 4.888495152129525e-06f;  // (log2 e - head) * ln 2
-  const float a = fabsf(x);
-  const float e0 = ex2_approx(-a * kLog2eHead);
-  const float e = fmaf(e0, -a * kLog2eTailLn2, e0);
-  const float r = rcp_approx(1.0f + e);
-  return x < 0.f ? e * r : r;
-}
-
-// bf16(sigmoid) of the four bf16 values in two packed words (channel pair at two positions), all four
-// arguments >= -20: sigmoid = 1 / (1 + 2^(-x log2 e)) directly; each denominator is below 2^30, so the product of
-// the four stays finite and ONE reciprocal of it serves all four (products of the other three give each quotient
-// back): 1.25 special-function operations per element instead of 2.
-__device__ __forceinline__ void sigmoid_2x2(uint32_t ca, uint32_t cb, uint32_t& sa, uint32_t& sb) {
-  constexpr float kNegLog2e = -1.4426950408889634f;
-  const float2 scale = make_float2(kNegLog2e, kNegLog2e);
-  const float2 ta = __fmul2_rn(bf16x2_to_float2(ca), scale);
-  const float2 tb = __fmul2_rn(bf16x2_to_float2(cb), scale);
-  const float2 one = make_float2(1.f, 1.f);
-  const float2 ya = __fadd2_rn(make_float2(ex2_approx(ta.x), ex2_approx(ta.y)), one);
-  const float2 yb = __fadd2_rn(make_float2(ex2_approx(tb.x), ex2_approx(tb.y)), one);
-  const float2 pab = __fmul2_rn(ya, yb);        // (ya.x*yb.x, ya.y*yb.y)
-  const float inv = rcp_approx(pab.x * pab.y);  // 1 / (all four)
-  const float2 rab = make_float2(inv * pab.y, inv * pab.x);  // 1/(ya.x*yb.x), 1/(ya.y*yb.y)
-  sa = float2_to_bf16x2(__fmul2_rn(rab, yb));   // 1/ya
-  sb = float2_to_bf16x2(__fmul2_rn(rab, ya));   // 1/yb
-}
 
 __global__ void __launch_bounds__(kConvThreads, 5)  // 48 registers: 5 CTAs per SM; forcing 6 (40 registers) measured 7 % slower
 mamba_conv1d_tail_kernel(const __nv_bfloat16* projected, const __nv_bfloat16* mask, const __nv_bfloat16* conv_weight,
@@ -252,12 +182,7 @@ mamba_conv1d_tail_kernel(const __nv_bfloat16* projected, const __nv_bfloat16* ma
   // ---- per-thread constants: taps and bias of this lane's channel pair ----
   float2 w[4], bias;
   {
-    const float2 wa01 = bf16x2_to_float2(wq.x), wa23 = bf16x2_to_float2(wq.y);  // channel c, taps 0..3
-    const float2 wb01 = bf16x2_to_float2(wq.z), wb23 = bf16x2_to_float2(wq.w);  // channel c + 1
-    w[0] = make_float2(wa01.x, wb01.x);
-    w[1] = make_float2(wa01.y, wb01.y);
-    w[2] = make_float2(wa23.x, wb23.x);
-    w[3] = make_float2(wa23.y, wb23.y);
+    unpack_taps(wq, w);
     bias = bf16x2_to_float2(bq);
   }
   __syncthreads();
@@ -366,6 +291,57 @@ mamba_conv1d_tail_kernel(const __nv_bfloat16* projected, const __nv_bfloat16* ma
 }
 
 // ------------------------------------------------------------------------------------------------------------
+// The outputs that the projection with the convolution in its epilogue leaves open: positions whose taps reach over an
+// edge of the 128-row blocks its CTAs own, at most three per block.  The projection has stored the three rows on either
+// side of every edge; a thread takes a channel pair at one edge.  (15 edges of 16384 channels: 2 % of the tail's work.)
+// ------------------------------------------------------------------------------------------------------------
+constexpr int kEdgeThreads = 256;
+__global__ void __launch_bounds__(kEdgeThreads)
+mamba_conv1d_edges_kernel(const __nv_bfloat16* projected, const __nv_bfloat16* mask, const __nv_bfloat16* conv_weight,
+                          const __nv_bfloat16* conv_bias, __nv_bfloat16* output, int first, int rows, int sequence,
+                          int channels, long long width) {
+  if (threadIdx.x == 0) gu::pdl_trigger();
+  const int c = 2 * static_cast<int>(blockIdx.x * kEdgeThreads + threadIdx.x);
+  const int edge = kPjTileM * (first + static_cast<int>(blockIdx.y) + 1);  // first row of a block; edge < rows
+  gu::pdl_wait();
+  if (c >= channels) return;
+  constexpr int kHist = kConvTaps - 1;
+  uint32_t x[2 * kHist];  // masked rows edge - 3 .. edge + 2
+  uint32_t keep[kHist];
+#pragma unroll
+  for (int i = 0; i < 2 * kHist; ++i) {
+    const int r = edge - kHist + i;
+    x[i] = 0u;
+    if (r < rows) {
+      const uint32_t mb = gu::ld_dep(reinterpret_cast<const uint16_t*>(mask) + r);
+      x[i] = mask_mul_bf16x2(gu::ld_dep(reinterpret_cast<const uint32_t*>(projected + r * width + c)), mb | (mb << 16));
+      if (i >= kHist) keep[i - kHist] = conv_keeps(mb);
+    }
+  }
+  float2 w[4];
+  unpack_taps(gu::ld_dep(reinterpret_cast<const uint4*>(conv_weight + static_cast<long long>(c) * kConvTaps)), w);
+  const float2 bias = bf16x2_to_float2(gu::ld_dep(reinterpret_cast<const uint32_t*>(conv_bias + c)));
+#pragma unroll
+  for (int q = 0; q < kHist; ++q) {
+    const int r = edge + q;
+    if (r >= rows) break;
+    const int b = r / sequence, l = r - b * sequence;
+    if (min(l, kHist) <= q) continue;  // all its taps lie in the block: done there
+    float2 t[kHist];  // positions l - 3 .. l - 1, zero before the sequence start
+#pragma unroll
+    for (int k = 0; k < kHist; ++k) t[k] = bf16x2_to_float2(l >= kHist - k ? x[q + k] : 0u);
+    const uint32_t conv = conv_pair(t[0], t[1], t[2], bf16x2_to_float2(x[q + kHist]), w, bias);
+    const bool small = __hbge2(*reinterpret_cast<const __nv_bfloat162*>(&conv), __floats2bfloat162_rn(-20.f, -20.f));
+    uint32_t ra, rb;
+    silu_2x2(conv, conv, small, ra, rb);
+    if (!keep[q]) ra = 0u;
+    uint16_t* dst = reinterpret_cast<uint16_t*>(output) + (static_cast<long long>(b) * channels + c) * sequence + l;
+    dst[0] = static_cast<uint16_t>(ra);
+    dst[sequence] = static_cast<uint16_t>(ra >> 16);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------------------
 // Host side of the input projection: tensor maps, per-device set-up, launch.
 // ------------------------------------------------------------------------------------------------------------
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -429,6 +405,8 @@ int proj_device(ProjDevice** out) {
     if (major != 10) return SO_EDEVICE;
     if (cudaFuncSetAttribute(proj_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              PjCfg<true>::pair_smem_bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(proj_conv_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             PjCfg<true>::pair_smem_bytes) != cudaSuccess ||
         cudaFuncSetAttribute(proj_gemm_lone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPjSmemBudget) !=
             cudaSuccess) {
       cudaGetLastError();
@@ -458,8 +436,9 @@ int proj_device(ProjDevice** out) {
   return SO_OK;
 }
 
+// `conv`: on CTA pairs the convolution runs in the epilogue of the first conv->channels columns; `fused` says whether it did.
 int launch_projection(const void* hidden, const void* weight, const void* bias, void* projected, int64_t m, int64_t k,
-                      int64_t n, cudaStream_t stream) {
+                      int64_t n, const ConvParams* conv, bool* fused, cudaStream_t stream) {
   ProjDevice* dev = nullptr;
   int rc = proj_device(&dev);
   if (rc != SO_OK) return rc;
@@ -492,6 +471,11 @@ int launch_projection(const void* hidden, const void* weight, const void* bias, 
     const int clusters = p.num_tiles < dev->pair_clusters ? p.num_tiles : dev->pair_clusters;
     p.stages = PjCfg<true>::pair_stages;
     p.staging_in_ring = 0;
+    if (conv) {
+      *fused = true;
+      return launch(proj_conv_pair_kernel, dim3(2 * clusters), kPjThreads, PjCfg<true>::pair_smem_bytes, stream, tm_a, tm_w, tm_o,
+                    p, *conv);
+    }
     return launch(proj_gemm_pair_kernel, dim3(2 * clusters), kPjThreads, PjCfg<true>::pair_smem_bytes, stream, tm_a, tm_w, tm_o,
                   p);
   }
@@ -547,9 +531,8 @@ int so_rmsnorm_qk(const float* query, const float* key, const float* weight_q, c
   return cudaGetLastError() == cudaSuccess ? SO_OK : SO_ECUDA;
 }
 
-int so_mamba_conv1d_tail(const void* projected, const void* attention_mask, const void* conv_weight,
-                         const void* conv_bias, void* output, int64_t batch, int64_t sequence, int64_t channels,
-                         int64_t projected_width, void* stream) {
+static int check_conv1d_tail(const void* projected, const void* attention_mask, const void* conv_weight, const void* conv_bias,
+                             const void* output, int64_t batch, int64_t sequence, int64_t channels, int64_t projected_width) {
   if (!projected || !attention_mask || !conv_weight || !conv_bias || !output) return SO_EINVAL_NULL;
   if (batch < 0 || sequence < 0 || channels < so::kConvChannels || channels % so::kConvChannels != 0 ||
       projected_width < channels || projected_width % 8 != 0 || batch > 65535 || sequence > (1ll << 30) ||
@@ -558,9 +541,17 @@ int so_mamba_conv1d_tail(const void* projected, const void* attention_mask, cons
   if (!so::aligned16(projected) || !so::aligned16(conv_weight) || (reinterpret_cast<uintptr_t>(conv_bias) & 3u) ||
       (reinterpret_cast<uintptr_t>(attention_mask) & 1u) || !so::aligned16(output))
     return SO_EINVAL_ALIGN;
+  return (sequence + so::kConvPositions - 1) / so::kConvPositions > 65535 ? SO_EINVAL_SHAPE : SO_OK;
+}
+
+int so_mamba_conv1d_tail(const void* projected, const void* attention_mask, const void* conv_weight,
+                         const void* conv_bias, void* output, int64_t batch, int64_t sequence, int64_t channels,
+                         int64_t projected_width, void* stream) {
+  const int rc = check_conv1d_tail(projected, attention_mask, conv_weight, conv_bias, output, batch, sequence, channels,
+                                   projected_width);
+  if (rc != SO_OK) return rc;
   if (batch == 0 || sequence == 0) return SO_OK;
   const long long seq_tiles = (sequence + so::kConvPositions - 1) / so::kConvPositions;
-  if (seq_tiles > 65535) return SO_EINVAL_SHAPE;
   const dim3 grid(static_cast<unsigned>(channels / so::kConvChannels), static_cast<unsigned>(seq_tiles),
                   static_cast<unsigned>(batch));
   return so::launch(so::mamba_conv1d_tail_kernel, grid, so::kConvThreads, 0, static_cast<cudaStream_t>(stream),
@@ -570,15 +561,59 @@ int so_mamba_conv1d_tail(const void* projected, const void* attention_mask, cons
                     projected_width);
 }
 
-int so_mamba_in_proj(const void* hidden, const void* weight, const void* bias, void* projected, int64_t m, int64_t k,
-                     int64_t n, void* stream) {
+static int check_in_proj(const void* hidden, const void* weight, const void* bias, const void* projected, int64_t m, int64_t k,
+                         int64_t n) {
   if (!hidden || !weight || !bias || !projected) return SO_EINVAL_NULL;
   if (m < 0 || k < 8 || n < 8 || k % 8 != 0 || n % 8 != 0 || m >= (1ll << 31) || k >= (1ll << 31) || n >= (1ll << 31))
     return SO_EINVAL_SHAPE;
   if (!so::aligned16(hidden) || !so::aligned16(weight) || !so::aligned16(bias) || !so::aligned16(projected))
     return SO_EINVAL_ALIGN;
+  return SO_OK;
+}
+
+int so_mamba_in_proj(const void* hidden, const void* weight, const void* bias, void* projected, int64_t m, int64_t k,
+                     int64_t n, void* stream) {
+  const int rc = check_in_proj(hidden, weight, bias, projected, m, k, n);
+  if (rc != SO_OK || m == 0) return rc;
+  return so::launch_projection(hidden, weight, bias, projected, m, k, n, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+int so_mamba_in_proj_conv(const void* hidden, const void* weight, const void* bias, void* projected,
+                          const void* attention_mask, const void* conv_weight, const void* conv_bias, void* output,
+                          int64_t batch, int64_t sequence, int64_t k, int64_t n, int64_t channels, void* stream_v) {
+  if (batch < 0 || sequence < 0 || (sequence > 0 && batch > (1ll << 31) / sequence)) return SO_EINVAL_SHAPE;
+  const int64_t m = batch * sequence;
+  int rc = check_in_proj(hidden, weight, bias, projected, m, k, n);
+  if (rc != SO_OK) return rc;
+  if ((rc = check_conv1d_tail(projected, attention_mask, conv_weight, conv_bias, output, batch, sequence, channels, n)) != SO_OK)
+    return rc;
   if (m == 0) return SO_OK;
-  return so::launch_projection(hidden, weight, bias, projected, m, k, n, static_cast<cudaStream_t>(stream));
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  so::ConvParams c;
+  c.mask = static_cast<const uint16_t*>(attention_mask);
+  c.weight = static_cast<const __nv_bfloat16*>(conv_weight);
+  c.bias = static_cast<const __nv_bfloat16*>(conv_bias);
+  c.out = static_cast<uint16_t*>(output);
+  c.sequence = static_cast<int>(sequence);
+  c.channels = static_cast<int>(channels);
+  bool fused = false;
+  if ((rc = so::launch_projection(hidden, weight, bias, projected, m, k, n, &c, &fused, stream)) != SO_OK) return rc;
+  if (!fused)
+    return so_mamba_conv1d_tail(projected, attention_mask, conv_weight, conv_bias, output, batch, sequence, channels, n, stream_v);
+  const int64_t edges = (m - 1) / so::kPjTileM;
+  if (edges == 0) return SO_OK;
+  const dim3 grid(static_cast<unsigned>((channels / 2 + so::kEdgeThreads - 1) / so::kEdgeThreads), 1);
+  // (grid.y is at most 65535: 8 million rows at a time)
+  for (int64_t first = 0; first < edges; first += 65535) {
+    const int64_t count = edges - first < 65535 ? edges - first : 65535;
+    rc = so::launch(so::mamba_conv1d_edges_kernel, dim3(grid.x, static_cast<unsigned>(count)), so::kEdgeThreads, 0, stream,
+                    static_cast<const __nv_bfloat16*>(projected), static_cast<const __nv_bfloat16*>(attention_mask),
+                    static_cast<const __nv_bfloat16*>(conv_weight), static_cast<const __nv_bfloat16*>(conv_bias),
+                    static_cast<__nv_bfloat16*>(output), static_cast<int>(first), static_cast<int>(m),
+                    static_cast<int>(sequence), static_cast<int>(channels), static_cast<long long>(n));
+    if (rc != SO_OK) return rc;
+  }
+  return SO_OK;
 }
 
 int so_last_status(int* detail, int clear) {

@@ -18,6 +18,7 @@ from .kernel import _on, _stream_ptr
 HEAD_DIM = 128
 CONV_TAPS = 4
 CONV_CHANNEL_TILE = 64
+PAIR_ROWS = 128  # above these the projection runs on CTA pairs, whose epilogue can take the convolution tail
 
 
 def _need(cond: bool, msg: str) -> None:
@@ -149,22 +150,49 @@ def mamba_conv1d_with_gating(hidden_states: torch.Tensor, attention_mask: torch.
                              conv1d_bias: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """Problem 029 as the reference exposes it: (output_hidden_states [B, C, L], gate [B, C, L] view).
 
-    Two launches of this package's kernels: the input projection (a tcgen05 bf16 GEMM with the bias in its epilogue;
-    the reference uses a CUTLASS builder GEMM there, kernel.cu:36-160) and the convolution tail.  `gate` is the
-    transposed view of the projection's upper half, as in the reference (binding.cpp:88-92).
+    Two launches of this package's kernels.  Up to 128 rows the input projection (a tcgen05 bf16 GEMM with the bias in its
+    epilogue; the reference uses a CUTLASS builder GEMM there, kernel.cu:36-160) and the convolution tail; above, the
+    projection with the tail in its epilogue, and a small kernel for the positions at the edges of its row blocks.  `gate`
+    is the transposed view of the projection's upper half, as in the reference (binding.cpp:88-92); the lower half of that
+    buffer is scratch.
     """
     _need(hidden_states.dim() == 3, "hidden_states must have shape [B, L, H]")
     projected_width = in_proj_weight.shape[0]
     _need(projected_width % 2 == 0, "in_proj_weight must have an even number of rows")
     channels = projected_width // 2
-    projected = torch.empty(hidden_states.shape[0], hidden_states.shape[1], projected_width,
-                            dtype=hidden_states.dtype, device=hidden_states.device)
-    mamba_in_proj(hidden_states, in_proj_weight, in_proj_bias, projected)
-    gate = projected[:, :, channels:].transpose(1, 2)
-    out = torch.empty(hidden_states.shape[0], channels, hidden_states.shape[1], dtype=hidden_states.dtype,
-                      device=hidden_states.device)
-    mamba_conv1d_tail(projected, attention_mask, conv1d_weight, conv1d_bias, out)
-    return out, gate
+    batch, sequence = hidden_states.shape[:2]
+    if batch * sequence <= PAIR_ROWS:
+        projected = torch.empty(batch, sequence, projected_width, dtype=hidden_states.dtype, device=hidden_states.device)
+        mamba_in_proj(hidden_states, in_proj_weight, in_proj_bias, projected)
+        out = torch.empty(batch, channels, sequence, dtype=hidden_states.dtype, device=hidden_states.device)
+        mamba_conv1d_tail(projected, attention_mask, conv1d_weight, conv1d_bias, out)
+        return out, projected[:, :, channels:].transpose(1, 2)
+    # the checks of those two functions, of what the caller passed (one call into the library, so all come first)
+    _need(in_proj_weight.dim() == 2, "in_proj_weight must have shape [N, K]")
+    k = in_proj_weight.shape[1]
+    if hidden_states.shape[2] != k:
+        raise ValueError(f"hidden_states must have shape [..., {k}]")
+    if in_proj_bias.shape != (projected_width,):
+        raise ValueError(f"in_proj_bias must have shape [{projected_width}]")
+    _need(k % 8 == 0 and projected_width % 8 == 0 and k >= 8 and projected_width >= 8, "K and N must be multiples of 8")
+    if conv1d_bias.dim() != 1 or conv1d_bias.shape[0] < CONV_CHANNEL_TILE or conv1d_bias.shape[0] % CONV_CHANNEL_TILE:
+        raise ValueError(f"conv1d_bias must have shape [C] with C a multiple of {CONV_CHANNEL_TILE}")
+    _need(attention_mask.shape == (batch, sequence), "attention_mask must have shape [B, L]")
+    if conv1d_weight.shape != (conv1d_bias.shape[0], 1, CONV_TAPS):
+        raise ValueError(f"conv1d_weight must have shape [{conv1d_bias.shape[0]}, 1, 4]")
+    _need(conv1d_bias.shape[0] == channels, "output_hidden_states must have shape [B, C, L]")
+    device = hidden_states.device
+    for t, name in ((hidden_states, "hidden_states"), (in_proj_weight, "in_proj_weight"), (in_proj_bias, "in_proj_bias"),
+                    (attention_mask, "attention_mask"), (conv1d_weight, "conv1d_weight"), (conv1d_bias, "conv1d_bias")):
+        _check_bf16(t, name, device)
+    projected = torch.empty(batch, sequence, projected_width, dtype=torch.bfloat16, device=device)
+    out = torch.empty(batch, channels, sequence, dtype=torch.bfloat16, device=device)
+    with _on(device):
+        _so.check(_so.lib.so_mamba_in_proj_conv(
+            hidden_states.data_ptr(), in_proj_weight.data_ptr(), in_proj_bias.data_ptr(), projected.data_ptr(),
+            attention_mask.data_ptr(), conv1d_weight.data_ptr(), conv1d_bias.data_ptr(), out.data_ptr(),
+            batch, sequence, k, projected_width, channels, _stream_ptr(device)))
+    return out, projected[:, :, channels:].transpose(1, 2)
 
 
 def launch_count() -> int:

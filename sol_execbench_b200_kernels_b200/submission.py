@@ -84,8 +84,8 @@ PROBLEMS: Dict[str, Dict[str, Any]] = {
                        "issued before the reduction, HBM-bound.",
         "destination_passing_style": True,
         "sources": [("binding.cpp", BINDINGS / "binding_038.cpp"), ("sideops.cu", CSRC / "sideops.cu"),
-                    ("proj_gemm.cuh", CSRC / "proj_gemm.cuh"), ("ptx_sm100.cuh", CSRC / "ptx_sm100.cuh"),
-                    ("sideops.h", INCLUDE / "sideops.h")],
+                    ("proj_gemm.cuh", CSRC / "proj_gemm.cuh"), ("mamba_conv.cuh", CSRC / "mamba_conv.cuh"),
+                    ("ptx_sm100.cuh", CSRC / "ptx_sm100.cuh"), ("sideops.h", INCLUDE / "sideops.h")],
     },
     "29": {
         "definition": "029_mamba_conv1d_with_gating",
@@ -95,8 +95,8 @@ PROBLEMS: Dict[str, Dict[str, Any]] = {
                        "[L, C] -> [C, L] transposition with packed f32x2 arithmetic.",
         "destination_passing_style": False,
         "sources": [("binding.cpp", BINDINGS / "binding_029.cpp"), ("sideops.cu", CSRC / "sideops.cu"),
-                    ("proj_gemm.cuh", CSRC / "proj_gemm.cuh"), ("ptx_sm100.cuh", CSRC / "ptx_sm100.cuh"),
-                    ("sideops.h", INCLUDE / "sideops.h")],
+                    ("proj_gemm.cuh", CSRC / "proj_gemm.cuh"), ("mamba_conv.cuh", CSRC / "mamba_conv.cuh"),
+                    ("ptx_sm100.cuh", CSRC / "ptx_sm100.cuh"), ("sideops.h", INCLUDE / "sideops.h")],
     },
 }
 
