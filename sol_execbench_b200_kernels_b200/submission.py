@@ -90,9 +90,9 @@ PROBLEMS: Dict[str, Dict[str, Any]] = {
     "29": {
         "definition": "029_mamba_conv1d_with_gating",
         "name": "mamba_in_proj_tcgen05_conv1d_tail_packed_f32x2",
-        "description": "Mamba input projection as a persistent tcgen05 bf16 GEMM on CTA pairs with the bias in its "
-                       "epilogue, then one kernel for mask, depthwise causal conv1d, SiLU, mask and the "
-                       "[L, C] -> [C, L] transposition with packed f32x2 arithmetic.",
+        "description": "Mamba input projection as a persistent tcgen05 bf16 GEMM on CTA pairs with the bias, mask, "
+                       "depthwise causal conv1d, SiLU, mask and the [L, C] -> [C, L] transposition in its epilogue "
+                       "(up to 128 rows a second kernel for what follows the bias), packed f32x2 arithmetic.",
         "destination_passing_style": False,
         "sources": [("binding.cpp", BINDINGS / "binding_029.cpp"), ("sideops.cu", CSRC / "sideops.cu"),
                     ("proj_gemm.cuh", CSRC / "proj_gemm.cuh"), ("mamba_conv.cuh", CSRC / "mamba_conv.cuh"),
