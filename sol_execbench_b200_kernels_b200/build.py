@@ -16,7 +16,7 @@ CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libgateup.so"
 SOURCES = [CSRC / "gateup.cu"]
 HEADERS = [CSRC / "ptx_sm100.cuh", CSRC / "gateup_tile.cuh", CSRC / "gateup_pair.cuh", CSRC / "gateup_stream.cuh",
-           CSRC / "gateup_split.cuh", CSRC / "quantize_act.cuh", CSRC / "reduce_gather.cuh", PKG_DIR.parent / "include" / "gateup.h"]
+           CSRC / "gateup_split.cuh", CSRC / "gateup_mlp.cuh", CSRC / "quantize_act.cuh", CSRC / "reduce_gather.cuh", PKG_DIR.parent / "include" / "gateup.h"]
 # the same library with the pair kernel's per-role cycle counters compiled in (gu_trace_read); a profiling aid
 TRACE_LIB_PATH = PKG_DIR / "libgateup_trace.so"
 

@@ -15,6 +15,7 @@
 #include "gateup_pair.cuh"
 #include "gateup_tile.cuh"
 #include "gateup_split.cuh"
+#include "gateup_mlp.cuh"
 #include "quantize_act.cuh"
 #include "reduce_gather.cuh"
 
@@ -136,6 +137,8 @@ int device_info(DeviceInfo** out) {
             cudaSuccess ||
         cudaFuncSetAttribute(gateup_stream_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
             cudaSuccess ||
+        cudaFuncSetAttribute(mlp_step_kernel<kMlpGateUp>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaFuncSetAttribute(mlp_step_kernel<kMlpDown>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
         cudaFuncSetAttribute(gateup_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
         cudaFuncSetAttribute(blockwise_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
             cudaSuccess ||
@@ -667,6 +670,66 @@ int launch_split_run(const gu_problem* pr, int splits, cudaStream_t stream) {
   return launch_split<kSplitGateUp>(p, m, k, n, n / kTileN, splits, tm_x, tm_g, tm_u, stream);
 }
 
+// ---------------------------------------------------------------------------
+// The MLP block with up to 16 tokens on the kernels of gateup_mlp.cuh.  Scratch: the launch count and tickets (the first
+// page), then the {sum, stamp} pairs of at most kStreamMaxGrid ranges; all zeroed once.
+// ---------------------------------------------------------------------------
+size_t mlp_stream_bytes(int64_t sm_count) {
+  return 4096 + size_t(sm_count < kStreamMaxGrid ? sm_count : kStreamMaxGrid) * kMlpSlotPairs * sizeof(uint2);
+}
+// How a pass over nb column blocks of kb K blocks is cut and what it keeps in shared memory.
+struct MlpGeometry {
+  int64_t grid, kept;
+  int stages;
+};
+MlpGeometry mlp_geometry(int op, int64_t nb, int64_t kb, int64_t sm_count) {
+  const int64_t steps = (kb + mlp_blocks_per_unit(op) - 1) / mlp_blocks_per_unit(op), units = nb * steps;
+  MlpGeometry g;
+  g.grid = sm_count < kStreamMaxGrid ? sm_count : kStreamMaxGrid;
+  if (units < g.grid) g.grid = units;
+  const int64_t range = (units + g.grid - 1) / g.grid;
+  g.kept = range < steps ? range : steps;
+  const int64_t left = g.kept > 1024 ? 0 : int64_t(kSmemBudget) - mlp_fixed_bytes(op, g.kept);
+  const int64_t fit = left > 0 ? left / mlp_stage_bytes(op) : 0;
+  g.stages = static_cast<int>(fit < kMlpMaxStages ? fit : kMlpMaxStages);
+  return g;
+}
+// Whether a step of the block streams its weights; `nb` column blocks of `kb` K blocks.  us of the whole block on B200, tiles /
+// streamed, (tokens, hidden, intermediate):
+//  * Gate/up, against whole tiles (there is no cut along K from 75 column blocks on): it gains what whole tiles leave idle
+//    in their last round and pays the joins.  62 of 148 SMs idle, (8, 4096, 11008), 36.7 / 34.5; 72 in two rounds,
+//    (8, 8192, 28672) 126.0 / 114.1 and (8, 1024, 28672) 38.9 / 35.1; 40, (8, 5120, 13824), 44.9 / 44.8; 36, (8, 4096,
+//    14336), 40.3 / 39.9 and with 16 tokens 40.9 / 41.7; 20, (8, 6144, 16384), 57.3 / 57.5; none, (8, 3584, 18944),
+//    43.9 / 44.0.  Where tiles are cut along K, (8, 8192, 8192), 41.8 / 43.5.
+//  * Down, against tiles cut along K in clusters: (8, 8192, 28672) 114.1 / 112.6 with gate/up streamed, (8, 4096, 14336)
+//    41.4 / 40.3, (8, 4096, 11008) 38.2 / 36.7, (8, 8192, 8192) 42.3 / 41.8, (8, 5120, 8192) 32.4 / 32.4, (8, 2048, 14336)
+//    30.2 / 30.7, (8, 2048, 5632) 20.9 / 21.6: from 9 units per CTA on; and with fewer where the clusters' K ranges are
+//    long, (8, 2048, 28672) 53.7 / 46.8, (8, 1024, 28672) 46.8 / 38.9.  (Below 8 column blocks an owner would collect more
+//    than 18 ranges.)
+bool mlp_step_streams(int op, int64_t m, int64_t kb, int64_t nb, int64_t sm_count) {
+  if (m > kMlpTokens || nb * kb >= (1ll << 31)) return false;
+  const MlpGeometry g = mlp_geometry(op, nb, kb, sm_count);
+  if (g.stages < 4) return false;
+#ifdef GU_BOUNDS
+  return true;  // (small shapes reach these kernels in the range-checked build only)
+#endif
+  const int64_t steps = (kb + mlp_blocks_per_unit(op) - 1) / mlp_blocks_per_unit(op);
+  const bool long_ranges = nb * steps >= 9 * g.grid;
+  if (op == kMlpDown) return nb >= 8 && (long_ranges || kb >= 160);
+  const int64_t idle = (nb + sm_count - 1) / sm_count * sm_count - nb;
+  return long_ranges && 2 * nb > sm_count && 148 * idle >= (m <= 8 ? 36 : 40) * sm_count;
+}
+template <int kOp>
+int launch_mlp_step(MlpStepParams& p, const DeviceInfo& dev, void* scratch, cudaStream_t stream, const CUtensorMap& tm_x,
+                    const CUtensorMap& tm_w0, const CUtensorMap& tm_w1) {
+  const MlpGeometry g = mlp_geometry(kOp, p.nb, p.kb, dev.sm_count);
+  p.stages = g.stages;
+  p.weights_ready = 1;  // (only behind the block's quantiser)
+  p.sync = static_cast<unsigned int*>(scratch);
+  p.partials = reinterpret_cast<uint2*>(static_cast<uint8_t*>(scratch) + 4096);
+  return launch(mlp_step_kernel<kOp>, static_cast<int>(g.grid), kStreamThreads,
+                g.stages * mlp_stage_bytes(kOp) + mlp_fixed_bytes(kOp, g.kept), stream, 1, tm_x, tm_w0, tm_w1, p);
+}
 int quantize_launch(const void* x, int x_is_f32, int64_t ld_x, void* q, float* scale, int64_t m, int64_t k,
                     void* stream_v) {
   if (!x || !q || !scale) return GU_EINVAL_NULL;
@@ -708,7 +771,7 @@ int quantize_launch(const void* x, int x_is_f32, int64_t ld_x, void* q, float* s
 
 // `chained`: a step of gu_mlp_block.  The chain opens with the block's quantiser, which lets nothing start before all in
 // front of it has completed, so the weights of both steps are ready.  `cut`: tiles may be cut along K.
-int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chained, bool cut, void* stream_v) {
+int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chained, bool cut, void* scratch, void* stream_v) {
   if (!pr || !out_q || !out_scale) return GU_EINVAL_NULL;
   if (!pr->x || !pr->scale_x || !pr->gate_w || !pr->scale_gate || !pr->up_w || !pr->scale_up) return GU_EINVAL_NULL;
   if (!shape_ok(pr->m, pr->k, pr->n)) return GU_EINVAL_SHAPE;
@@ -726,6 +789,22 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
   if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
 
+  if (scratch && mlp_step_streams(kMlpGateUp, m, k / 128, n / 128, dev->sm_count)) {
+    CUtensorMap tm_rows;
+    if ((rc = get_map(&tm_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, kMlpTokens)) != GU_OK) return rc;
+    MlpStepParams mp;
+    std::memset(&mp, 0, sizeof(mp));
+    mp.scale_x = pr->scale_x;
+    mp.scale_gate = pr->scale_gate;
+    mp.scale_up = pr->scale_up;
+    mp.out = out_q;
+    mp.scale_out = out_scale;
+    mp.ld_out = n;
+    mp.m = static_cast<int>(m);
+    mp.kb = static_cast<int>(k / 128);
+    mp.nb = static_cast<int>(n / 128);
+    return launch_mlp_step<kMlpGateUp>(mp, *dev, scratch, static_cast<cudaStream_t>(stream_v), tm_rows, tm_g, tm_u);
+  }
   if (cut) {
     const int splits = split_ctas(*dev, m, k / 128, n / kTileN, chained);
     if (splits > 1) {
@@ -782,7 +861,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
 }
 
 int gemm_launch(const void* a, const float* scale_a, const void* b, const float* scale_b, void* c, int64_t m,
-                int64_t k, int64_t n, int64_t ld_c, bool chained, bool cut, void* stream_v) {
+                int64_t k, int64_t n, int64_t ld_c, bool chained, bool cut, void* scratch, void* stream_v) {
   if (!a || !scale_a || !b || !scale_b || !c) return GU_EINVAL_NULL;
   if (!shape_ok(m, k, n) || ld_c < n) return GU_EINVAL_SHAPE;
   if (!aligned16(a) || !aligned16(b) || !aligned16(c) || (reinterpret_cast<uintptr_t>(scale_a) & 3u) ||
@@ -797,6 +876,20 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
   if ((rc = get_map(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, n, m, ld_c * 2, 64, 128)) != GU_OK) return rc;
 
+  if (scratch && mlp_step_streams(kMlpDown, m, k / 128, n / 128, dev->sm_count)) {
+    CUtensorMap tm_rows;
+    if ((rc = get_map(&tm_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k, 128, kMlpTokens)) != GU_OK) return rc;
+    MlpStepParams mp;
+    std::memset(&mp, 0, sizeof(mp));
+    mp.scale_x = scale_a;
+    mp.scale_gate = scale_b;
+    mp.out = c;
+    mp.ld_out = ld_c;
+    mp.m = static_cast<int>(m);
+    mp.kb = static_cast<int>(k / 128);
+    mp.nb = static_cast<int>(n / 128);
+    return launch_mlp_step<kMlpDown>(mp, *dev, scratch, static_cast<cudaStream_t>(stream_v), tm_rows, tm_b, tm_b);
+  }
   if (cut) {
     const int64_t col_tiles = (n / 128 + 1) / 2;
     const int splits = split_ctas(*dev, m, k / 128, col_tiles, chained);
@@ -922,6 +1015,9 @@ int gu_select_tile_kernel(int op, int64_t m, int64_t k, int64_t n, int with_work
   if (op != GU_OP_GATEUP && op != GU_OP_GATEUP_FP8 && op != GU_OP_GEMM) return GU_EINVAL_PLAN;
   const int sms = gu::sm_count_or_default(), clusters = sms / 2;
   const int64_t col_tiles = op == GU_OP_GEMM ? (n / 128 + 1) / 2 : n / gu::kTileN;
+  if (in_mlp && with_workspace == 2 &&
+      gu::mlp_step_streams(op == GU_OP_GEMM ? gu::kMlpDown : gu::kMlpGateUp, m, k / 128, n / 128, sms))
+    return GU_PLAN_STREAM;
   if (with_workspace && (in_mlp || op == GU_OP_GATEUP) && gu::prefers_split(m, k / 128, col_tiles, clusters, in_mlp))
     return GU_PLAN_TILE_SPLIT;
   if (gu::tile_prefers_lone(op, m, k / 128, col_tiles, sms, clusters, with_workspace != 0)) {
@@ -1280,15 +1376,31 @@ int gu_quantize_activation(const void* x, int x_is_f32, int64_t ld_x, void* q, f
 }
 
 int gu_run_fp8out(const gu_problem* pr, void* out_q, float* out_scale, void* stream) {
-  return gu::fp8out_launch(pr, out_q, out_scale, false, false, stream);
+  return gu::fp8out_launch(pr, out_q, out_scale, false, false, nullptr, stream);
 }
 
 int gu_blockwise_gemm(const void* a, const float* scale_a, const void* b, const float* scale_b, void* c, int64_t m,
                       int64_t k, int64_t n, int64_t ld_c, void* stream) {
-  return gu::gemm_launch(a, scale_a, b, scale_b, c, m, k, n, ld_c, false, false, stream);
+  return gu::gemm_launch(a, scale_a, b, scale_b, c, m, k, n, ld_c, false, false, nullptr, stream);
 }
 
-int gu_mlp_block(const gu_mlp* b, void* stream) {
+size_t gu_mlp_workspace_bytes(int64_t m, int64_t k, int64_t n, int64_t h_out) {
+  if (!gu::shape_ok(m, k, n) || !gu::shape_ok(m, n, h_out)) return 0;
+  const int sms = gu::sm_count_or_default();
+  return gu::mlp_step_streams(gu::kMlpGateUp, m, k / 128, n / 128, sms) ||
+                 gu::mlp_step_streams(gu::kMlpDown, m, n / 128, h_out / 128, sms)
+             ? gu::mlp_stream_bytes(sms)
+             : 0;
+}
+
+int gu_mlp_workspace_init(void* workspace, size_t bytes, void* stream) {
+  if (!workspace || bytes == 0) return GU_OK;
+  return cudaMemsetAsync(workspace, 0, bytes, static_cast<cudaStream_t>(stream)) == cudaSuccess ? GU_OK : GU_ECUDA;
+}
+
+int gu_mlp_block(const gu_mlp* b, void* stream) { return gu_mlp_block_ws(b, nullptr, 0, stream); }
+
+int gu_mlp_block_ws(const gu_mlp* b, void* workspace, size_t workspace_bytes, void* stream) {
   if (!b) return GU_EINVAL_NULL;
   // everything is checked before the first launch
   if (!b->x || !b->gate_w || !b->scale_gate || !b->up_w || !b->scale_up || !b->down_w || !b->scale_down || !b->x_q ||
@@ -1304,6 +1416,10 @@ int gu_mlp_block(const gu_mlp* b, void* stream) {
     if (reinterpret_cast<uintptr_t>(p) & 3u) return GU_EINVAL_ALIGN;
   if ((b->ld_x * (b->x_is_f32 ? 4 : 2)) % 16 != 0 || b->ld_output % 8 != 0) return GU_EINVAL_ALIGN;
 
+  // scratch that is too small is no scratch, and whole tiles take none
+  const size_t need = workspace && b->whole_tiles == 0 ? gu_mlp_workspace_bytes(b->m, b->k, b->n, b->h_out) : 0;
+  void* scratch = need > 0 && workspace_bytes >= need ? workspace : nullptr;
+  if (scratch && !gu::aligned16(scratch)) return GU_EINVAL_ALIGN;
   int rc = gu::quantize_launch(b->x, b->x_is_f32, b->ld_x, b->x_q, b->x_scale, b->m, b->k, stream);
   if (rc != GU_OK) return rc;
   gu_problem pr;
@@ -1319,9 +1435,9 @@ int gu_mlp_block(const gu_mlp* b, void* stream) {
   pr.n = b->n;
   // both steps load weights early (`chained`), because the quantiser above is the first launch of the block
   const bool cut = b->whole_tiles == 0;
-  if ((rc = gu::fp8out_launch(&pr, b->mid_q, b->mid_scale, true, cut, stream)) != GU_OK) return rc;
+  if ((rc = gu::fp8out_launch(&pr, b->mid_q, b->mid_scale, true, cut, scratch, stream)) != GU_OK) return rc;
   return gu::gemm_launch(b->mid_q, b->mid_scale, b->down_w, b->scale_down, b->output, b->m, b->n, b->h_out, b->ld_output, true,
-                         cut, stream);
+                         cut, scratch, stream);
 }
 
 int gu_last_status(int* detail, int clear) {

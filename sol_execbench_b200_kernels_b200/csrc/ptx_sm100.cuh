@@ -450,6 +450,16 @@ __device__ __forceinline__ void st_release_gpu(unsigned int* p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// A value and the stamp that says which launch it is of, as one 8-byte access: whoever reads the stamp has the value.
+__device__ __forceinline__ void st_pair(uint2* p, float v, uint32_t stamp) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((static_cast<uint64_t>(stamp) << 32) | __float_as_uint(v)) : "memory");
+}
+__device__ __forceinline__ uint2 ld_pair(const uint2* p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return make_uint2(static_cast<uint32_t>(v), static_cast<uint32_t>(v >> 32));
+}
+
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 // out = bf16( f32(bf16(silu(f32(bf16 gate)))) * f32(bf16 up) ): the three

@@ -31,6 +31,7 @@ _PLANS = {"auto": PLAN_AUTO, "tile": PLAN_TILE, "stream": PLAN_STREAM, "tile_dp"
 # Scratch for the stream-K hand-off, one buffer per (device, stream): it is
 # written and consumed inside a single call and carries no result across calls.
 _WORKSPACES: Dict[Tuple[int, int], torch.Tensor] = {}
+_MLP_WORKSPACES: Dict[Tuple[int, int], torch.Tensor] = {}  # likewise for mlp_block
 
 
 def select_plan(m: int, k: int, n: int) -> str:
@@ -135,19 +136,25 @@ def _scratch_bytes(device_index: int, m: int, k: int, n: int, plan_id: int, whol
     return _cabi.lib.gu_workspace_bytes(m, k, n, plan_id)
 
 
-def _workspace(device: torch.device, stream_ptr: int, nbytes: int) -> Optional[torch.Tensor]:
+@lru_cache(maxsize=4096)
+def _mlp_scratch_bytes(device_index: int, m: int, k: int, n: int, h_out: int) -> int:
+    return _cabi.lib.gu_mlp_workspace_bytes(m, k, n, h_out)
+
+
+def _workspace(device: torch.device, stream_ptr: int, nbytes: int, init=_cabi.lib.gu_workspace_init,
+               kept=_WORKSPACES) -> Optional[torch.Tensor]:
     if nbytes == 0:
         return None
     key = (device.index if device.index is not None else torch.cuda.current_device(), stream_ptr)
-    ws = _WORKSPACES.get(key)
+    ws = kept.get(key)
     if ws is None or ws.numel() < nbytes:
         # Under stream capture (torch.cuda.graph switches to a stream of its own, which no eager call has used) the
         # scratch comes from the graph's memory pool and its initialisation is recorded with the launch: every replay
         # then starts from zeroed flags and a zero epoch counter, which is a valid state for the kernels.  The tensor
         # kept here holds the pool's block alive for later calls on that stream.
         ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _cabi.check(_cabi.lib.gu_workspace_init(ws.data_ptr(), nbytes, stream_ptr))
-        _WORKSPACES[key] = ws
+        _cabi.check(init(ws.data_ptr(), nbytes, stream_ptr))
+        kept[key] = ws
     return ws
 
 
@@ -306,7 +313,9 @@ def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch
         1 if x.dtype == torch.float32 else 0, 1 if whole_tiles else 0)
     with _on(x.device):
         stream_ptr = _stream_ptr(x.device)
-        code = _cabi.lib.gu_mlp_block(ctypes.byref(block), stream_ptr)
+        nbytes = 0 if whole_tiles else _mlp_scratch_bytes(torch.cuda.current_device(), m, k, n, h_out)
+        ws = _workspace(x.device, stream_ptr, nbytes, _cabi.lib.gu_mlp_workspace_init, _MLP_WORKSPACES)
+        code = _cabi.lib.gu_mlp_block_ws(ctypes.byref(block), ws.data_ptr() if ws is not None else None, nbytes, stream_ptr)
     _raise_for(code)
     return output
 

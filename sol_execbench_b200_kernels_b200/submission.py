@@ -74,6 +74,7 @@ PROBLEMS: Dict[str, Dict[str, Any]] = {
         "sources": [("binding.cpp", BINDINGS / "binding_179.cpp"), ("gateup.cu", CSRC / "gateup.cu"),
                     ("gateup_tile.cuh", CSRC / "gateup_tile.cuh"), ("gateup_pair.cuh", CSRC / "gateup_pair.cuh"),
                     ("gateup_stream.cuh", CSRC / "gateup_stream.cuh"), ("gateup_split.cuh", CSRC / "gateup_split.cuh"),
+                    ("gateup_mlp.cuh", CSRC / "gateup_mlp.cuh"),
                     ("quantize_act.cuh", CSRC / "quantize_act.cuh"), ("reduce_gather.cuh", CSRC / "reduce_gather.cuh"),
                     ("ptx_sm100.cuh", CSRC / "ptx_sm100.cuh"), ("gateup.h", INCLUDE / "gateup.h")],
     },
