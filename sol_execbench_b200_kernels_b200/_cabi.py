@@ -6,6 +6,7 @@ this module raises, and every entry point that computes needs a B200.
 from __future__ import annotations
 
 import ctypes
+import struct
 from ctypes import POINTER, Structure, c_char_p, c_int, c_int32, c_int64, c_size_t, c_void_p
 
 from .build import LIB_PATH
@@ -55,6 +56,12 @@ class GuMlp(Structure):
                                               "x_q", "x_scale", "mid_q", "mid_scale", "output")]
     _fields_ += [(name, c_int64) for name in ("m", "k", "n", "h_out", "ld_x", "ld_output")]
     _fields_ += [("x_is_f32", c_int32), ("whole_tiles", c_int32)]
+
+
+# The same two structures as bytes, for callers that fill one per call (less than half of the time that a Structure takes).
+PROBLEM_ARGS = struct.Struct("7Q4q2Q2i")
+MLP_ARGS = struct.Struct("12Q6q2i")
+assert PROBLEM_ARGS.size == ctypes.sizeof(GuProblem) and MLP_ARGS.size == ctypes.sizeof(GuMlp)
 
 
 class GateUpError(RuntimeError):
@@ -125,6 +132,17 @@ def _load() -> ctypes.CDLL:
 
 
 lib = _load()
+
+
+def _taking_bytes(name: str, *rest):
+    """Another handle on an entry point, whose first argument is a packed structure."""
+    fn = lib[name]  # (a new object each time; `lib.name` keeps its own argument types)
+    fn.restype, fn.argtypes = c_int, [c_char_p, *rest]
+    return fn
+
+
+run_packed = _taking_bytes("gu_run", c_void_p)
+mlp_block_packed = _taking_bytes("gu_mlp_block_ws", c_void_p, c_size_t, c_void_p)
 
 
 def error_string(code: int) -> str:

@@ -24,6 +24,7 @@ from ._cabi import (PLAN_AUTO, PLAN_STREAM, PLAN_TILE, PLAN_TILE_DP, PLAN_TILE_P
                     PLAN_TILE_SPLIT, GuProblem)
 
 BLOCK = 128
+_E4M3, _F32 = torch.float8_e4m3fn, torch.float32
 _PLANS = {"auto": PLAN_AUTO, "tile": PLAN_TILE, "stream": PLAN_STREAM, "tile_dp": PLAN_TILE_DP, "tile_sk": PLAN_TILE_SK,
           "tile_pair": PLAN_TILE_PAIR, "tile_pair_sk": PLAN_TILE_PAIR_SK,
           "tile_split": PLAN_TILE_SPLIT}
@@ -111,13 +112,43 @@ def _validate(x, scale_x, gate_w, scale_gate, up_w, scale_up, output) -> Tuple[i
     return m, k, n
 
 
+def _plain(operands, index: int) -> bool:
+    """Whether every (tensor, shape, dtype) is just that, on device `index` and contiguous: what `_check` accepts, seen
+    without building what it needs to say what is wrong."""
+    for t, shape, dtype in operands:
+        if t.shape != shape or t.dtype != dtype or t.get_device() != index or not t.is_contiguous():
+            return False
+    return True
+
+
+def _plainly_valid(x, scale_x, gate_w, scale_gate, up_w, scale_up, output) -> Optional[Tuple[int, int, int]]:
+    """(m, k, n) where `_validate` would accept the call; None sends the caller there.  (Small shapes are bound by the host:
+    1 x 1024 x 4096 12.7 -> 9.7 us a call with this and the packed arguments.)"""
+    xs, gs = x.shape, gate_w.shape
+    if len(xs) != 2 or len(gs) != 2:
+        return None
+    m, k = xs
+    n = gs[0]
+    index = x.get_device()
+    if m < 1 or k < BLOCK or n < BLOCK or k % BLOCK or n % BLOCK or not x.is_cuda:
+        return None
+    kb, nb = k // BLOCK, n // BLOCK
+    if not _plain(((x, (m, k), _E4M3), (scale_x, (m, kb), _F32), (gate_w, (n, k), _E4M3), (scale_gate, (nb, kb), _F32),
+                   (up_w, (n, k), _E4M3), (scale_up, (nb, kb), _F32)), index):
+        return None
+    if output.shape != (m, n) or output.dtype != torch.bfloat16 or output.get_device() != index:
+        return None
+    rows, cols = output.stride()
+    return (m, k, n) if cols == 1 and rows >= n else None
+
+
 _ALREADY_CURRENT = nullcontext()
 
 
 def _on(device: torch.device):
     """Context with `device` current; costs next to nothing when it already is."""
     index = device.index
-    if index is None or index == torch.cuda.current_device():
+    if index is None or index == torch._C._cuda_getDevice():
         return _ALREADY_CURRENT
     return torch.cuda.device(device)
 
@@ -125,7 +156,7 @@ def _on(device: torch.device):
 def _stream_ptr(device: torch.device) -> int:
     """The current stream of `device` as a cudaStream_t, without building a Stream object."""
     index = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice() if index is None else index)
 
 
 @lru_cache(maxsize=4096)
@@ -159,20 +190,21 @@ def _workspace(device: torch.device, stream_ptr: int, nbytes: int, init=_cabi.li
 
 
 def _launch(x, scale_x, gate_w, scale_gate, up_w, scale_up, output, plan: str, whole_tiles: bool = False) -> None:
-    m, k, n = _validate(x, scale_x, gate_w, scale_gate, up_w, scale_up, output)
+    m, k, n = (_plainly_valid(x, scale_x, gate_w, scale_gate, up_w, scale_up, output) or
+               _validate(x, scale_x, gate_w, scale_gate, up_w, scale_up, output))
     plan_id = _PLANS[plan]
     device = x.device
     with _on(device):
         stream_ptr = _stream_ptr(device)
-        nbytes = _scratch_bytes(torch.cuda.current_device(), m, k, n, plan_id, whole_tiles)
-        ws = _workspace(device, stream_ptr, nbytes)
-        pr = GuProblem(
+        nbytes = _scratch_bytes(torch._C._cuda_getDevice(), m, k, n, plan_id, whole_tiles)
+        ws = _workspace(device, stream_ptr, nbytes) if nbytes else None
+        code = _cabi.run_packed(_cabi.PROBLEM_ARGS.pack(
             x.data_ptr(), scale_x.data_ptr(), gate_w.data_ptr(), scale_gate.data_ptr(),
             up_w.data_ptr(), scale_up.data_ptr(), output.data_ptr(),
             m, k, n, output.stride(0),
-            ws.data_ptr() if ws is not None else None, nbytes, plan_id, 0 if whole_tiles else 1)
-        code = _cabi.lib.gu_run(ctypes.byref(pr), stream_ptr)
-    _raise_for(code)
+            ws.data_ptr() if ws is not None else 0, nbytes, plan_id, 0 if whole_tiles else 1), stream_ptr)
+    if code:
+        _raise_for(code)
 
 
 def run(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch.Tensor,
@@ -263,6 +295,16 @@ def run_fp8_output(x: torch.Tensor, scale_x: torch.Tensor, gate_proj_weight: tor
     _raise_for(code)
 
 
+@lru_cache(maxsize=4096)
+def _mlp_layout(m: int, k: int, n: int) -> Tuple[Tuple[int, ...], int]:
+    """Offsets of mlp_block's four intermediates in one allocation, and its size."""
+    offsets, nbytes = [], 0
+    for size in (m * k, 4 * m * (k // BLOCK), m * n, 4 * m * (n // BLOCK)):
+        offsets.append(nbytes)
+        nbytes += (size + 255) // 256 * 256
+    return tuple(offsets), nbytes
+
+
 def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch.Tensor, up_proj_weight: torch.Tensor,
               scale_up: torch.Tensor, down_proj_weight: torch.Tensor, scale_down: torch.Tensor,
               output: Optional[torch.Tensor] = None, whole_tiles: bool = False) -> torch.Tensor:
@@ -284,39 +326,41 @@ def mlp_block(x: torch.Tensor, gate_proj_weight: torch.Tensor, scale_gate: torch
         if cols % BLOCK or rows % BLOCK or cols < BLOCK or rows < BLOCK:
             raise ValueError(f"Unsupported contract shape M={m}, K={cols}, N={rows}: need M >= 1 and K, N multiples of {BLOCK}")
     kb, nb, hb = k // BLOCK, n // BLOCK, h_out // BLOCK
-    expected = {
-        "gate_proj_weight": (gate_proj_weight, (n, k), torch.float8_e4m3fn),
-        "scale_gate": (scale_gate, (nb, kb), torch.float32),
-        "up_proj_weight": (up_proj_weight, (n, k), torch.float8_e4m3fn),
-        "scale_up": (scale_up, (nb, kb), torch.float32),
-        "b": (down_proj_weight, (h_out, n), torch.float8_e4m3fn),
-        "scale_b": (scale_down, (hb, nb), torch.float32),
-    }
-    if output is not None:
-        expected["output"] = (output, (m, h_out), torch.bfloat16)
-    _check(expected, x.device)
+    index = x.get_device()
+    if not _plain(((gate_proj_weight, (n, k), _E4M3), (scale_gate, (nb, kb), _F32), (up_proj_weight, (n, k), _E4M3),
+                   (scale_up, (nb, kb), _F32), (down_proj_weight, (h_out, n), _E4M3), (scale_down, (hb, nb), _F32)), index) or (
+            output is not None and (output.shape != (m, h_out) or output.dtype != torch.bfloat16 or output.get_device() != index)):
+        expected = {
+            "gate_proj_weight": (gate_proj_weight, (n, k), torch.float8_e4m3fn),
+            "scale_gate": (scale_gate, (nb, kb), torch.float32),
+            "up_proj_weight": (up_proj_weight, (n, k), torch.float8_e4m3fn),
+            "scale_up": (scale_up, (nb, kb), torch.float32),
+            "b": (down_proj_weight, (h_out, n), torch.float8_e4m3fn),
+            "scale_b": (scale_down, (hb, nb), torch.float32),
+        }
+        if output is not None:
+            expected["output"] = (output, (m, h_out), torch.bfloat16)
+        _check(expected, x.device)
     if output is None:
         output = torch.empty(m, h_out, dtype=torch.bfloat16, device=x.device)
     elif output.stride(1) != 1 or output.stride(0) < h_out:
         raise ValueError("output must be row-major with unit column stride")
     # one allocation for the quantised activations and the quantised intermediate with their scales
-    offsets, nbytes = [], 0
-    for size in (m * k, 4 * m * kb, m * n, 4 * m * nb):
-        offsets.append(nbytes)
-        nbytes += (size + 255) // 256 * 256
+    offsets, nbytes = _mlp_layout(m, k, n)
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     base = scratch.data_ptr()
-    block = _cabi.GuMlp(
-        x.data_ptr(), gate_proj_weight.data_ptr(), scale_gate.data_ptr(), up_proj_weight.data_ptr(), scale_up.data_ptr(),
-        down_proj_weight.data_ptr(), scale_down.data_ptr(), base + offsets[0], base + offsets[1], base + offsets[2],
-        base + offsets[3], output.data_ptr(), m, k, n, h_out, x.stride(0), output.stride(0),
-        1 if x.dtype == torch.float32 else 0, 1 if whole_tiles else 0)
     with _on(x.device):
         stream_ptr = _stream_ptr(x.device)
-        nbytes = 0 if whole_tiles else _mlp_scratch_bytes(torch.cuda.current_device(), m, k, n, h_out)
-        ws = _workspace(x.device, stream_ptr, nbytes, _cabi.lib.gu_mlp_workspace_init, _MLP_WORKSPACES)
-        code = _cabi.lib.gu_mlp_block_ws(ctypes.byref(block), ws.data_ptr() if ws is not None else None, nbytes, stream_ptr)
-    _raise_for(code)
+        nbytes = 0 if whole_tiles else _mlp_scratch_bytes(torch._C._cuda_getDevice(), m, k, n, h_out)
+        ws = _workspace(x.device, stream_ptr, nbytes, _cabi.lib.gu_mlp_workspace_init, _MLP_WORKSPACES) if nbytes else None
+        code = _cabi.mlp_block_packed(_cabi.MLP_ARGS.pack(
+            x.data_ptr(), gate_proj_weight.data_ptr(), scale_gate.data_ptr(), up_proj_weight.data_ptr(), scale_up.data_ptr(),
+            down_proj_weight.data_ptr(), scale_down.data_ptr(), base + offsets[0], base + offsets[1], base + offsets[2],
+            base + offsets[3], output.data_ptr(), m, k, n, h_out, x.stride(0), output.stride(0),
+            1 if x.dtype == torch.float32 else 0, 1 if whole_tiles else 0),
+            ws.data_ptr() if ws is not None else None, nbytes, stream_ptr)
+    if code:
+        _raise_for(code)
     return output
 
 
