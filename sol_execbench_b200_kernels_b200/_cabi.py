@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import struct
-from ctypes import POINTER, Structure, c_char_p, c_int, c_int32, c_int64, c_size_t, c_void_p
+from ctypes import POINTER, Structure, c_char_p, c_int, c_int32, c_int64, c_size_t, c_uint64, c_void_p
 
 from .build import LIB_PATH
 
@@ -34,7 +34,7 @@ EXPORTS = (
     "gu_version", "gu_error_string", "gu_select_plan", "gu_select_tile_kernel", "gu_workspace_bytes", "gu_workspace_init",
     "gu_run", "gu_run_concat", "gu_last_status", "gu_launch_count", "gu_run_decode_static", "gu_run_gather", "gu_quantize_activation", "gu_blockwise_gemm", "gu_run_fp8out",
     "gu_blockwise_gemm_scatter", "gu_reduce_gather", "gu_set_wait_limit_ns", "gu_trace_read", "gu_wait_probe", "gu_peer_barrier", "gu_is_range_checked_build",
-    "gu_mlp_block", "gu_mlp_block_ws", "gu_mlp_workspace_bytes", "gu_mlp_workspace_init",
+    "gu_mlp_block", "gu_mlp_block_ws", "gu_mlp_workspace_bytes", "gu_mlp_workspace_init", "gu_capture_id",
 )
 
 
@@ -116,6 +116,8 @@ def _load() -> ctypes.CDLL:
     lib.gu_mlp_workspace_bytes.argtypes = [c_int64, c_int64, c_int64, c_int64]
     lib.gu_mlp_workspace_init.restype = c_int
     lib.gu_mlp_workspace_init.argtypes = [c_void_p, c_size_t, c_void_p]
+    lib.gu_capture_id.restype = c_uint64
+    lib.gu_capture_id.argtypes = [c_void_p]
     lib.gu_last_status.restype = c_int
     lib.gu_last_status.argtypes = [POINTER(c_int), c_int]
     lib.gu_launch_count.restype = c_int64

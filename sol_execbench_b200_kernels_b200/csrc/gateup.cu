@@ -1056,6 +1056,16 @@ int gu_workspace_init(void* workspace, size_t bytes, void* stream) {
   return cudaMemsetAsync(workspace, 0, n, static_cast<cudaStream_t>(stream)) == cudaSuccess ? GU_OK : GU_ECUDA;
 }
 
+unsigned long long gu_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 int gu_run(const gu_problem* pr, void* stream_v) {
   int rc = gu::check_problem(pr);
   if (rc != GU_OK) return rc;

@@ -29,10 +29,10 @@ _PLANS = {"auto": PLAN_AUTO, "tile": PLAN_TILE, "stream": PLAN_STREAM, "tile_dp"
           "tile_pair": PLAN_TILE_PAIR, "tile_pair_sk": PLAN_TILE_PAIR_SK,
           "tile_split": PLAN_TILE_SPLIT}
 
-# Scratch for the stream-K hand-off, one buffer per (device, stream): it is
-# written and consumed inside a single call and carries no result across calls.
-_WORKSPACES: Dict[Tuple[int, int], torch.Tensor] = {}
-_MLP_WORKSPACES: Dict[Tuple[int, int], torch.Tensor] = {}  # likewise for mlp_block
+# Scratch for the stream-K hand-off, one buffer per (device, stream, capture): it is written and consumed inside a single
+# call and carries no result across calls.  `capture` is 0 for eager calls (see `_workspace`).
+_WORKSPACES: Dict[Tuple[int, int, int], torch.Tensor] = {}
+_MLP_WORKSPACES: Dict[Tuple[int, int, int], torch.Tensor] = {}  # likewise for mlp_block
 
 
 def select_plan(m: int, k: int, n: int) -> str:
@@ -176,15 +176,21 @@ def _workspace(device: torch.device, stream_ptr: int, nbytes: int, init=_cabi.li
                kept=_WORKSPACES) -> Optional[torch.Tensor]:
     if nbytes == 0:
         return None
-    key = (device.index if device.index is not None else torch.cuda.current_device(), stream_ptr)
+    # A recorded call has scratch of its graph's own: launches of one stream never overlap, but graphs recorded on one
+    # stream (torch.cuda.graph records all on one by default) may be replayed in any order, on any streams, and next to
+    # eager calls on theirs.  It comes from the graph's memory pool with its initialisation recorded in front of the
+    # graph's first launch on this stream, so every replay starts from zeroed flags and counters.  It is kept for the
+    # capture's later calls, until the next capture on this stream: afterwards the graph's pool alone holds the block.
+    capture = _cabi.lib.gu_capture_id(stream_ptr) if torch._C._cuda_isCurrentStreamCapturing() else 0
+    key = (device.index if device.index is not None else torch.cuda.current_device(), stream_ptr, capture)
     ws = kept.get(key)
     if ws is None or ws.numel() < nbytes:
-        # Under stream capture (torch.cuda.graph switches to a stream of its own, which no eager call has used) the
-        # scratch comes from the graph's memory pool and its initialisation is recorded with the launch: every replay
-        # then starts from zeroed flags and a zero epoch counter, which is a valid state for the kernels.  The tensor
-        # kept here holds the pool's block alive for later calls on that stream.
         ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
         _cabi.check(init(ws.data_ptr(), nbytes, stream_ptr))
+        if capture:
+            for other in list(kept):
+                if other[:2] == key[:2] and other[2] not in (0, capture):
+                    kept.pop(other, None)
         kept[key] = ws
     return ws
 
