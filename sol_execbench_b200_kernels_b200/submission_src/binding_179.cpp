@@ -9,7 +9,7 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
-#include <utility>
+#include <tuple>
 
 #include "gateup.h"
 
@@ -21,23 +21,28 @@ void check_cuda_contiguous(const torch::Tensor& t, const char* name, c10::Scalar
   TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
 }
 
-// Scratch of the small-M plan (stream-K hand-off flags and partial sums): one buffer per (device, stream),
-// grown on demand and initialised once per allocation.  It carries no numbers from one call to the next:
-// every call stamps the flags it reads with a fresh epoch.
+// Scratch of the small-M plan (stream-K hand-off flags and partial sums): one buffer per (device, stream, capture), grown
+// on demand and initialised once per allocation.  It carries no numbers from one call to the next: every call stamps the
+// flags it reads with a fresh epoch.  A recorded call's buffer comes from its graph's memory pool and is initialised by an
+// operation of that graph, since graphs recorded on one stream may be replayed in any order and on any streams; it is kept
+// here for the later calls of its capture, until the next capture on the stream.
 torch::Tensor workspace_for(const torch::Tensor& like, cudaStream_t stream, size_t bytes) {
+  using Key = std::tuple<int, cudaStream_t, unsigned long long>;
   static std::mutex mutex;
-  static std::map<std::pair<int, cudaStream_t>, torch::Tensor> cache;
+  static std::map<Key, torch::Tensor> cache;
+  const int device = static_cast<int>(like.get_device());
+  const unsigned long long capture = gu_capture_id(stream);
   std::lock_guard<std::mutex> lock(mutex);
-  auto key = std::make_pair(static_cast<int>(like.get_device()), stream);
+  const Key key(device, stream, capture);
   auto it = cache.find(key);
-  if (it == cache.end() || static_cast<size_t>(it->second.numel()) < bytes) {
-    torch::Tensor ws = torch::empty({static_cast<int64_t>(bytes)}, like.options().dtype(torch::kUInt8));
-    const int rc = gu_workspace_init(ws.data_ptr(), bytes, stream);
-    TORCH_CHECK(rc == GU_OK, "gu_workspace_init: ", gu_error_string(rc));
-    cache[key] = ws;
-    return ws;
-  }
-  return it->second;
+  if (it != cache.end() && static_cast<size_t>(it->second.numel()) >= bytes) return it->second;
+  torch::Tensor ws = torch::empty({static_cast<int64_t>(bytes)}, like.options().dtype(torch::kUInt8));
+  const int rc = gu_workspace_init(ws.data_ptr(), bytes, stream);
+  TORCH_CHECK(rc == GU_OK, "gu_workspace_init: ", gu_error_string(rc));
+  if (capture != 0)  // (eager calls' entry is the one with capture 0)
+    cache.erase(cache.upper_bound(Key(device, stream, 0)), cache.upper_bound(Key(device, stream, ~0ull)));
+  cache[key] = ws;
+  return ws;
 }
 
 }  // namespace

@@ -40,6 +40,34 @@ def test_problem_179_submission_equals_package_run():
         ext.run(*inp.args(), got.float())
 
 
+def test_problem_179_graphs_recorded_on_one_stream():
+    """Two recorded calls, replayed in the other order and at once on two streams."""
+    import sol_execbench_b200_kernels_b200 as pkg
+    ext = _extension("179")
+    dev = torch.device("cuda:0")
+    for shape in ((16, 4096, 8192), (512, 384, 4864)):
+        inputs = [W.make_inputs(*shape, seed=s, device=dev) for s in (1, 2)]
+        want = [torch.empty(shape[0], shape[2], dtype=torch.bfloat16, device=dev) for _ in inputs]
+        for inp, w in zip(inputs, want):
+            pkg.run(*inp.args(), w)
+        got = [torch.empty_like(w) for w in want]
+        graphs = [torch.cuda.CUDAGraph() for _ in inputs]
+        for graph, inp, out in zip(graphs, inputs, got):
+            with torch.cuda.graph(graph):
+                ext.run(*inp.args(), out)
+                ext.run(*inp.args(), out)
+        side = [torch.cuda.Stream(), torch.cuda.Stream()]
+        for replays in ([(1, 0), (0, 0)], [(0, 0), (1, 1), (0, 0), (1, 1)]):  # (graph, stream)
+            for out in got:
+                out.fill_(float("nan"))
+            torch.cuda.synchronize()
+            for g, s in replays:
+                with torch.cuda.stream(side[s]):
+                    graphs[g].replay()
+            torch.cuda.synchronize()
+            assert all(torch.equal(out, w) for out, w in zip(got, want)), shape
+
+
 def test_problem_038_submission_equals_package_rmsnorm():
     from sol_execbench_b200_kernels_b200 import side_ops
     ext = _extension("38")
