@@ -49,7 +49,7 @@ struct MlpStepParams {
   int m, kb, nb;
   int stages;               // ring depth
   int weights_ready;        // see TileParams::weights_ready
-  unsigned int* sync;       // [0] launches counted on this scratch, [1] tickets of the running one
+  unsigned int* sync;       // [0] the last launch's stamp on this scratch, [1] tickets of the running one
   uint2* partials;          // [gridDim.x][kMlpSlotPairs]
 };
 
@@ -408,11 +408,11 @@ mlp_step_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
       nbk = nbk_next;
       if (++e == steps) e = 0;
     }
-    // whoever drew the last ticket (every CTA has read the count by then) counts the launch
+    // whoever drew the last ticket (every CTA has read the count by then) counts the launch: the count becomes its stamp,
+    // so that 1 follows 0xffffffff once and the launch after it stamps with 2
     if (ctid == 0 && ticket == gridDim.x - 1u) {
+      p.sync[0] = epoch;
       p.sync[1] = 0u;
-      __threadfence();
-      atomicAdd(p.sync, 1u);
     }
   }
 

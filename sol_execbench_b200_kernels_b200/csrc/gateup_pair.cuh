@@ -569,9 +569,8 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap& tm_x, const 
           if (e == 0u) e = 1u;
           *epoch_gen = e;
           if (atomicAdd(p.flags + kPairSyncTickets, 1u) == gridDim.x - 1u) {
+            p.flags[kPairSyncLaunches] = e;  // (not the count + 1: 1 follows 0xffffffff and is not stamped twice)
             p.flags[kPairSyncTickets] = 0u;
-            __threadfence();
-            atomicAdd(p.flags + kPairSyncLaunches, 1u);
           }
         }
       }

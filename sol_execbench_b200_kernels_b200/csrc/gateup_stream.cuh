@@ -49,8 +49,8 @@ struct StreamParams {
 // The epoch of a launch is kept on the device, so that a launch recorded once (a CUDA graph) can be replayed: word
 // kStreamSyncLaunches of the flag area counts completed launches on this workspace, every CTA reads it when it starts
 // and stamps with that count + 1 and takes a ticket (word kStreamSyncTickets) right after reading; the CTA that drew
-// the last ticket advances the count when its work is done.  All CTAs have read the count before the last ticket is
-// taken.
+// the last ticket makes the launch's stamp the new count when its work is done (which is the count + 1 but where that is 0:
+// 1 follows 0xffffffff, and is not stamped twice).  All CTAs have read the count before the last ticket is taken.
 constexpr int kStreamSyncLaunches = 1022;
 constexpr int kStreamSyncTickets = 1023;
 static_assert(kStreamMaxGrid <= kStreamSyncLaunches, "hand-off flags and the launch counters share the flag area");
@@ -347,9 +347,8 @@ gateup_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     // Whoever drew the launch's last ticket — every CTA had read the count by then — advances the count: the next
     // launch (or a replay of this one) stamps with a new epoch.
     if (ctid == 0 && ticket == gridDim.x - 1u) {
+      p.flags[kStreamSyncLaunches] = epoch;
       p.flags[kStreamSyncTickets] = 0u;
-      __threadfence();
-      atomicAdd(p.flags + kStreamSyncLaunches, 1u);
     }
   }
 
