@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape", [(16, 4096, 8192), (8, 8192, 28672), (32, 8192, 28672), (256, 1024, 2048),
-                                   (512, 384, 4864)])
+                                   (512, 384, 4864), (512, 4096, 14336)])
 def test_replayed_graph_equals_eager_calls(shape):
     import sol_execbench_b200_kernels_b200 as pkg
 
@@ -69,7 +69,7 @@ def test_replays_and_eager_calls_may_interleave_on_one_workspace():
     assert torch.equal(out_a, want) and torch.equal(out_b, want)
 
 
-def _run_call(m, k, n):
+def _run_call(m, k, n, plan="auto"):
     """A recorded call, its live input, inputs to put there, and the eager result for each of them."""
     import sol_execbench_b200_kernels_b200 as pkg
 
@@ -79,7 +79,7 @@ def _run_call(m, k, n):
     feeds = [W.make_inputs(m, k, n, seed=20 + i, device="cuda:0").x for i in range(2)]
 
     def call(dst=out):
-        pkg.run(x, base.scale_x, base.gate_proj_weight, base.scale_gate, base.up_proj_weight, base.scale_up, dst)
+        pkg.run_with_plan(x, base.scale_x, base.gate_proj_weight, base.scale_gate, base.up_proj_weight, base.scale_up, dst, plan)
 
     return call, x.view(torch.uint8), [f.view(torch.uint8) for f in feeds], out
 
@@ -97,8 +97,10 @@ def _mlp_call(m, k, n):
     return (lambda dst=out: pkg.mlp_block(x, *weights, dst)), x, feeds, out
 
 
-# the three kernels that keep counters in their scratch: weight streaming, the pair kernel's stream-K schedule, the MLP's steps
-_WITH_SCRATCH = [(_run_call, (16, 4096, 8192)), (_run_call, (512, 384, 4864)), (_mlp_call, (8, 4096, 14336))]
+# the kernels that use scratch: weight streaming, the stream-K schedules of the pair and the lone-CTA kernel (whose stamp comes
+# from the host and is recorded: a replay must find its flags zeroed), the MLP's steps
+_WITH_SCRATCH = [(_run_call, (16, 4096, 8192)), (_run_call, (512, 4096, 14336)), (_run_call, (128, 4096, 14336, "tile_sk")),
+                 (_mlp_call, (8, 4096, 14336))]
 
 
 def _two_graphs(make, shape, pool=None):

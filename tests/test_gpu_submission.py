@@ -45,7 +45,7 @@ def test_problem_179_graphs_recorded_on_one_stream():
     import sol_execbench_b200_kernels_b200 as pkg
     ext = _extension("179")
     dev = torch.device("cuda:0")
-    for shape in ((16, 4096, 8192), (512, 384, 4864)):
+    for shape in ((16, 4096, 8192), (512, 4096, 14336)):
         inputs = [W.make_inputs(*shape, seed=s, device=dev) for s in (1, 2)]
         want = [torch.empty(shape[0], shape[2], dtype=torch.bfloat16, device=dev) for _ in inputs]
         for inp, w in zip(inputs, want):
