@@ -49,21 +49,23 @@ __device__ __forceinline__ uint32_t conv_pair(float2 x0, float2 x1, float2 x2, f
 
 // sigmoid of one value in full relative accuracy at any magnitude: e = 2^(-|x| log2 e) with log2 e split into a
 // 16-bit head (its product with an 8-bit bf16 significand is exact in fp32) and a tail applied as a first-order
-// factor; 1/(1+e) for x >= 0, e/(1+e) for x < 0
+// factor; 1/(1+e) for x >= 0, e/(1+e) for x < 0.  The magnitude stops at 1024, where e is 0 already: an infinity would
+// make the tail's product 0 times infinity.  (A NaN takes some finite sigmoid here and is one again in the product with x.)
 __device__ __noinline__ float sigmoid_wide(float x) {
   constexpr float kLog2eHead = 1.44268798828125f;      // 0x3fb8aa00
   constexpr float kLog2eTailLn2 = 4.888495152129525e-06f;  // (log2 e - head) * ln 2
-  const float a = fabsf(x);
+  const float a = fminf(fabsf(x), 1024.f);
   const float e0 = ex2_approx(-a * kLog2eHead);
   const float e = fmaf(e0, -a * kLog2eTailLn2, e0);
   const float r = rcp_approx(1.0f + e);
   return x < 0.f ? e * r : r;
 }
 
-// bf16(sigmoid) of the four bf16 values in two packed words (channel pair at two positions), all four
-// arguments >= -20: sigmoid = 1 / (1 + 2^(-x log2 e)) directly; each denominator is below 2^30, so the product of
-// the four stays finite and ONE reciprocal of it serves all four (products of the other three give each quotient
-// back): 1.25 special-function operations per element instead of 2.
+// bf16(sigmoid) of the four bf16 values in two packed words (the tail kernel takes a channel pair at two positions, the
+// projection's epilogue two channel pairs at one), all four arguments >= -20 and none a NaN, which would reach the other
+// three (+infinity does not: its denominator is 1): sigmoid = 1 / (1 + 2^(-x log2 e)) directly; each denominator is below
+// 2^30, so the product of the four stays finite and ONE reciprocal of it serves all four (products of the other three
+// give each quotient back): 1.25 special-function operations per element instead of 2.
 __device__ __forceinline__ void sigmoid_2x2(uint32_t ca, uint32_t cb, uint32_t& sa, uint32_t& sb) {
   constexpr float kNegLog2e = -1.4426950408889634f;
   const float2 scale = make_float2(kNegLog2e, kNegLog2e);

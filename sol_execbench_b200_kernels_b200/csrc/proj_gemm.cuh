@@ -173,7 +173,7 @@ __device__ __forceinline__ void conv_row_32(long long sequence, const uint32_t (
     }
     __nv_bfloat162 lowest = *reinterpret_cast<const __nv_bfloat162*>(&conv[0]);
 #pragma unroll
-    for (int i = 1; i < 4; ++i) lowest = __hmin2(lowest, *reinterpret_cast<const __nv_bfloat162*>(&conv[i]));
+    for (int i = 1; i < 4; ++i) lowest = __hmin2_nan(lowest, *reinterpret_cast<const __nv_bfloat162*>(&conv[i]));
     const bool small = __hbge2(lowest, __floats2bfloat162_rn(-20.f, -20.f));
 #pragma unroll
     for (int i = 0; i < 4; i += 2) {

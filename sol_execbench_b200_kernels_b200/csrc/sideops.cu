@@ -214,7 +214,7 @@ mamba_conv1d_tail_kernel(const __nv_bfloat16* projected, const __nv_bfloat16* ma
       }
       __nv_bfloat162 lowest = *reinterpret_cast<const __nv_bfloat162*>(&conv[0]);
 #pragma unroll
-      for (int j = 1; j < kHalf; ++j) lowest = __hmin2(lowest, *reinterpret_cast<const __nv_bfloat162*>(&conv[j]));
+      for (int j = 1; j < kHalf; ++j) lowest = __hmin2_nan(lowest, *reinterpret_cast<const __nv_bfloat162*>(&conv[j]));
       if (__hbge2(lowest, __floats2bfloat162_rn(-20.f, -20.f))) {
 #pragma unroll
         for (int j = 0; j < kHalf; j += 2) {

@@ -83,3 +83,40 @@ def test_a_refused_call_launches_nothing():
         with pytest.raises(ValueError):
             side_ops.mamba_conv1d_with_gating(*bad)
     assert side_ops.launch_count() == before
+
+
+def _bad_channels(conv_b):
+    """Single channels whose convolutions are not finite, or below -20, each among ordinary neighbours."""
+    for channel, value in ((5, "nan"), (16, "inf"), (17, "-50"), (30, "-inf"), (44, "inf"), (47, "-30"), (63, "nan")):
+        conv_b[channel] = float(value)
+
+
+def _same_where_not_finite(got, want, what):
+    got, want = got.float().cpu(), want.float().cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)), what
+    assert torch.equal(torch.isinf(got), torch.isinf(want)), what
+    fine = torch.isfinite(want)
+    diff, size = (got - want).abs()[fine], want.abs()[fine]
+    bad = diff > 1e-30  # (as in the tests of the tail against its oracle: at most 1e-3 of the values, by two bf16 steps)
+    assert int(bad.sum()) <= max(2, 1e-3 * bad.numel()) and bool((diff[bad] <= size[bad] * 2.0 ** -6).all()), what
+
+
+@pytest.mark.parametrize("batch,seq,channels", [(1, 300, 64), (2, 129, 128), (65, 3, 64), (1, 100, 64)])
+def test_values_that_are_not_finite_stay_in_their_channel(batch, seq, channels):
+    """Both forms of the tail against the oracle: channels with a NaN, an infinity or convolutions below -20, and one token
+    whose activations are NaN (it reaches the three positions after it)."""
+    from oracle import sideops_oracle
+    from sol_execbench_b200_kernels_b200 import side_ops
+
+    hidden, mask, weight, bias, conv_w, conv_b = _inputs(batch, seq, 64, channels)
+    _bad_channels(conv_b)
+    hidden[batch - 1, seq // 2] = float("nan")
+    out, _ = side_ops.mamba_conv1d_with_gating(hidden, mask, weight, bias, conv_w, conv_b)
+    projected = torch.empty(batch, seq, 2 * channels, dtype=torch.bfloat16, device="cuda:0")
+    alone = torch.empty_like(out)
+    side_ops.mamba_in_proj(hidden, weight, bias, projected)
+    side_ops.mamba_conv1d_tail(projected, mask, conv_w, conv_b, alone)
+    want = sideops_oracle.mamba_conv1d_tail(projected.cpu(), mask.cpu(), conv_w.cpu(), conv_b.cpu())
+    assert bool(torch.isnan(want).any()) and bool(torch.isinf(want).any()) and bool(torch.isfinite(want).any())
+    _same_where_not_finite(alone, want, "tail")
+    _same_where_not_finite(out, want, "epilogue")
