@@ -694,18 +694,24 @@ MlpGeometry mlp_geometry(int op, int64_t nb, int64_t kb, int64_t sm_count) {
   g.stages = static_cast<int>(fit < kMlpMaxStages ? fit : kMlpMaxStages);
   return g;
 }
-// Whether a step of the block streams its weights; `nb` column blocks of `kb` K blocks.  us of the whole block on B200, tiles /
-// streamed, (tokens, hidden, intermediate):
-//  * Gate/up, against whole tiles (there is no cut along K from 75 column blocks on): it gains what whole tiles leave idle
-//    in their last round and pays the joins.  62 of 148 SMs idle, (8, 4096, 11008), 36.7 / 34.5; 72 in two rounds,
-//    (8, 8192, 28672) 126.0 / 114.1 and (8, 1024, 28672) 38.9 / 35.1; 40, (8, 5120, 13824), 44.9 / 44.8; 36, (8, 4096,
-//    14336), 40.3 / 39.9 and with 16 tokens 40.9 / 41.7; 20, (8, 6144, 16384), 57.3 / 57.5; none, (8, 3584, 18944),
-//    43.9 / 44.0.  Where tiles are cut along K, (8, 8192, 8192), 41.8 / 43.5.
-//  * Down, against tiles cut along K in clusters: (8, 8192, 28672) 114.1 / 112.6 with gate/up streamed, (8, 4096, 14336)
-//    41.4 / 40.3, (8, 4096, 11008) 38.2 / 36.7, (8, 8192, 8192) 42.3 / 41.8, (8, 5120, 8192) 32.4 / 32.4, (8, 2048, 14336)
-//    30.2 / 30.7, (8, 2048, 5632) 20.9 / 21.6: from 9 units per CTA on; and with fewer where the clusters' K ranges are
-//    long, (8, 2048, 28672) 53.7 / 46.8, (8, 1024, 28672) 46.8 / 38.9.  (Below 8 column blocks an owner would collect more
-//    than 18 ranges.)
+// Whether a step of the block streams its weights; `nb` column blocks of `kb` K blocks.  Figures: us of the whole block on B200
+// over rotating operands (600 MB and more between two uses of one), tiles / streamed, or the difference; repeats within 0.3 %.
+//  * Gate/up, against whole tiles (there is no cut along K from 75 column blocks on).  It gains what the idle SMs of the last
+//    round leave of HBM's rate, and pays for joins whose time grows with the tokens and not with the weights.
+//    One round of tiles, gained with 1 / 8 / 16 tokens: K = 2560, 64 of 148 SMs idle +0.5 / -0.2 / -1.5; K = 3072, 64 idle
+//    +1.2 / +0.5 / -0.8, 48 +0.3 / -0.5 / -1.8; K = 4096 (37 us), 60 idle +3.0 / +2.6 / +1.3, 44 +1.2 / +0.5 / -0.7, 36 +0.4 /
+//    -0.2 / -1.3, 28 0.0 / -0.8 / -2.0; K = 8192 (63 us), 40 idle +3.0 / +1.9 / +0.3, 28 +1.8 / +0.6 / -0.9.  So 28 idle SMs and
+//    two more per token, in proportion more below K = 4096 and two thirds of it from K = 8192 on.
+//    Several rounds, which streaming also spares the edges between (K = 1024 (36 us), two: 120 idle +3.2 / +2.6 / +0.3, 40
+//    +1.8 / +0.7 / -2.3, 24 +1.2 / 0.0 / -2.8; K = 4096 (73 us), two: 72 idle +6.4 / +5.1 / +3.2, 40 +3.2 / +1.8 / -0.2, 8 +1.3 /
+//    +0.2 / -1.5; three: 4 idle +2.9 / +2.1 / +4.5; K = 8192, two: none idle +5.8 / +5.4 / +6.3): from five idle SMs per token
+//    above four on, in proportion more where a CTA has less than 32 K blocks in all, and always from 96 on.
+//  * Down, against tiles cut along K in clusters, 8 tokens: (4096, 11008) 36.7 / 33.9, (4096, 14336) 41.4 / 39.6, (8192, 28672)
+//    114.1 / 112.3, (2560, 17920) 36.5 / 35.2, (5120, 9216) 33.9 / 34.0, (5120, 8192) 31.8 / 31.9, (4096, 8192) 29.2 / 29.0,
+//    (2048, 14336) 30.2 / 30.0, (3584, 8192) 26.3 / 27.2, (2048, 8192) 22.3 / 23.3: from 9 units per CTA on; and with fewer
+//    where the clusters' K ranges are long, (1024, 28672) 39.5 / 34.9, (1536, 20480) 35.5 / 32.4, but (1536, 15360) 28.1 / 27.9
+//    and (1024, 14336) 24.8 / 26.4.  16 tokens cost up to 0.5 us more than tiles near the line (5120, 9216).  (Below 8 column
+//    blocks an owner would collect more than 18 ranges.)
 bool mlp_step_streams(int op, int64_t m, int64_t kb, int64_t nb, int64_t sm_count) {
   if (m > kMlpTokens || nb * kb >= (1ll << 31)) return false;
   const MlpGeometry g = mlp_geometry(op, nb, kb, sm_count);
@@ -716,8 +722,12 @@ bool mlp_step_streams(int op, int64_t m, int64_t kb, int64_t nb, int64_t sm_coun
   const int64_t steps = (kb + mlp_blocks_per_unit(op) - 1) / mlp_blocks_per_unit(op);
   const bool long_ranges = nb * steps >= 9 * g.grid;
   if (op == kMlpDown) return nb >= 8 && (long_ranges || kb >= 160);
-  const int64_t idle = (nb + sm_count - 1) / sm_count * sm_count - nb;
-  return long_ranges && 2 * nb > sm_count && 148 * idle >= (m <= 8 ? 36 : 40) * sm_count;
+  if (!long_ranges || 2 * nb <= sm_count) return false;
+  const int64_t rounds = (nb + sm_count - 1) / sm_count, blocks = kb * rounds;  // K blocks of the busiest CTA of whole tiles
+  const int64_t idle = 148 * (rounds * sm_count - nb) / sm_count;
+  const int64_t weight = blocks < 32 ? blocks : 32;
+  if (rounds > 1) return blocks >= 96 || idle * weight >= 160 * (m - 4);
+  return idle * (kb < 64 ? weight : 48) >= 32 * (28 + 2 * m);
 }
 template <int kOp>
 int launch_mlp_step(MlpStepParams& p, const DeviceInfo& dev, void* scratch, cudaStream_t stream, const CUtensorMap& tm_x,

@@ -100,7 +100,7 @@ def _mlp_call(m, k, n):
 # the kernels that use scratch: weight streaming, the stream-K schedules of the pair and the lone-CTA kernel (whose stamp comes
 # from the host and is recorded: a replay must find its flags zeroed), the MLP's steps
 _WITH_SCRATCH = [(_run_call, (16, 4096, 8192)), (_run_call, (512, 4096, 14336)), (_run_call, (128, 4096, 14336, "tile_sk")),
-                 (_mlp_call, (8, 4096, 14336))]
+                 (_mlp_call, (8, 4096, 11008))]
 
 
 def _two_graphs(make, shape, pool=None):

@@ -19,7 +19,8 @@ def _weights(g, k, n, h):
 # tokens at the edges of the padded 16; K blocks that no range divides, odd ones in the down projection (a last step with
 # one tile), ranges longer and shorter than a column block, few and many column blocks
 @pytest.mark.parametrize("m,kb,nb,hb", [(1, 32, 112, 32), (8, 33, 147, 29), (15, 64, 225, 64), (16, 41, 111, 40), (16, 8, 224, 160),
-                                        (2, 128, 64, 96), (3, 16, 449, 5)])
+                                        (2, 128, 64, 96), (3, 16, 449, 5), (8, 33, 150, 29), (16, 41, 80, 40), (15, 9, 170, 16),
+                                        (1, 32, 100, 32), (16, 65, 108, 8)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_streamed_steps_match_whole_tiles(m, kb, nb, hb, dtype):
     import sol_execbench_b200_kernels_b200 as pkg
