@@ -118,8 +118,8 @@ for shape, plan in (((1, 4224, 128), "tile"), ((31, 7168, 384), "tile"), ((200, 
     mask = torch.ones_like(wide, dtype=torch.bool)
     mask[1:m + 1, 128:128 + n] = False
     assert bool((wide[mask] == 7.0).all()), f"{shape} {plan}: wrote outside the destination"
-# mlp_block, cut and whole: (tokens, hidden, intermediate, output); both steps cut, one of them, pairs, lone CTAs, an odd
-# count of 128-column output blocks
+# mlp_block, whole, streamed and cut: (tokens, hidden, intermediate, output); without scratch both steps are cut, or one of
+# them; pairs, lone CTAs, an odd count of 128-column output blocks
 for m, k, n, h in ((1, 1664, 1536, 128), (33, 2048, 2304, 640), (8, 1024, 9600, 1152), (128, 1536, 2432, 384),
                    (129, 384, 2176, 256), (300, 512, 4992, 2048), (515, 256, 384, 128)):
     x = torch.randn(m, k, device=dev).to(torch.bfloat16)
@@ -131,7 +131,10 @@ for m, k, n, h in ((1, 1664, 1536, 128), (33, 2048, 2304, 640), (8, 1024, 9600, 
     ref = torch.empty(m, h, dtype=torch.bfloat16, device=dev)
     pkg.blockwise_gemm(q, sc, *ws[4:], ref)
     launches += 3
-    for whole in (True, False):
+    # whole tiles; streamed up to 16 tokens (any shape in this build) and cut above; cut along K without that scratch
+    scratch_bytes = pkg.kernel._mlp_scratch_bytes
+    for whole, scratch in ((True, scratch_bytes), (False, scratch_bytes), (False, lambda *shape: 0)):
+        pkg.kernel._mlp_scratch_bytes = scratch
         wide = torch.full((m + 2, h + 256), 7.0, dtype=torch.bfloat16, device=dev)
         view = wide[1:m + 1, 128:128 + h]
         pkg.mlp_block(x, *ws, view, whole_tiles=whole)
@@ -145,6 +148,7 @@ for m, k, n, h in ((1, 1664, 1536, 128), (33, 2048, 2304, 640), (8, 1024, 9600, 
         mask = torch.ones_like(wide, dtype=torch.bool)
         mask[1:m + 1, 128:128 + h] = False
         assert bool((wide[mask] == 7.0).all()), f"mlp_block {(m, k, n, h)}: wrote outside the destination"
+    pkg.kernel._mlp_scratch_bytes = scratch_bytes
 print(f"swept {launches} launches under the range-checked build: status 0 throughout")
 """
 

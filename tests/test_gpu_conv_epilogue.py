@@ -45,6 +45,14 @@ def _compare(shape):
     assert code == 0, f"{shape}: device status {code}, detail {detail:#x}"
     want_gate = projected[:, :, channels:].transpose(1, 2)
     assert torch.equal(gate, want_gate) and gate.stride() == want_gate.stride()
+    # every output and every gate value is written, whatever the buffers held
+    again, buf = torch.full_like(out, float("nan")), torch.full_like(projected, float("nan"))
+    side_ops._so.check(side_ops._so.lib.so_mamba_in_proj_conv(
+        hidden.data_ptr(), weight.data_ptr(), bias.data_ptr(), buf.data_ptr(), mask.data_ptr(), conv_w.data_ptr(),
+        conv_b.data_ptr(), again.data_ptr(), batch, seq, hidden.shape[2], 2 * channels, channels,
+        torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert torch.equal(again, out) and torch.equal(buf[:, :, channels:], projected[:, :, channels:])
     # The same operations up to the sigmoid, whose reciprocal is shared by other groups of four values: its last fp32 bit
     # may differ, and a bf16 rounding with it (2^-8 relative, then once more in the product) where it is within 2^-22 of
     # a tie, fewer than one in a thousand.

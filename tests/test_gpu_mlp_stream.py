@@ -108,6 +108,7 @@ def test_small_scratch_is_no_scratch():
     block = _cabi.GuMlp(x.data_ptr(), *[t.data_ptr() for t in weights], x_q.data_ptr(), x_s.data_ptr(), mid_q.data_ptr(),
                         mid_s.data_ptr(), without.data_ptr(), m, k, n, k, k, k, 0, 0)
     plain = without.clone()
+    without.fill_(float("nan"))
     _cabi.check(_cabi.lib.gu_mlp_block(ctypes.byref(block), stream))
     torch.cuda.synchronize()
     assert torch.equal(without, plain)

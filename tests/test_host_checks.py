@@ -1,5 +1,5 @@
-"""The quick acceptance in front of `run`'s checks, against those checks, on stand-ins for CUDA tensors: it accepts a call only
-where they do, with the same sizes, and accepts every plain one."""
+"""The quick acceptance in front of the checks of `run` and `mlp_block`, against those checks, on stand-ins for CUDA tensors:
+it accepts a call only where they do, with the same sizes, and accepts every plain one."""
 import itertools
 
 import pytest
@@ -86,6 +86,54 @@ def test_whatever_the_checks_refuse_is_left_to_them():
         ok[0], ok[2], ok[4] = (Fake(torch.zeros(r, k, dtype=torch.uint8).view(torch.float8_e4m3fn)) for r in (m, n, n))
         ok[6] = Fake(torch.zeros(m, n, dtype=torch.bfloat16))
         assert _both(ok) == (None, None)
+
+
+class _Accepted(Exception):
+    pass
+
+
+def _mlp_operands(m=3, k=256, n=384, h=128):
+    out = [torch.zeros(m, k, dtype=torch.bfloat16)]
+    for rows, cols in ((n, k), (n, k), (h, n)):
+        out += [torch.zeros(rows, cols, dtype=torch.uint8).view(torch.float8_e4m3fn), torch.zeros(rows // 128, cols // 128)]
+    return out + [torch.zeros(m, h, dtype=torch.bfloat16)]
+
+
+def test_mlp_block_refuses_what_its_full_checks_refuse(monkeypatch):
+    """`mlp_block` with its quick acceptance and with `_check` on every call: the same calls get past, with the same messages."""
+    def layout(*shape):
+        raise _Accepted(*shape)
+
+    monkeypatch.setattr(kernel, "_mlp_layout", layout)
+    quick = kernel._plain
+
+    def outcome(operands, plain):
+        monkeypatch.setattr(kernel, "_plain", plain)
+        try:
+            kernel.mlp_block(*operands)
+        except (_Accepted, ValueError, IndexError) as e:
+            return type(e), str(e)
+
+    def both(operands):
+        got = outcome(operands, quick), outcome(operands, lambda operands, index: False)
+        assert got[0] == got[1] and got[0] is not None
+        return got[0][0]
+
+    base = _mlp_operands()
+    assert both([Fake(t) for t in base]) is _Accepted
+    wide = torch.zeros(4, 192, dtype=torch.bfloat16)
+    assert both([Fake(t) for t in base[:7]] + [Fake(wide[1:, 64:])]) is _Accepted
+    pitched = Fake(torch.zeros(3, 264)[:, :256])
+    assert both([pitched] + [Fake(t) for t in base[1:]]) is _Accepted
+    refused = 0
+    for i, j in itertools.product(range(8), range(8)):
+        for v, w in itertools.product(_variants(base[i]), _variants(base[j])):
+            operands = [Fake(t) for t in base]
+            operands[i] = v
+            if j != i:
+                operands[j] = w
+            refused += both(operands) is not _Accepted
+    assert refused > 5000
 
 
 def test_packed_arguments_have_the_structures_layout():
