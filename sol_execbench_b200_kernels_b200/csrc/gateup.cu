@@ -734,7 +734,6 @@ int launch_mlp_step(MlpStepParams& p, const DeviceInfo& dev, void* scratch, cuda
                     const CUtensorMap& tm_w0, const CUtensorMap& tm_w1) {
   const MlpGeometry g = mlp_geometry(kOp, p.nb, p.kb, dev.sm_count);
   p.stages = g.stages;
-  p.weights_ready = 1;  // (only behind the block's quantiser)
   p.sync = static_cast<unsigned int*>(scratch);
   p.partials = reinterpret_cast<uint2*>(static_cast<uint8_t*>(scratch) + 4096);
   return launch(mlp_step_kernel<kOp>, static_cast<int>(g.grid), kStreamThreads,
@@ -793,11 +792,9 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
   int rc = device_info(&dev);
   if (rc != GU_OK) return rc;
   const int64_t m = pr->m, k = pr->k, n = pr->n;
-  CUtensorMap tm_x, tm_g, tm_u, tm_q;
-  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
+  CUtensorMap tm_x, tm_g, tm_u, tm_q;  // (each where its kernel is chosen)
   if ((rc = get_map(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->gate_w, k, n, k, 128, 128)) != GU_OK) return rc;
   if ((rc = get_map(&tm_u, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->up_w, k, n, k, 128, 128)) != GU_OK) return rc;
-  if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
 
   if (scratch && mlp_step_streams(kMlpGateUp, m, k / 128, n / 128, dev->sm_count)) {
     CUtensorMap tm_rows;
@@ -815,6 +812,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
     mp.nb = static_cast<int>(n / 128);
     return launch_mlp_step<kMlpGateUp>(mp, *dev, scratch, static_cast<cudaStream_t>(stream_v), tm_rows, tm_g, tm_u);
   }
+  if ((rc = get_map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, pr->x, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
   if (cut) {
     const int splits = split_ctas(*dev, m, k / 128, n / kTileN, chained);
     if (splits > 1) {
@@ -830,6 +828,7 @@ int fp8out_launch(const gu_problem* pr, void* out_q, float* out_scale, bool chai
       return launch_split<kSplitFp8>(sp, m, k, n, n / kTileN, splits, tm_x, tm_g, tm_u, static_cast<cudaStream_t>(stream_v));
     }
   }
+  if ((rc = get_map(&tm_q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, out_q, n, m, n, 128, 128)) != GU_OK) return rc;
   TileParams p;
   p.scale_x = pr->scale_x;
   p.scale_gate = pr->scale_gate;
@@ -882,9 +881,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
   if (rc != GU_OK) return rc;
 
   CUtensorMap tm_a, tm_b, tm_c;
-  if ((rc = get_map(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
   if ((rc = get_map(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b, k, n, k, 128, 128)) != GU_OK) return rc;
-  if ((rc = get_map(&tm_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, n, m, ld_c * 2, 64, 128)) != GU_OK) return rc;
 
   if (scratch && mlp_step_streams(kMlpDown, m, k / 128, n / 128, dev->sm_count)) {
     CUtensorMap tm_rows;
@@ -900,6 +897,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
     mp.nb = static_cast<int>(n / 128);
     return launch_mlp_step<kMlpDown>(mp, *dev, scratch, static_cast<cudaStream_t>(stream_v), tm_rows, tm_b, tm_b);
   }
+  if ((rc = get_map(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k, 128, x_box_rows(m))) != GU_OK) return rc;
   if (cut) {
     const int64_t col_tiles = (n / 128 + 1) / 2;
     const int splits = split_ctas(*dev, m, k / 128, col_tiles, chained);
@@ -915,6 +913,7 @@ int gemm_launch(const void* a, const float* scale_a, const void* b, const float*
       return launch_split<kSplitGemm>(sp, m, k, n, col_tiles, splits, tm_a, tm_b, tm_b, static_cast<cudaStream_t>(stream_v));
     }
   }
+  if ((rc = get_map(&tm_c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, n, m, ld_c * 2, 64, 128)) != GU_OK) return rc;
   TileParams p;
   p.scale_x = scale_a;
   p.scale_gate = scale_b;

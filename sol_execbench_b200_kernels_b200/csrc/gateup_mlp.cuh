@@ -48,7 +48,6 @@ struct MlpStepParams {
   long long ld_out;
   int m, kb, nb;
   int stages;               // ring depth
-  int weights_ready;        // see TileParams::weights_ready
   unsigned int* sync;       // [0] the last launch's stamp on this scratch, [1] tickets of the running one
   uint2* partials;          // [gridDim.x][kMlpSlotPairs]
 };
@@ -142,25 +141,15 @@ mlp_step_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
       tma_load_2d_hint(dst + kOperandTileBytes, &tm_w1, full, j * kBlockK, nbk * 128, stream_once);
     }
   };
-  int early = 0;  // (producer) units whose weights are loaded before the wait
+  // (producer) the first ring's weights, before the wait: the block's quantiser lets nothing start before all in front of it
+  // has completed, so they are ready (see TileParams::weights_ready)
+  const int early = min(count, p.stages);
   if (warp == 0 && lane == 0) {
     int nbk = nbk0, j = j0;
-    const int ahead = min(count, p.stages);
-    for (int i = 0; i < ahead; ++i) {
-      if (in_range(i, nbk, j)) {
-        if (p.weights_ready) {
-          load_weights(i, nbk, j);
-        } else if constexpr (kDown) {
-          tma_prefetch_2d(&tm_w0, 2 * j * kBlockK, nbk * 128);
-          if (second(j)) tma_prefetch_2d(&tm_w0, (2 * j + 1) * kBlockK, nbk * 128);
-        } else {
-          tma_prefetch_2d(&tm_w0, j * kBlockK, nbk * 128);
-          tma_prefetch_2d(&tm_w1, j * kBlockK, nbk * 128);
-        }
-      }
+    for (int i = 0; i < early; ++i) {
+      if (in_range(i, nbk, j)) load_weights(i, nbk, j);
       if (++j == steps) { j = 0; ++nbk; }
     }
-    if (p.weights_ready) early = ahead;
   }
   pdl_wait();
 
