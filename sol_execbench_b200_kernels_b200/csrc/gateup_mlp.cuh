@@ -143,9 +143,11 @@ mlp_step_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   };
   // (producer) the first ring's weights, before the wait: the block's quantiser lets nothing start before all in front of it
   // has completed, so they are ready (see TileParams::weights_ready)
-  const int early = min(count, p.stages);
+  int early = 0;
   if (warp == 0 && lane == 0) {
     int nbk = nbk0, j = j0;
+    early = min(count, p.stages);
+#pragma unroll 1
     for (int i = 0; i < early; ++i) {
       if (in_range(i, nbk, j)) load_weights(i, nbk, j);
       if (++j == steps) { j = 0; ++nbk; }
