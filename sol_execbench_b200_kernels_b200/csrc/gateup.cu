@@ -695,23 +695,34 @@ MlpGeometry mlp_geometry(int op, int64_t nb, int64_t kb, int64_t sm_count) {
   return g;
 }
 // Whether a step of the block streams its weights; `nb` column blocks of `kb` K blocks.  Figures: us of the whole block on B200
-// over rotating operands (600 MB and more between two uses of one), tiles / streamed, or the difference; repeats within 0.3 %.
+// in loops of 0.1 s over rotating operands (500 MB and more between two uses of one), both sides in turn, tiles / streamed or
+// the difference.  Repeats are within 0.1 us up to K = 4096 and within 1 us above.  (In bursts of 1 ms, at full clock, streaming
+// gains 0.3 to 0.5 us less.)
 //  * Gate/up, against whole tiles (there is no cut along K from 75 column blocks on).  It gains what the idle SMs of the last
-//    round leave of HBM's rate, and pays for joins whose time grows with the tokens and not with the weights.
-//    One round of tiles, gained with 1 / 8 / 16 tokens: K = 2560, 64 of 148 SMs idle +0.5 / -0.2 / -1.5; K = 3072, 64 idle
-//    +1.2 / +0.5 / -0.8, 48 +0.3 / -0.5 / -1.8; K = 4096 (37 us), 60 idle +3.0 / +2.6 / +1.3, 44 +1.2 / +0.5 / -0.7, 36 +0.4 /
-//    -0.2 / -1.3, 28 0.0 / -0.8 / -2.0; K = 8192 (63 us), 40 idle +3.0 / +1.9 / +0.3, 28 +1.8 / +0.6 / -0.9.  So 28 idle SMs and
-//    two more per token, in proportion more below K = 4096 and two thirds of it from K = 8192 on.
-//    Several rounds, which streaming also spares the edges between (K = 1024 (36 us), two: 120 idle +3.2 / +2.6 / +0.3, 40
-//    +1.8 / +0.7 / -2.3, 24 +1.2 / 0.0 / -2.8; K = 4096 (73 us), two: 72 idle +6.4 / +5.1 / +3.2, 40 +3.2 / +1.8 / -0.2, 8 +1.3 /
-//    +0.2 / -1.5; three: 4 idle +2.9 / +2.1 / +4.5; K = 8192, two: none idle +5.8 / +5.4 / +6.3): from five idle SMs per token
-//    above four on, in proportion more where a CTA has less than 32 K blocks in all, and always from 96 on.
-//  * Down, against tiles cut along K in clusters, 8 tokens: (4096, 11008) 36.7 / 33.9, (4096, 14336) 41.4 / 39.6, (8192, 28672)
-//    114.1 / 112.3, (2560, 17920) 36.5 / 35.2, (5120, 9216) 33.9 / 34.0, (5120, 8192) 31.8 / 31.9, (4096, 8192) 29.2 / 29.0,
-//    (2048, 14336) 30.2 / 30.0, (3584, 8192) 26.3 / 27.2, (2048, 8192) 22.3 / 23.3: from 9 units per CTA on; and with fewer
-//    where the clusters' K ranges are long, (1024, 28672) 39.5 / 34.9, (1536, 20480) 35.5 / 32.4, but (1536, 15360) 28.1 / 27.9
-//    and (1024, 14336) 24.8 / 26.4.  16 tokens cost up to 0.5 us more than tiles near the line (5120, 9216).  (Below 8 column
-//    blocks an owner would collect more than 18 ranges.)
+//    round leave of HBM's rate, and pays for joins whose time grows with the tokens and not with the weights.  Gained with
+//    1 / 4 / 8 / 16 tokens, one round of tiles:
+//      K = 2048 (27 us)  56 of 148 SMs idle +0.3 / 0.0 / -0.3 / -1.8
+//      K = 2560 (30 us)  72 +0.9 / +0.6 / +0.2 / -1.1, 40 -0.1 / -0.4 / -0.9 / -2.1
+//      K = 3072 (33 us)  72 +1.7 / +1.4 / +1.0 / -0.2, 56 +1.0 / +0.7 / +0.1 / -1.3, 40 0.0 / -0.4 / -0.8 / -2.0
+//      K = 3584 (36 us)  48 +1.7 / +1.3 / +1.2 / -0.4, 36 +0.6 / +0.5 / +0.6 / -0.9
+//      K = 4096 (39 us)  60 +3.2 / +3.0 / +2.9 / +1.4, 52 +2.3 / +1.9 / +1.9 / +0.3, 44 +1.2 / +1.1 / +0.9 / -0.8,
+//                        36 +0.9 / +0.6 / +0.4 / -1.0, 28 +0.7 / 0.0 / 0.0 / -1.5, 20 +0.4 / -0.2 / -0.1 / -1.5
+//      K = 6144 (53 us)  48 +2.1 / +2.4 / +1.8 / -0.2, 36 +1.0 / 0.0 / +0.5 / -1.2
+//      K = 8192 (69 us)  40 +3.9 / +3.7 / +3.4 / +1.9, 28 +2.0 / +1.7 / +0.9 / 0.0, 20 +1.0 / +1.1 / -0.3 / -1.0
+//    So 18 idle SMs and two more per token; more where K is below 4096, four fifths of it from K = 8192 on.
+//    Several rounds, which streaming also spares the edges between:
+//      K = 1024 (36 us, bursts), two  104 +2.4 / +2.2 / +1.9 / -0.4, 40 +1.8 / +1.4 / +0.7 / -2.3
+//      K = 2048 (47 us), two          40 +2.9 / +2.5 / +2.5 / -0.1
+//      K = 4096 (80 us), two          72 +7.0 / +7.2 / +6.1 / +3.9, 40 +4.0 / +3.6 / +3.2 / +0.1, 24 +2.9 / +0.9 / +1.1 / -1.5
+//      K = 4096 (bursts), three       4 +2.9 with one token, +2.1 with 8, +4.5 with 16
+//      K = 8192 (140 us), two         40 +8.3 / +7.6 / +6.4 / +2.3
+//    So four idle SMs per token above three, in proportion more where a CTA has less than 32 K blocks in all, and none from 96 on.
+//  * Down, against tiles cut along K in clusters, 8 tokens, bursts: (4096, 11008) 36.7 / 33.9, (4096, 14336) 41.4 / 39.6,
+//    (8192, 28672) 114.1 / 112.3, (2560, 17920) 36.5 / 35.2, (5120, 9216) 33.9 / 34.0, (5120, 8192) 31.8 / 31.9, (4096, 8192)
+//    29.2 / 29.0, (2048, 14336) 30.2 / 30.0, (3584, 8192) 26.3 / 27.2, (2048, 8192) 22.3 / 23.3: from 9 units per CTA on; and
+//    with fewer where the clusters' K ranges are long, (1024, 28672) 39.5 / 34.9, (1536, 20480) 35.5 / 32.4, but (1536, 15360)
+//    28.1 / 27.9 and (1024, 14336) 24.8 / 26.4.  16 tokens cost up to 0.5 us more than tiles near the line (5120, 9216).
+//    (Below 8 column blocks an owner would collect more than 18 ranges.)
 bool mlp_step_streams(int op, int64_t m, int64_t kb, int64_t nb, int64_t sm_count) {
   if (m > kMlpTokens || nb * kb >= (1ll << 31)) return false;
   const MlpGeometry g = mlp_geometry(op, nb, kb, sm_count);
@@ -725,9 +736,8 @@ bool mlp_step_streams(int op, int64_t m, int64_t kb, int64_t nb, int64_t sm_coun
   if (!long_ranges || 2 * nb <= sm_count) return false;
   const int64_t rounds = (nb + sm_count - 1) / sm_count, blocks = kb * rounds;  // K blocks of the busiest CTA of whole tiles
   const int64_t idle = 148 * (rounds * sm_count - nb) / sm_count;
-  const int64_t weight = blocks < 32 ? blocks : 32;
-  if (rounds > 1) return blocks >= 96 || idle * weight >= 160 * (m - 4);
-  return idle * (kb < 64 ? weight : 48) >= 32 * (28 + 2 * m);
+  if (rounds > 1) return blocks >= 96 || idle * (blocks < 32 ? blocks : 32) >= 128 * (m - 3);
+  return idle * (kb < 32 ? 3 * kb / 2 - 16 : kb < 64 ? 32 : 40) >= 32 * (18 + 2 * m);
 }
 template <int kOp>
 int launch_mlp_step(MlpStepParams& p, const DeviceInfo& dev, void* scratch, cudaStream_t stream, const CUtensorMap& tm_x,

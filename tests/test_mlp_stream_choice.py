@@ -16,15 +16,17 @@ def _choice(op, m, k, n, with_workspace):
     (8, 2048, 5632, False, False), (8, 1024, 4096, False, False), (8, 7168, 2304, False, False),
     (17, 4096, 14336, False, False), (17, 8192, 28672, False, False), (8, 512, 14336, False, False),
     # us of the block with operands that stay out of L2, gate/up in whole tiles / streamed
-    (8, 4096, 14336, False, True),   # 39.4 / 39.6
-    (1, 4096, 14336, True, True),    # 38.8 / 38.4
+    (8, 4096, 14336, True, True),    # 40.1 / 39.8
+    (8, 5120, 13824, True, True),
     (8, 2048, 14336, False, False),  # 30.1 / 30.7
-    (8, 3072, 13824, False, False), # 34.0 / 34.9
-    (16, 2048, 11776, False, False), # 28.2 / 30.0
+    (8, 3072, 13824, False, False),  # 34.2 / 34.9
+    (16, 2048, 11776, False, False), # 28.3 / 30.0
+    (1, 4096, 16384, True, True),    # 42.4 / 42.0
+    (8, 4096, 16384, False, True),   # 43.6 / 43.6
     (16, 1024, 32768, False, True),  # 37.4 / 39.7: two rounds of tiles
     (4, 1024, 32768, True, True),    # 35.8 / 34.4
     (16, 4096, 56320, True, True),   # 118 / 114: three
-    (8, 8192, 34816, True, True),    # 140 / 133
+    (8, 8192, 32768, True, True),    # 142 / 135
 ])
 def test_steps_that_stream(m, k, n, gateup, down):
     assert (_choice(_cabi.OP_MLP_GATEUP, m, k, n, 2) == "stream") == gateup
