@@ -18,6 +18,7 @@ from .kernel import _on, _stream_ptr
 HEAD_DIM = 128
 CONV_TAPS = 4
 CONV_CHANNEL_TILE = 64
+PAIR_ROWS = 128  # above these the projection runs on CTA pairs, whose epilogue can take the convolution tail
 
 
 def _need(cond: bool, msg: str) -> None:
@@ -149,7 +150,7 @@ def mamba_conv1d_with_gating(hidden_states: torch.Tensor, attention_mask: torch.
                              conv1d_bias: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """Problem 029 as the reference exposes it: (output_hidden_states [B, C, L], gate [B, C, L] view).
 
-    One call into the library, two launches: up to 128 rows the input projection (a tcgen05 bf16 GEMM with the bias in its
+    Two launches of this package's kernels.  Up to 128 rows the input projection (a tcgen05 bf16 GEMM with the bias in its
     epilogue; the reference uses a CUTLASS builder GEMM there, kernel.cu:36-160) and the convolution tail; above, the
     projection with the tail in its epilogue, and a small kernel for the positions at the edges of its row blocks.  `gate`
     is the transposed view of the projection's upper half, as in the reference (binding.cpp:88-92); the lower half of that
@@ -160,7 +161,13 @@ def mamba_conv1d_with_gating(hidden_states: torch.Tensor, attention_mask: torch.
     _need(projected_width % 2 == 0, "in_proj_weight must have an even number of rows")
     channels = projected_width // 2
     batch, sequence = hidden_states.shape[:2]
-    # the checks of `mamba_in_proj` and `mamba_conv1d_tail`, of what the caller passed; all come before the first launch
+    if batch * sequence <= PAIR_ROWS:
+        projected = torch.empty(batch, sequence, projected_width, dtype=hidden_states.dtype, device=hidden_states.device)
+        mamba_in_proj(hidden_states, in_proj_weight, in_proj_bias, projected)
+        out = torch.empty(batch, channels, sequence, dtype=hidden_states.dtype, device=hidden_states.device)
+        mamba_conv1d_tail(projected, attention_mask, conv1d_weight, conv1d_bias, out)
+        return out, projected[:, :, channels:].transpose(1, 2)
+    # the checks of those two functions, of what the caller passed (one call into the library, so all come first)
     _need(in_proj_weight.dim() == 2, "in_proj_weight must have shape [N, K]")
     k = in_proj_weight.shape[1]
     if hidden_states.shape[2] != k:
@@ -180,12 +187,11 @@ def mamba_conv1d_with_gating(hidden_states: torch.Tensor, attention_mask: torch.
         _check_bf16(t, name, device)
     projected = torch.empty(batch, sequence, projected_width, dtype=torch.bfloat16, device=device)
     out = torch.empty(batch, channels, sequence, dtype=torch.bfloat16, device=device)
-    if batch * sequence > 0:
-        with _on(device):
-            _so.check(_so.lib.so_mamba_in_proj_conv(
-                hidden_states.data_ptr(), in_proj_weight.data_ptr(), in_proj_bias.data_ptr(), projected.data_ptr(),
-                attention_mask.data_ptr(), conv1d_weight.data_ptr(), conv1d_bias.data_ptr(), out.data_ptr(),
-                batch, sequence, k, projected_width, channels, _stream_ptr(device)))
+    with _on(device):
+        _so.check(_so.lib.so_mamba_in_proj_conv(
+            hidden_states.data_ptr(), in_proj_weight.data_ptr(), in_proj_bias.data_ptr(), projected.data_ptr(),
+            attention_mask.data_ptr(), conv1d_weight.data_ptr(), conv1d_bias.data_ptr(), out.data_ptr(),
+            batch, sequence, k, projected_width, channels, _stream_ptr(device)))
     return out, projected[:, :, channels:].transpose(1, 2)
 
 
