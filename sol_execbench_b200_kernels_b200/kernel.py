@@ -181,7 +181,8 @@ def _workspace(device: torch.device, stream_ptr: int, nbytes: int, init=_cabi.li
     # eager calls on theirs.  It comes from the graph's memory pool with its initialisation recorded in front of the
     # graph's first launch on this stream, so every replay starts from zeroed flags and counters.  It is kept for the
     # capture's later calls, until the next capture on this stream: afterwards the graph's pool alone holds the block.
-    capture = _cabi.lib.gu_capture_id(stream_ptr) if torch._C._cuda_isCurrentStreamCapturing() else 0
+    # (The default stream, 0, cannot be recorded: a lone call there is spared the question, 0.3 us.)
+    capture = _cabi.lib.gu_capture_id(stream_ptr) if stream_ptr and torch._C._cuda_isCurrentStreamCapturing() else 0
     key = (device.index if device.index is not None else torch.cuda.current_device(), stream_ptr, capture)
     ws = kept.get(key)
     if ws is None or ws.numel() < nbytes:

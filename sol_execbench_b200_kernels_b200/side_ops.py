@@ -162,6 +162,7 @@ def mamba_conv1d_with_gating(hidden_states: torch.Tensor, attention_mask: torch.
     channels = projected_width // 2
     batch, sequence = hidden_states.shape[:2]
     if batch * sequence <= PAIR_ROWS:
+        # two calls: the tail's checks run while the projection does (a lone call of 128 rows: 119 us, 122 with all first)
         projected = torch.empty(batch, sequence, projected_width, dtype=hidden_states.dtype, device=hidden_states.device)
         mamba_in_proj(hidden_states, in_proj_weight, in_proj_bias, projected)
         out = torch.empty(batch, channels, sequence, dtype=hidden_states.dtype, device=hidden_states.device)
